@@ -16,6 +16,7 @@
 // The eigen-decomposition of L, the tanh fit of the sweep and the neighbour lists (a sort per
 // column) stay with the caller.  The sweep evaluates exp in float32 and sums in float64 per
 // block; everything else is float64.
+#include <algorithm>
 #include <cstdint>
 
 #include "mem_internal.cuh"
@@ -26,119 +27,288 @@ namespace {
 constexpr double kZeroDist = 1e-6;
 constexpr int kTile = 32;
 
-// 1. Y from D (row-major n x n); listed = nullptr: every entry is a listed neighbour (k = n)
-__global__ void dm_sym_kernel(const double* __restrict__ D, int64_t n,
-                              const uint8_t* __restrict__ listed, double* __restrict__ Y) {
-    __shared__ double tD[kTile][kTile + 1];      // D block transposed: the (j, i) entries
+// 1. Y from D (row-major n x n); listed = nullptr: every entry is a listed neighbour (k = n).
+// One CTA per unordered pair of 32 x 32 tiles (bi, bj), bi <= bj: it reads both tiles once and
+// writes both, and a pair of entries shares its square roots -- one where D_ij and D_ji are
+// equal, as in every D of the distance stage -- because FP64 (2 FMA per clock and SM) bounds
+// this kernel: n = 3000 takes 152 us, 387 us with four square roots per pair.
+__device__ __forceinline__ double dm_pair_value(double sij, double sji, bool zero_edge) {
+    const double y = sij * sij + sji * sji - sij * sji;
+    return (y != 0.0 || zero_edge) ? y : -1.0;
+}
+
+__global__ void __launch_bounds__(256) dm_sym_kernel(
+        const double* __restrict__ D, int64_t n, const uint8_t* __restrict__ listed,
+        double* __restrict__ Y) {
+    __shared__ double tY[kTile][kTile + 1];      // D block (bj, bi), then its Y block
     __shared__ uint8_t tL[kTile][kTile + 1];
     const int64_t bi = (int64_t)blockIdx.y * kTile, bj = (int64_t)blockIdx.x * kTile;
+    if (bj < bi) return;
     const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8 threads
-    for (int r = ty; r < kTile; r += 8) {
-        const int64_t gi = bj + r, gj = bi + tx;   // load D[bj + r][bi + tx]
+    double dij[kTile / 8];
+    uint8_t lij[kTile / 8];
+#pragma unroll
+    for (int q = 0; q < kTile / 8; ++q) {
+        const int r = ty + 8 * q;
+        const int64_t gi = bj + r, gj = bi + tx;   // D[bj + r][bi + tx]
         const bool in = gi < n && gj < n;
-        tD[tx][r] = in ? D[gi * n + gj] : 0.0;
-        tL[tx][r] = in ? (listed ? listed[gi * n + gj] : (uint8_t)1) : (uint8_t)0;
+        tY[r][tx] = in ? D[gi * n + gj] : 0.0;
+        tL[r][tx] = in ? (listed ? listed[gi * n + gj] : (uint8_t)1) : (uint8_t)0;
+        const int64_t i = bi + r, j = bj + tx;
+        const bool in2 = i < n && j < n;
+        dij[q] = in2 ? D[i * n + j] : 0.0;
+        lij[q] = in2 ? (listed ? listed[i * n + j] : (uint8_t)1) : (uint8_t)0;
     }
     __syncthreads();
-    for (int r = ty; r < kTile; r += 8) {
+#pragma unroll
+    for (int q = 0; q < kTile / 8; ++q) {
+        const int r = ty + 8 * q;
         const int64_t i = bi + r, j = bj + tx;
         if (i >= n || j >= n) continue;
-        const double dij = D[i * n + j];           // D_ij: value of s_ji
-        const double dji = tD[r][tx];              // D_ji: value of s_ij
-        const bool lij = listed ? listed[i * n + j] != 0 : true;   // j listed for point i
-        const bool lji = tL[r][tx] != 0;                              // i listed for point j
-        const double sij = (lij && i != j && dji >= kZeroDist) ? sqrt(dji) : 0.0;
-        const double sji = (lji && i != j && dij >= kZeroDist) ? sqrt(dij) : 0.0;
-        const double y = sij * sij + sji * sji - sij * sji;
-        const bool zero_edge = lij && (i == j || dji < kZeroDist);
-        Y[i * n + j] = (y != 0.0 || zero_edge) ? y : -1.0;
+        const double dji = tY[tx][r];                          // D_ji
+        const bool l1 = lij[q] != 0, l2 = tL[tx][r] != 0;      // j listed for i, i listed for j
+        const bool u1 = l1 && i != j && dji >= kZeroDist;      // s_ij = sqrt(D_ji)
+        const bool u2 = l2 && i != j && dij[q] >= kZeroDist;   // s_ji = sqrt(D_ij)
+        const double rji = (u1 || u2) ? sqrt(dji) : 0.0;
+        const double sij = u1 ? rji : 0.0;
+        const double sji = u2 ? (dij[q] == dji ? rji : sqrt(dij[q])) : 0.0;
+        Y[i * n + j] = dm_pair_value(sij, sji, l1 && (i == j || dji < kZeroDist));
+        // this thread alone reads and writes element (tx, r) of the shared tile
+        tY[tx][r] = dm_pair_value(sji, sij, l2 && (i == j || dij[q] < kZeroDist));
+    }
+    if (bi == bj) return;                          // the diagonal tile is complete
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kTile / 8; ++q) {
+        const int r = ty + 8 * q;
+        if (bj + r < n && bi + tx < n) Y[(bj + r) * n + bi + tx] = tY[r][tx];
     }
 }
 
-// 2. sweep partial sums; every thread holds kPer entries of Y and walks all the log eps values
-constexpr int kSweepThreads = 256, kPer = 8, kMaxEps = 2048;
+// 2. Sweep.  Every thread holds kPer entries of Y and would walk all the log eps values, but for
+// most of them a warp's 256 entries are all beyond the threshold (a term is 0, except a zero
+// distance's 1) or all so close that exp rounds to 1: a term lies strictly between only while
+// d = Y/(2 eps) runs from the threshold down to 2^-26, about 20 of the sweep's 300 in ln eps.  So
+// per chunk of entries the CTA first classifies every log eps from each warp's smallest positive
+// and largest Y, adds the exact counts where all its warps are trivial, and evaluates the listed
+// rest.  Float sums per warp and their order are those of a full evaluation; a block keeps the
+// FP64 sums of all its chunks in shared memory and adds them to global memory once.
+// NT: 256 threads (2048 entries per chunk), or 64 while there are fewer than two such chunks per
+// SM, so that n = 300 runs on 152 SMs instead of 44.
+constexpr int kPer = 8, kMaxEps = 2048;
+constexpr int kSweepList = 256;                   // listed scales evaluated between two barriers
+constexpr float kExpOne = 1.4901161193847656e-8f; // 2^-26: exp2f(-d) = 1 for 0 <= d <= 2^-26
 
-__global__ void __launch_bounds__(kSweepThreads) dm_sweep_kernel(
+template <int NT>
+__global__ void __launch_bounds__(NT) dm_sweep_kernel(
         const double* __restrict__ Y, int64_t total, const float* __restrict__ scale,
-        int n_eps, float thr, double* __restrict__ sums) {
+        int n_eps, float thr, int aligned, double* __restrict__ sums) {
+    constexpr int NW = NT / 32;
     __shared__ double part[kMaxEps];
-    for (int e = threadIdx.x; e < n_eps; e += kSweepThreads) part[e] = 0.0;
-    float y[kPer];
-    const int64_t base = ((int64_t)blockIdx.x * kSweepThreads + threadIdx.x) * kPer;
+    __shared__ uint16_t list[kMaxEps];
+    __shared__ float wsum[kSweepList][NW];
+    __shared__ float wmin[NW], wmax[NW];
+    __shared__ int wzero[NW], wedge[NW], n_list;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    for (int e = t; e < n_eps; e += NT) part[e] = 0.0;
+    const float tl = thr * 1.4426950408889634f;   // the threshold on d = Y/(2 eps), base 2
+    constexpr int64_t per_block = (int64_t)NT * kPer;
+    const int64_t chunks = (total + per_block - 1) / per_block;
+    for (int64_t ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
+        float y[kPer];
+        const int64_t base = ch * per_block + (int64_t)t * kPer;
+        if (aligned && base + kPer <= total) {    // Y on a 16-byte boundary
+            const double2* p = reinterpret_cast<const double2*>(Y + base);
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-        const int64_t g = base + u;
-        y[u] = g < total ? (float)Y[g] : -1.0f;     // -1: not an edge
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    for (int e = 0; e < n_eps; ++e) {
-        const float c = scale[e];                   // log2(e) / (2 eps)
-        const float tl = thr * 1.4426950408889634f; // the threshold on d = Y/(2 eps), base 2
-        float acc = 0.f;
+            for (int u = 0; u < kPer / 2; ++u) {
+                const double2 v = p[u];
+                y[2 * u] = (float)v.x;
+                y[2 * u + 1] = (float)v.y;
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < kPer; ++u)
+                y[u] = base + u < total ? (float)Y[base + u] : -1.0f;    // -1: not an edge
+        }
+        float lo = __int_as_float(0x7f800000), hi = 0.f;
+        int zero = 0, edge = 0;
 #pragma unroll
         for (int u = 0; u < kPer; ++u) {
-            // d log2(e); scale is +inf for the smallest eps (beyond float range): zero-distance
-            // edges still give exp(0) = 1 there, all others are beyond the threshold
-            const float d2 = y[u] == 0.f ? 0.f : y[u] * c;
-            acc += (y[u] >= 0.f && d2 < tl) ? exp2f(-d2) : 0.f;
+            if (y[u] > 0.f) {
+                lo = fminf(lo, y[u]);
+                hi = fmaxf(hi, y[u]);
+            }
+            zero += y[u] == 0.f;
+            edge += y[u] >= 0.f;
         }
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0 && acc != 0.f) atomicAdd(&part[e], (double)acc);
+        for (int o = 16; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        zero = __reduce_add_sync(0xffffffffu, zero);
+        edge = __reduce_add_sync(0xffffffffu, edge);
+        __syncthreads();                          // the last chunk's lists and sums are done with
+        if (lane == 0) {
+            wmin[warp] = lo;
+            wmax[warp] = hi;
+            wzero[warp] = zero;
+            wedge[warp] = edge;
+        }
+        if (t == 0) n_list = 0;
+        __syncthreads();
+        for (int e = t; e < n_eps; e += NT) {
+            const float c = scale[e];             // log2(e) / (2 eps)
+            int ones = 0;
+            bool todo = false;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) {
+                const bool none = wedge[w] == wzero[w];         // no positive entry
+                const float dmax = wmax[w] * c;
+                if (none || wmin[w] * c >= tl)
+                    ones += 0.f < tl ? wzero[w] : 0;
+                else if (dmax >= 0.f && dmax <= kExpOne && dmax < tl)
+                    ones += wedge[w];
+                else
+                    todo = true;
+            }
+            if (todo)
+                list[atomicAdd(&n_list, 1)] = (uint16_t)e;
+            else if (ones)
+                part[e] += (double)ones;
+        }
+        __syncthreads();
+        const int nl = n_list;
+        for (int l0 = 0; l0 < nl; l0 += kSweepList) {
+            const int l1 = min(nl, l0 + kSweepList);
+#pragma unroll 2
+            for (int l = l0; l < l1; ++l) {
+                const float c = scale[list[l]];
+                float acc = 0.f;
+#pragma unroll
+                for (int u = 0; u < kPer; ++u) {
+                    // d log2(e); scale is +inf for the smallest eps (beyond float range):
+                    // zero-distance edges still give exp(0) = 1 there, all others are beyond
+                    // the threshold
+                    const float d2 = y[u] == 0.f ? 0.f : y[u] * c;
+                    acc += (y[u] >= 0.f && d2 < tl) ? exp2f(-d2) : 0.f;
+                }
+                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                if (lane == 0) wsum[l - l0][warp] = acc;
+            }
+            __syncthreads();
+            for (int i = t; i < l1 - l0; i += NT) {
+                double s = 0.0;
+#pragma unroll
+                for (int w = 0; w < NW; ++w) s += (double)wsum[i][w];
+                part[list[l0 + i]] += s;
+            }
+            __syncthreads();
+        }
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < n_eps; e += kSweepThreads)
+    for (int e = t; e < n_eps; e += NT)
         if (part[e] != 0.0) atomicAdd(&sums[e], part[e]);
 }
 
-// 3a. W = exp(-Y / sigma^2) on edges (in place over Y) and its column sums
-__global__ void dm_weights_kernel(double* __restrict__ W, int64_t n, double inv_s2,
-                                  double* __restrict__ colsum) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    double s = 0.0;
-    for (int64_t i = 0; i < n; ++i) {
-        const double y = W[i * n + j];
-        const double w = y >= 0.0 ? exp(-y * inv_s2) : 0.0;
-        W[i * n + j] = w;
-        s += w;
+// 3. The normalised kernel, four launches over W (in L2 up to n = 4000):
+//   a. W = exp(-Y / sigma^2) on edges, in place, tile pairs as in dm_sym_kernel: one FP64 exp
+//      for both entries of a pair where Y_ij = Y_ji;
+//   b. d = column sums of W;
+//   c. e_j = sqrt(sum_i W_ij / (d_i d_j)), from reciprocals 1/d kept per row;
+//   d. L_ij = W_ij f_i f_j with f = 1 / (d e), L = |L + L^T| / 2, tile pairs.
+// A column sum is split over the rows of a 16-column slice (64 row threads, added in a fixed
+// order), so that n = 300 already fills 19 SMs and n = 3000 all of them; one thread per column
+// walking all rows took 2498 + 1564 us at n = 3000 (now 162 + 34 + 30) and 249 + 148 us at
+// n = 300 (the whole embedding work there: 85 us now, 918 us before).
+__global__ void __launch_bounds__(256) dm_weights_kernel(double* __restrict__ W, int64_t n,
+                                                         double inv_s2) {
+    __shared__ double tb[kTile][kTile + 1];
+    const int64_t bi = (int64_t)blockIdx.y * kTile, bj = (int64_t)blockIdx.x * kTile;
+    if (bj < bi) return;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    double a[kTile / 8];
+#pragma unroll
+    for (int q = 0; q < kTile / 8; ++q) {
+        const int r = ty + 8 * q;
+        tb[r][tx] = (bj + r < n && bi + tx < n) ? W[(bj + r) * n + bi + tx] : -1.0;
+        a[q] = (bi + r < n && bj + tx < n) ? W[(bi + r) * n + bj + tx] : -1.0;
     }
-    colsum[j] = s;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kTile / 8; ++q) {
+        const int r = ty + 8 * q;
+        const double yij = a[q], yji = tb[tx][r];
+        const double wij = yij >= 0.0 ? exp(-yij * inv_s2) : 0.0;
+        const double wji = yji == yij ? wij : (yji >= 0.0 ? exp(-yji * inv_s2) : 0.0);
+        if (bi + r < n && bj + tx < n) W[(bi + r) * n + bj + tx] = wij;
+        tb[tx][r] = wji;
+    }
+    if (bi == bj) return;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kTile / 8; ++q) {
+        const int r = ty + 8 * q;
+        if (bj + r < n && bi + tx < n) W[(bj + r) * n + bi + tx] = tb[r][tx];
+    }
 }
 
-// 3b. W'_ij = W_ij / (d_i d_j) in place, and e_j = sqrt(column sums of W')
-__global__ void dm_normalise_kernel(double* __restrict__ W, int64_t n,
-                                    const double* __restrict__ d, double* __restrict__ e) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const double dj = d[j];
+// column sums of a 16-column slice: first = d (PASS 0: 1 / d to out), then e (PASS 1: out = f)
+constexpr int kColW = 16, kColRows = 64;
+template <int PASS>
+__global__ void __launch_bounds__(kColW* kColRows) dm_colsum_kernel(
+        const double* __restrict__ W, int64_t n, const double* __restrict__ rd,
+        double* __restrict__ out) {
+    __shared__ double part[kColRows][kColW + 1];
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int64_t j = (int64_t)blockIdx.x * kColW + tx;
     double s = 0.0;
-    for (int64_t i = 0; i < n; ++i) {
-        const double w = W[i * n + j] / (d[i] * dj);
-        W[i * n + j] = w;
-        s += w;
+    if (j < n) {
+#pragma unroll 4
+        for (int64_t i = ty; i < n; i += kColRows) {
+            const double w = W[i * n + j];
+            s = PASS == 0 ? s + w : fma(w, rd[i], s);
+        }
     }
-    e[j] = sqrt(s);
+    part[ty][tx] = s;
+    __syncthreads();
+    for (int h = kColRows / 2; h > 0; h >>= 1) {
+        if (ty < h) part[ty][tx] += part[ty + h][tx];
+        __syncthreads();
+    }
+    if (ty == 0 && j < n)
+        out[j] = PASS == 0 ? 1.0 / part[0][tx] : rd[j] / sqrt(part[0][tx] * rd[j]);
 }
 
-// 3c. L_ij = W'_ij / (e_i e_j), then L = |L + L^T| / 2 (tile pairs (bi, bj), (bj, bi))
-__global__ void dm_finish_kernel(double* __restrict__ W, int64_t n, const double* __restrict__ e) {
-    __shared__ double ta[kTile][kTile + 1], tb[kTile][kTile + 1];
+// L_ij = W_ij f_i f_j, then L = |L + L^T| / 2 (tile pairs (bi, bj), (bj, bi))
+__global__ void __launch_bounds__(256) dm_finish_kernel(double* __restrict__ W, int64_t n,
+                                                        const double* __restrict__ f) {
+    __shared__ double tb[kTile][kTile + 1];
     const int64_t bi = (int64_t)blockIdx.y * kTile, bj = (int64_t)blockIdx.x * kTile;
     if (bj < bi) return;                           // each unordered tile pair once
     const int tx = threadIdx.x, ty = threadIdx.y;
-    for (int r = ty; r < kTile; r += 8) {
-        const int64_t i = bi + r, j = bj + tx;
-        ta[r][tx] = (i < n && j < n) ? W[i * n + j] / (e[i] * e[j]) : 0.0;
-        const int64_t i2 = bj + r, j2 = bi + tx;
-        tb[r][tx] = (i2 < n && j2 < n) ? W[i2 * n + j2] / (e[i2] * e[j2]) : 0.0;
+    double a[kTile / 8];
+#pragma unroll
+    for (int q = 0; q < kTile / 8; ++q) {
+        const int r = ty + 8 * q;
+        tb[r][tx] = (bj + r < n && bi + tx < n) ? W[(bj + r) * n + bi + tx] : 0.0;
+        a[q] = (bi + r < n && bj + tx < n) ? W[(bi + r) * n + bj + tx] : 0.0;
     }
     __syncthreads();
-    for (int r = ty; r < kTile; r += 8) {
-        const int64_t i = bi + r, j = bj + tx;
-        if (i < n && j < n) W[i * n + j] = fabs(ta[r][tx] + tb[tx][r]) / 2.0;
-        const int64_t i2 = bj + r, j2 = bi + tx;
-        if (i2 < n && j2 < n) W[i2 * n + j2] = fabs(tb[r][tx] + ta[tx][r]) / 2.0;
+    const double fj = bj + tx < n ? f[bj + tx] : 0.0;
+#pragma unroll
+    for (int q = 0; q < kTile / 8; ++q) {
+        const int r = ty + 8 * q;
+        const double fi = bi + r < n ? f[bi + r] : 0.0;
+        const double v = fabs((a[q] + tb[tx][r]) * (fi * fj)) / 2.0;
+        if (bi + r < n && bj + tx < n) W[(bi + r) * n + bj + tx] = v;
+        tb[tx][r] = v;
+    }
+    if (bi == bj) return;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kTile / 8; ++q) {
+        const int r = ty + 8 * q;
+        if (bj + r < n && bi + tx < n) W[(bj + r) * n + bi + tx] = tb[r][tx];
     }
 }
 
@@ -164,9 +334,16 @@ int mem_dm_sweep(const double* Y, int64_t n, const float* scale, int32_t n_eps, 
     cudaStream_t s = (cudaStream_t)stream;
     MEM_CUDA_TRY(cudaMemsetAsync(sums, 0, sizeof(double) * n_eps, s));
     const int64_t total = n * n;
-    const int64_t per_block = (int64_t)kSweepThreads * kPer;
-    dm_sweep_kernel<<<(unsigned)((total + per_block - 1) / per_block), kSweepThreads, 0, s>>>(
-            Y, total, scale, n_eps, (float)thr, sums);
+    // persistent: as many CTAs as fit the SMs at most, each adding its sums to global memory once
+    const int aligned = (reinterpret_cast<uintptr_t>(Y) & 15) == 0;
+    const int64_t wide = (total + 256 * kPer - 1) / (256 * kPer);
+    const int64_t narrow = (total + 64 * kPer - 1) / (64 * kPer);
+    if (wide >= 2 * 152)
+        dm_sweep_kernel<256><<<(unsigned)std::min<int64_t>(wide, 4 * 152), 256, 0, s>>>(
+                Y, total, scale, n_eps, (float)thr, aligned, sums);
+    else
+        dm_sweep_kernel<64><<<(unsigned)std::min<int64_t>(narrow, 8 * 152), 64, 0, s>>>(
+                Y, total, scale, n_eps, (float)thr, aligned, sums);
     MEM_LAUNCH_CHECK();
     return MEM_OK;
 }
@@ -174,13 +351,16 @@ int mem_dm_sweep(const double* Y, int64_t n, const float* scale, int32_t n_eps, 
 int mem_dm_laplacian(double* Y, int64_t n, double sigma, double* scratch, void* stream) {
     if (!Y || !scratch || n < 1 || !(sigma > 0.0)) return MEM_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
-    const unsigned nb1 = (unsigned)((n + 127) / 128);
-    dm_weights_kernel<<<nb1, 128, 0, s>>>(Y, n, 1.0 / (sigma * sigma), scratch);
-    MEM_LAUNCH_CHECK();
-    dm_normalise_kernel<<<nb1, 128, 0, s>>>(Y, n, scratch, scratch + n);
-    MEM_LAUNCH_CHECK();
     const unsigned nb = (unsigned)((n + kTile - 1) / kTile);
-    dm_finish_kernel<<<dim3(nb, nb), dim3(kTile, 8), 0, s>>>(Y, n, scratch + n);
+    const unsigned nc = (unsigned)((n + kColW - 1) / kColW);
+    double *rd = scratch, *f = scratch + n;
+    dm_weights_kernel<<<dim3(nb, nb), dim3(kTile, 8), 0, s>>>(Y, n, 1.0 / (sigma * sigma));
+    MEM_LAUNCH_CHECK();
+    dm_colsum_kernel<0><<<nc, dim3(kColW, kColRows), 0, s>>>(Y, n, nullptr, rd);
+    MEM_LAUNCH_CHECK();
+    dm_colsum_kernel<1><<<nc, dim3(kColW, kColRows), 0, s>>>(Y, n, rd, f);
+    MEM_LAUNCH_CHECK();
+    dm_finish_kernel<<<dim3(nb, nb), dim3(kTile, 8), 0, s>>>(Y, n, f);
     MEM_LAUNCH_CHECK();
     return MEM_OK;
 }
