@@ -3,7 +3,9 @@ plain FP64 numpy.
 
 Tolerances: the bandwidth sweep evaluates exp in float32 (2 ulp) and adds at most 256 terms in
 float32, so a sum is within 8 * 2^-24 + 2 * 2^-24 < 1e-6 of FP64; the normalised kernel is FP64
-throughout (a few 2^-53 per operation, sums of n terms: 1e-12).
+throughout (a few 2^-53 per operation, sums of n terms: 1e-12); a projected mask is a comparison
+whose undecided pixels are summed in FP64, so it equals FP64 wherever the sum is not within 1e-9
+of the threshold.
 """
 import ctypes
 import math
@@ -89,3 +91,74 @@ def test_embedding_kernels(cuda_ready, n, asym, knn):
         L = W / (r[:, None] * r[None])
         L = np.abs(L + L.T) / 2
         assert np.abs(y.cpu().numpy().reshape(n, n) - L).max() <= 1e-12 * L.max()
+
+
+def _spline_sums(P, N, T):
+    """sum_k of the clamped cubic spline of P (M^3, 12 samples of padding) along each line."""
+    M = P.shape[0]
+    i, j, k = np.meshgrid(*(np.arange(N, dtype=np.float64),) * 3, indexing='ij')
+    w, f = [], []
+    for a in range(3):
+        u = T[3 * a] * i + T[3 * a + 1] * j + T[3 * a + 2] * k + T[9 + a]
+        fl = np.floor(u)
+        t = u - fl
+        v = 1 - t
+        w.append((v ** 3 / 6, 2 / 3 - t * t * (1 - t / 2), 2 / 3 - v * v * (1 - v / 2),
+                  t ** 3 / 6))
+        f.append(fl.astype(np.int64))
+    out = 0.0
+    for a in range(4):
+        ia = np.clip(12 + f[0] - 1 + a, 0, M - 1)
+        for b in range(4):
+            ib = np.clip(12 + f[1] - 1 + b, 0, M - 1)
+            for c in range(4):
+                ic = np.clip(12 + f[2] - 1 + c, 0, M - 1)
+                out = out + w[0][a] * w[1][b] * w[2][c] * P[ia, ib, ic]
+    return out.sum(2)
+
+
+@pytest.mark.parametrize('N', [2, 15, 16, 17, 33, 48])
+def test_mask_projection(cuda_ready, N):
+    """Rotations, the identity (whole sums at the threshold), and maps that are no rotation
+    (scaled up: the box does not fit; scaled down; far outside the volume)."""
+    torch = cuda_ready
+    from manifoldem_python_gb300 import _lib
+    rng = np.random.default_rng(N)
+    vol = np.zeros((N, N, N), np.float32)
+    vol[N // 4:N - N // 4, N // 4:N - N // 3, N // 3:N - N // 4] = 0.37
+    vol += (rng.random((N, N, N)) < 0.02) * rng.standard_normal((N, N, N)) * 2
+    vol = vol.astype(np.float32)
+    size = ctypes.c_size_t()
+    _lib.check(_lib.load().mem_mask_coefficients_size(N, ctypes.byref(size)), 'size')
+    C = torch.empty(size.value // 8, dtype=torch.float64, device='cuda')
+    v = torch.from_numpy(vol).cuda()
+    _call(torch, 'mem_mask_prepare', v.data_ptr(), N, C.data_ptr())
+    xf = []
+    for k in range(5):
+        q = rng.standard_normal(4)
+        w, x, y, z = q / np.linalg.norm(q)
+        R = np.array([[1 - 2 * (y * y + z * z), 2 * (x * y - w * z), 2 * (x * z + w * y)],
+                      [2 * (x * y + w * z), 1 - 2 * (x * x + z * z), 2 * (y * z - w * x)],
+                      [2 * (x * z - w * y), 2 * (y * z + w * x), 1 - 2 * (x * x + y * y)]])
+        if k == 0:
+            R = np.eye(3)
+        if k == 3:
+            R = 3.0 * R
+        if k == 4:
+            R = 0.2 * R
+        off = np.full(3, N / 2) - R @ np.full(3, N / 2)
+        if k == 2:
+            off = off + np.array([4.0 * N, -0.3, 0.2])
+        xf.append(np.concatenate([R.reshape(-1), off]))
+    xf.append(np.concatenate([np.eye(3).reshape(-1), [3e5, 0.0, 0.0]]))
+    xf = np.array(xf)
+    out = torch.empty((len(xf), N, N), dtype=torch.uint8, device='cuda')
+    xd = torch.from_numpy(xf).cuda()
+    _call(torch, 'mem_mask_project', C.data_ptr(), N, len(xf), xd.data_ptr(), out.data_ptr())
+    M = N + 24
+    P = C.cpu().numpy().reshape(M, M, M)
+    got = out.cpu().numpy()
+    for k in range(len(xf)):
+        sums = _spline_sums(P, N, xf[k]).T
+        sure = np.abs(sums - 1) > 1e-9
+        assert np.array_equal(got[k][sure] > 0, sums[sure] > 1), k
