@@ -648,49 +648,179 @@ __device__ __forceinline__ float ctf_eval(int m, uint64_t qf, const CtfConst& cc
 // 4. per-PD sums over images (partial, one item = up to kSumChunk images of one PD)
 //    S0 = sum C^2, S1/S2 = sum C F, S3/S4 = sum sign(C) F, S5 = sum |F|^2
 // ------------------------------------------------------------------------------------------
-// WHICH: 1 = S0..S2 (the Wiener sums), 2 = S3..S5, 3 = all six
+// WHICH: 1 = S0..S2 (the Wiener sums), 2 = S3..S5, 3 = all six.  Every sum is one compensated
+// chain over the item's images in order, whichever kernel runs it (the results are the same bits).
+//
+// pd_sums_kernel: a thread owns the frequencies (ka, kb) and (N - ka, kb), which share |k|^2 and so
+// the CTF: its evaluation (half of a thread's instructions) serves both.  Issue-bound: 10.6 K
+// images of 128 px take 176 us, 219 us with one frequency per thread.
 template <int WHICH>
-__global__ void __launch_bounds__(256) pd_sums_kernel(
+__global__ void __launch_bounds__(128) pd_sums_kernel(
         const float2* __restrict__ spec, const uint64_t* __restrict__ qfix,
         const SumItem* __restrict__ items, float* __restrict__ partial, int N, int Nh, int64_t Kc,
         CtfConst cc) {
-    const int64_t k = blockIdx.y * 256ll + threadIdx.x;
+    constexpr int B = 4;
+    const int e = blockIdx.y * 128 + threadIdx.x;
     const SumItem it = items[blockIdx.x];
-    if (k < Kc) {
-        const int ka = (int)(k / Nh), kb = (int)(k - (int64_t)ka * Nh);
-        const int fa = min(ka, N - ka);
-        const int m = fa * fa + kb * kb;
-        KSum2 s05, s12, s34;        // (S0, S5), (S1, S2), (S3, S4)
-#pragma unroll 4
-        for (int64_t i = it.img_begin; i < it.img_end; ++i) {
-            const float2 F = spec[i * Kc + k];
-            int sg;
-            float C = 0.f;
-            if (WHICH & 1) {
-                C = ctf_eval(m, qfix[i], cc, &sg);
-                s12.add(__fmul2_rn(make_float2(C, C), F));
-            } else {
-                sg = ctf_sign(m, qfix[i], cc);
-            }
-            if (WHICH & 2) {
-                const float g = (float)sg;
-                s34.add(__fmul2_rn(make_float2(g, g), F));
-            }
-            s05.add(make_float2((WHICH & 1) ? C * C : 0.f,
-                                (WHICH & 2) ? F.x * F.x + F.y * F.y : 0.f));
+    const int ka = e / Nh, kb = e - ka * Nh;
+    if (ka > N / 2) return;
+    const int kp = ka == 0 ? 0 : N - ka;            // the mirrored row (itself for 0 and N/2)
+    const int m = ka * ka + kb * kb;
+    const int64_t k0 = (int64_t)ka * Nh + kb, k1 = (int64_t)kp * Nh + kb;
+    KSum s0;
+    KSum2 s55, s12[2], s34[2];                      // (S5, S5'), (S1, S2), (S3, S4)
+    // the next B images are loaded before the last B are added
+    const int n = (int)(it.img_end - it.img_begin);
+    const float2* p0 = spec + it.img_begin * Kc + k0;
+    const float2* p1 = spec + it.img_begin * Kc + k1;
+    const uint64_t* qp = qfix + it.img_begin;
+    float2 F[B][2];
+    uint64_t q[B];
+    auto load = [&](int i0) {
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const int64_t i = min(i0 + u, n - 1);
+            F[u][0] = p0[i * Kc];
+            F[u][1] = p1[i * Kc];
+            q[u] = qp[i];
         }
-        float* out = partial + (int64_t)blockIdx.x * 6 * Kc + k;
-        const float2 v05 = s05.value(), v12 = s12.value(), v34 = s34.value();
+    };
+    auto add = [&](const float2 (&G)[2], uint64_t qf) {
+        int sg;
         if (WHICH & 1) {
-            out[0 * Kc] = v05.x;
+            const float C = ctf_eval(m, qf, cc, &sg);
+            s0.add(__fmul_rn(C, C));                  // rounded, as in the paired sums
+#pragma unroll
+            for (int h = 0; h < 2; ++h) s12[h].add(__fmul2_rn(make_float2(C, C), G[h]));
+        } else {
+            sg = ctf_sign(m, qf, cc);
+        }
+        if (WHICH & 2) {
+            const float g = (float)sg;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) s34[h].add(__fmul2_rn(make_float2(g, g), G[h]));
+            s55.add(make_float2(G[0].x * G[0].x + G[0].y * G[0].y,
+                                G[1].x * G[1].x + G[1].y * G[1].y));
+        }
+    };
+    load(0);
+    int i0 = 0;
+    for (; i0 + B <= n; i0 += B) {
+        float2 G[B][2];
+        uint64_t qg[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            G[u][0] = F[u][0];
+            G[u][1] = F[u][1];
+            qg[u] = q[u];
+        }
+        load(i0 + B);
+#pragma unroll
+        for (int u = 0; u < B; ++u) add(G[u], qg[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+        if (i0 + u < n) add(F[u], q[u]);
+    const float2 v55 = s55.value();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if (h == 1 && kp == ka) break;
+        float* out = partial + (int64_t)blockIdx.x * 6 * Kc + (h == 0 ? k0 : k1);
+        const float2 v12 = s12[h].value(), v34 = s34[h].value();
+        if (WHICH & 1) {
+            out[0 * Kc] = s0.value();
             out[1 * Kc] = v12.x;
             out[2 * Kc] = v12.y;
         }
         if (WHICH & 2) {
             out[3 * Kc] = v34.x;
             out[4 * Kc] = v34.y;
-            out[5 * Kc] = v05.y;
+            out[5 * Kc] = h == 0 ? v55.x : v55.y;
         }
+    }
+}
+
+// pd_sums_few_kernel: the same sums for a few items, where a thread that loads, evaluates and adds
+// its item's up to 256 images alone leaves the chip idle and is bound by that serial chain
+// (41 us for 300 images of 70 px).  32 frequencies per CTA: the four warps load and evaluate 8 of
+// 32 images each into shared memory, then warps 0, 1 and 2 each add one pair of sums over the 32,
+// double-buffered (12 us).
+template <int WHICH>
+__global__ void __launch_bounds__(128) pd_sums_few_kernel(
+        const float2* __restrict__ spec, const uint64_t* __restrict__ qfix,
+        const SumItem* __restrict__ items, float* __restrict__ partial, int N, int Nh, int64_t Kc,
+        CtfConst cc) {
+    constexpr int CH = 32;
+    __shared__ float2 sF[2][CH][32];
+    __shared__ float2 sC[2][CH][32];                // (C, sign C)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const SumItem it = items[blockIdx.x];
+    const int64_t k = blockIdx.y * 32ll + lane;
+    const bool valid = k < Kc;
+    const int kk = valid ? (int)k : 0;
+    const int ka = kk / Nh, kb = kk - ka * Nh;
+    const int fa = min(ka, N - ka);
+    const int m = fa * fa + kb * kb;
+    KSum2 sum;
+    int buf = 0;
+    constexpr int PW = CH / 4;                      // images per warp and chunk
+    float2 F[PW];
+    uint64_t qf[PW];
+    auto load = [&](int64_t i0) {                   // one chunk ahead of the sums
+#pragma unroll
+        for (int u = 0; u < PW; ++u) {
+            const int64_t i = min(i0 + warp * PW + u, it.img_end - 1);
+            F[u] = spec[i * Kc + kk];
+            qf[u] = qfix[i];
+        }
+    };
+    load(it.img_begin);
+    for (int64_t i0 = it.img_begin; i0 < it.img_end; i0 += CH, buf ^= 1) {
+        const int n = (int)min((int64_t)CH, it.img_end - i0);
+#pragma unroll
+        for (int u = 0; u < PW; ++u) {
+            int sg;
+            float C = 0.f;
+            if (WHICH & 1) C = ctf_eval(m, qf[u], cc, &sg);
+            else sg = ctf_sign(m, qf[u], cc);
+            sF[buf][warp * PW + u][lane] = F[u];
+            sC[buf][warp * PW + u][lane] = make_float2(C, (float)sg);
+        }
+        load(i0 + CH);
+        __syncthreads();                            // also: the last but one buffer is read
+        if (warp == 0) {
+            for (int j = 0; j < n; ++j) {
+                const float2 F = sF[buf][j][lane];
+                const float C = sC[buf][j][lane].x;
+                sum.add(make_float2((WHICH & 1) ? C * C : 0.f,
+                                    (WHICH & 2) ? F.x * F.x + F.y * F.y : 0.f));
+            }
+        } else if (warp == 1 && (WHICH & 1)) {
+            for (int j = 0; j < n; ++j) {
+                const float C = sC[buf][j][lane].x;
+                sum.add(__fmul2_rn(make_float2(C, C), sF[buf][j][lane]));
+            }
+        } else if (warp == 2 && (WHICH & 2)) {
+            for (int j = 0; j < n; ++j) {
+                const float g = sC[buf][j][lane].y;
+                sum.add(__fmul2_rn(make_float2(g, g), sF[buf][j][lane]));
+            }
+        }
+    }
+    if (!valid || warp == 3) return;
+    float* out = partial + (int64_t)blockIdx.x * 6 * Kc + k;
+    const float2 v = sum.value();
+    if (warp == 0) {
+        if (WHICH & 1) out[0 * Kc] = v.x;
+        if (WHICH & 2) out[5 * Kc] = v.y;
+    } else if (warp == 1) {
+        if (WHICH & 1) {
+            out[1 * Kc] = v.x;
+            out[2 * Kc] = v.y;
+        }
+    } else if (WHICH & 2) {
+        out[3 * Kc] = v.x;
+        out[4 * Kc] = v.y;
     }
 }
 
@@ -963,46 +1093,53 @@ __global__ void avg_store_kernel(const float* __restrict__ avg_real, double* __r
     if (img_avg_flip) img_avg_flip[e] = keep ? (double)avg_real[(pd * 2 + 1) * NN + p] : 0.0;
 }
 
-// 8. imgAllIntensity = mean_i imgAllFlip_i^2 (reference :400)
-__global__ void __launch_bounds__(256) intensity_kernel(
+// 8. imgAllIntensity = mean_i imgAllFlip_i^2 (reference :400).  V consecutive pixels per thread
+// (one V-float load per image), each pixel one compensated chain over the PD's images; the next
+// B images are loaded before the last B are added.  V = 4 where the PDs give enough threads,
+// V = 1 for fewer PDs: one PD of 2000 images of 128 px takes 69 us with V = 1, and 500 us with
+// the 4096 threads of V = 4 and a load at a time.
+template <int V>
+struct __align__(4 * V) FloatV {
+    float x[V];
+};
+
+template <int V, int NT>
+__global__ void __launch_bounds__(NT) intensity_kernel(
         const float* __restrict__ flip_imgs, const PdDev* __restrict__ pds,
         double* __restrict__ out, int NN) {
-    const int p = blockIdx.y * 256 + threadIdx.x;
+    constexpr int B = V == 1 ? 32 : 8;
+    const int p = (blockIdx.y * NT + threadIdx.x) * V;
     const int pd = blockIdx.x;
     if (p >= NN) return;
     const PdDev d = pds[pd];
-    KSum s;
-    for (int i = 0; i < d.n; ++i) {
-        const float v = flip_imgs[(d.img_off + i) * (int64_t)NN + p];
-        s.add(v * v);
+    const float* src = flip_imgs + d.img_off * (int64_t)NN + p;
+    KSum s[V];
+    FloatV<V> v[B];
+    auto load = [&](int i0) {
+#pragma unroll
+        for (int u = 0; u < B; ++u)
+            v[u] = *reinterpret_cast<const FloatV<V>*>(src + (int64_t)min(i0 + u, d.n - 1) * NN);
+    };
+    auto add = [&](const FloatV<V>& x) {
+#pragma unroll
+        for (int q = 0; q < V; ++q) s[q].add(x.x[q] * x.x[q]);
+    };
+    load(0);
+    int i0 = 0;
+    for (; i0 + B <= d.n; i0 += B) {
+        FloatV<V> w[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) w[u] = v[u];
+        load(i0 + B);
+#pragma unroll
+        for (int u = 0; u < B; ++u) add(w[u]);
     }
-    out[(int64_t)pd * NN + p] = (double)s.value() / d.n;
-}
-
-
-// the same for NN % 4 == 0 with four pixels per thread (16-byte loads: four times the bytes in
-// flight per load; each pixel's sum in the same order)
-__global__ void __launch_bounds__(256) intensity4_kernel(
-        const float* __restrict__ flip_imgs, const PdDev* __restrict__ pds,
-        double* __restrict__ out, int NN) {
-    const int q = blockIdx.y * 256 + threadIdx.x;
-    const int pd = blockIdx.x;
-    if (4 * q >= NN) return;
-    const PdDev d = pds[pd];
-    KSum s0, s1, s2, s3;
-    for (int i = 0; i < d.n; ++i) {
-        const float4 v =
-            reinterpret_cast<const float4*>(flip_imgs + (d.img_off + i) * (int64_t)NN)[q];
-        s0.add(v.x * v.x);
-        s1.add(v.y * v.y);
-        s2.add(v.z * v.z);
-        s3.add(v.w * v.w);
-    }
-    double* o = out + (int64_t)pd * NN + 4 * q;
-    o[0] = (double)s0.value() / d.n;
-    o[1] = (double)s1.value() / d.n;
-    o[2] = (double)s2.value() / d.n;
-    o[3] = (double)s3.value() / d.n;
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+        if (i0 + u < d.n) add(v[u]);
+    double* o = out + (int64_t)pd * NN + p;
+#pragma unroll
+    for (int q = 0; q < V; ++q) o[q] = (double)s[q].value() / d.n;
 }
 
 }  // namespace
@@ -1133,13 +1270,28 @@ int qfix(const mem_plan& P, const mem_inputs& in, uint64_t* qf, cudaStream_t s) 
 int pd_sums(const mem_plan& P, const float2* spec, const uint64_t* qf, const SumItem* items,
             float* partial, int which, cudaStream_t s) {
     if (P.items.empty()) return MEM_OK;
-    dim3 grid((unsigned)P.items.size(), (unsigned)((P.Kc + 255) / 256));
+    // one thread per frequency pair needs about 512 threads per SM to hide its loads; fewer items
+    // than that take the kernel that splits an item's evaluations over warps
+    const int64_t pairs = (int64_t)(P.N / 2 + 1) * P.Nh;
+    const bool few = (int64_t)P.items.size() * pairs < 152 * 512;
+    const dim3 grid((unsigned)P.items.size(),
+                    (unsigned)(few ? (P.Kc + 31) / 32 : (pairs + 127) / 128));
+#define MEM_SUMS(W)                                                                            \
+    do {                                                                                       \
+        if (few)                                                                               \
+            pd_sums_few_kernel<W><<<grid, 128, 0, s>>>(spec, qf, items, partial, P.N, P.Nh,    \
+                                                       P.Kc, P.ctf);                           \
+        else                                                                                   \
+            pd_sums_kernel<W><<<grid, 128, 0, s>>>(spec, qf, items, partial, P.N, P.Nh, P.Kc,  \
+                                                   P.ctf);                                     \
+    } while (0)
     if (which == 1)
-        pd_sums_kernel<1><<<grid, 256, 0, s>>>(spec, qf, items, partial, P.N, P.Nh, P.Kc, P.ctf);
+        MEM_SUMS(1);
     else if (which == 2)
-        pd_sums_kernel<2><<<grid, 256, 0, s>>>(spec, qf, items, partial, P.N, P.Nh, P.Kc, P.ctf);
+        MEM_SUMS(2);
     else
-        pd_sums_kernel<3><<<grid, 256, 0, s>>>(spec, qf, items, partial, P.N, P.Nh, P.Kc, P.ctf);
+        MEM_SUMS(3);
+#undef MEM_SUMS
     MEM_LAUNCH_CHECK();
     return MEM_OK;
 }
@@ -1211,13 +1363,15 @@ int intensity(const mem_plan& P, const float* flip_imgs, const PdDev* pds, doubl
               cudaStream_t s) {
     if (!out) return MEM_OK;
     const int NN = P.N * P.N;
-    // 16-byte loads need every image to start on a 16-byte boundary
-    if (NN % 4 == 0 && (reinterpret_cast<uintptr_t>(flip_imgs) & 15) == 0) {
-        dim3 grid((unsigned)P.n_pd, (unsigned)((NN / 4 + 255) / 256));
-        intensity4_kernel<<<grid, 256, 0, s>>>(flip_imgs, pds, out, NN);
+    // 16-byte loads need every image to start on a 16-byte boundary, and four pixels per thread
+    // enough PDs for about 1024 threads per SM
+    if (NN % 4 == 0 && (reinterpret_cast<uintptr_t>(flip_imgs) & 15) == 0 &&
+        (int64_t)P.n_pd * (NN / 4) >= 152 * 1024) {
+        dim3 grid((unsigned)P.n_pd, (unsigned)((NN / 4 + 127) / 128));
+        intensity_kernel<4, 128><<<grid, 128, 0, s>>>(flip_imgs, pds, out, NN);
     } else {
-        dim3 grid((unsigned)P.n_pd, (unsigned)((NN + 255) / 256));
-        intensity_kernel<<<grid, 256, 0, s>>>(flip_imgs, pds, out, NN);
+        dim3 grid((unsigned)P.n_pd, (unsigned)((NN + 63) / 64));
+        intensity_kernel<1, 64><<<grid, 64, 0, s>>>(flip_imgs, pds, out, NN);
     }
     MEM_LAUNCH_CHECK();
     return MEM_OK;

@@ -162,3 +162,40 @@ def test_mask_projection(cuda_ready, N):
         sums = _spline_sums(P, N, xf[k]).T
         sure = np.abs(sums - 1) > 1e-9
         assert np.array_equal(got[k][sure] > 0, sums[sure] > 1), k
+
+
+@pytest.mark.parametrize('N,n_pd', [(33, 280), (64, 75)])
+def test_sums_of_many_and_of_few_items(cuda_ready, N, n_pd):
+    """The per-PD sums and the mean intensity of a plan of many PDs (two frequencies per thread)
+    and of one PD alone (an item split over warps) are the same bits: every sum is one
+    compensated chain in both."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    rng = np.random.default_rng(N)
+    counts = [int(c) for c in rng.integers(1, 8, n_pd)]
+    counts[1] = 300                                        # two items of one PD
+    n = sum(counts)
+    stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
+    idx = torch.arange(n, device='cuda')
+    flip = torch.from_numpy(rng.integers(0, 2, n).astype(np.uint8)).cuda()
+    psi = torch.from_numpy(rng.uniform(-3, 3, n)).cuda()
+    df = torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda()
+    psi_p = rng.uniform(0, 360, n_pd)
+    params = StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1)
+    names = ('img_avg', 'img_avg_flip', 'img_all_intensity', 'D')
+    plan = Plan(params, counts, psi_p)
+    out = plan.allocate_outputs(names)
+    plan.execute(stack, idx, flip, psi, df, out)
+    a = 0
+    d = 0
+    for k in range(3):
+        s = slice(a, a + counts[k])
+        one = Plan(params, counts[k:k + 1], psi_p[k:k + 1])
+        o1 = one.allocate_outputs(names)
+        one.execute(stack, idx[s].contiguous(), flip[s].contiguous(), psi[s].contiguous(),
+                    df[s].contiguous(), o1)
+        for name in names[:3]:
+            assert torch.equal(out[name][k], o1[name][0]), (k, name)
+        assert torch.equal(out['D'][d:d + counts[k] ** 2], o1['D'])
+        a += counts[k]
+        d += counts[k] ** 2
