@@ -592,6 +592,11 @@ int mem_plan_upload(mem_plan* plan, void* workspace, size_t workspace_bytes, voi
     }
     MEM_CUDA_TRY(cudaMemcpyAsync(at<char>(workspace, L.twid), tw.data(), sizeof(float) * tw.size(),
                                  cudaMemcpyHostToDevice, s));
+    // the low-pass filter table, a function of the plan's parameters (12 us of FP64 pow)
+    {
+        const int st = kern::lowpass_table(P, at<float>(workspace, L.gtab), s);
+        if (st != MEM_OK) return st;
+    }
     // padding rows of the feature matrices stay zero for the whole life of the workspace
     const size_t feat_elem = (P.params.precision == MEM_PREC_FP32) ? 4 : 2;
     const size_t row_bytes = feat_elem * P.Kf;
@@ -685,7 +690,6 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     // the stack is read by exactly one kernel (the first), issued on the load stream
     MEM_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(uint32_t) * 4, ls));
     MEM_STEP(mark(0));
-    MEM_STEP(kern::lowpass_table(P, at<float>(ws, L.gtab), ls));
     mem_inputs lin = *in;
     const int64_t* ident = at<int64_t>(ws, L.ident);
     cudaStream_t cs = ls;                                // stream of the image arithmetic
@@ -763,7 +767,8 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
         return exec_fft(P, CUFFT_R2C, P.n_images, NN, specN, const_cast<float*>(images), spec,
                         work, s);
     };
-    if (!fused) MEM_STEP(spectrum(img_all));
+    // (a volume mask's first spectra, those of imgAll itself, serve the Wiener average only)
+    if (!fused && (!in->pd_mask || out->img_avg)) MEM_STEP(spectrum(img_all));
     MEM_STEP(mark(4));
     MEM_STEP(kern::qfix(P, *in, qf, s));
     float* partial = at<float>(ws, L.partial);
@@ -773,18 +778,27 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     const SumItem* items = at<SumItem>(ws, L.sum_items);
     const int32_t* item_off = at<int32_t>(ws, L.item_off);
     const FeatTables ft = feat_tables(P, at<char>(ws, L.colmap));
+    // the features serve D and its a_i, the sums serve the features and the averages: an image-only
+    // call (avg_only without averages, say) needs neither
+    const bool want_feat = (!P.params.avg_only && out->D) || out->pair_norm;
+    const bool want_sums = want_feat || out->img_avg || out->img_avg_flip;
+    const bool want_flip = out->img_all_flip || out->img_all_intensity;
     if (in->pd_mask) {
         // the Wiener average from the unmasked spectra, then everything else (centring vectors
         // included, so that they centre the features D is computed from) from the masked ones
-        MEM_STEP(kern::pd_sums(P, spec, qf, items, partial, 1, s));
-        MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
-                                   avg_spec, pd_max, 1, s));
+        if (out->img_avg) {
+            MEM_STEP(kern::pd_sums(P, spec, qf, items, partial, 1, s));
+            MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
+                                       avg_spec, pd_max, 1, s));
+        }
         MEM_STEP(kern::apply_pd_mask(P, img_all, xbuf, in->pd_mask, img_pd, s));
         MEM_STEP(spectrum(xbuf));
-        MEM_STEP(kern::pd_sums(P, spec, qf, items, partial, 3, s));
-        MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
-                                   avg_spec, pd_max, 2, s));
-    } else {
+        if (want_feat || out->img_avg_flip) {
+            MEM_STEP(kern::pd_sums(P, spec, qf, items, partial, 3, s));
+            MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
+                                       avg_spec, pd_max, 2, s));
+        }
+    } else if (want_sums) {
         MEM_STEP(kern::pd_sums(P, spec, qf, items, partial, 3, s));
         MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
                                    avg_spec, pd_max, 3, s));
@@ -795,9 +809,13 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     void* feat_b = at<char>(ws, L.feat_b);
     double* pair_norm = out->pair_norm ? out->pair_norm : at<double>(ws, L.pair_norm);
     const uint32_t* scale_bits = pd_max;
-    MEM_STEP(kern::features(P, spec, qf, pds, img_pd, img_row, ft, means,
-                            scale_bits, feat_a, feat_b, pair_norm, out->ctf, out->spectrum,
-                            !P.smem_fft && (out->img_all_flip || out->img_all_intensity), s));
+    const bool write_signed = !P.smem_fft && want_flip;
+    if (want_feat)
+        MEM_STEP(kern::features(P, spec, qf, pds, img_pd, img_row, ft, means, scale_bits, feat_a,
+                                feat_b, pair_norm, out->spectrum, write_signed, s));
+    else
+        MEM_STEP(kern::sign_spectrum(P, spec, qf, out->spectrum, write_signed, s));
+    MEM_STEP(kern::ctf(P, qf, out->ctf, s));
     MEM_STEP(mark(6));
     // averages: one inverse transform per PD (linearity of the reference's per-image sums)
     float* avg_real = at<float>(ws, L.avg_real);
@@ -810,7 +828,7 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     }
     MEM_STEP(mark(7));
     // phase-flipped images and their mean intensity
-    if (out->img_all_flip || out->img_all_intensity) {
+    if (want_flip) {
         float* flip_imgs = out->img_all_flip ? out->img_all_flip : xbuf;
         if (P.smem_fft)
             MEM_STEP(kern::inverse_fft(P, P.n_images, spec, twid, flip_imgs, qf, true, s));

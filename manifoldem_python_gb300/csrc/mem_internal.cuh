@@ -222,8 +222,13 @@ int pd_finalize(const mem_plan& P, const float* partial, const SumItem* items,
 int features(const mem_plan& P, float2* spec, const uint64_t* qf, const PdDev* pds,
              const int32_t* img_pd, const int32_t* img_row, const FeatTables& ft,
              const float* means, const uint32_t* scale_bits, void* feat_a, void* feat_b,
-             double* pair_norm, float* ctf_out, float* spectrum_out, bool write_signed,
-             cudaStream_t s);
+             double* pair_norm, float* spectrum_out, bool write_signed, cudaStream_t s);
+// the full-plane CTF of every image
+int ctf(const mem_plan& P, const uint64_t* qf, float* ctf_out, cudaStream_t s);
+// without features: copies the spectra to spectrum_out (may be null) and, with write_signed,
+// replaces them by sign(C) F / N^2
+int sign_spectrum(const mem_plan& P, float2* spec, const uint64_t* qf, float* spectrum_out,
+                  bool write_signed, cudaStream_t s);
 int avg_store(const mem_plan& P, const float* avg_real, double* img_avg, double* img_avg_flip,
               const uint8_t* pd_mask, cudaStream_t s);
 int intensity(const mem_plan& P, const float* flip_imgs, const PdDev* pds, double* out,

@@ -911,8 +911,7 @@ __global__ void __launch_bounds__(NT) features_kernel(
         const int32_t* __restrict__ img_row, const FeatTables ft,
         const float* __restrict__ means,
         const uint32_t* __restrict__ scale_bits, void* __restrict__ feat_a, void* __restrict__ feat_b,
-        double* __restrict__ pair_norm, float* __restrict__ ctf_out,
-        float2* __restrict__ spectrum_out, int N, int Nh, int64_t Kc, int64_t Kc_pad,
+        double* __restrict__ pair_norm, float2* __restrict__ spectrum_out, int N, int Nh, int64_t Kc, int64_t Kc_pad,
         int64_t Kr, int64_t Kr_pad, int64_t mstride, CtfConst cc, int write_signed,
         int pair_loads) {
     __shared__ double red[32];
@@ -1069,13 +1068,49 @@ __global__ void __launch_bounds__(NT) features_kernel(
     const double a = block_sum_double<NT>((double)acc.value() + (double)a2.x + (double)a2.y,
                                           red);
     if (threadIdx.x == 0) pair_norm[img] = a;
-    if (ctf_out) {
-        float* co = ctf_out + img * (int64_t)N * N;
-        for (int p = threadIdx.x; p < N * N; p += NT) {
-            const int r = p / N, c = p - r * N;
-            const int fa = min(r, N - r), fb = min(c, N - c);
-            int sg;
-            co[p] = ctf_eval(fa * fa + fb * fb, qf, cc, &sg);
+}
+
+// 6b. the CTF of every image over the full plane (the reference's CTF array).  One evaluation
+// serves the four mirrored elements (+-fa, +-fb): with one per element the evaluations took
+// twice as long as the writes (in the features kernel, 268 of its 860 us for 10.6 K images of
+// 128 px); a quarter of them leaves this kernel to the HBM writes (139 us, 5.0 TB/s).
+__global__ void __launch_bounds__(256) ctf_kernel(const uint64_t* __restrict__ qfix, int N,
+                                                  CtfConst cc, float* __restrict__ ctf) {
+    const int64_t img = blockIdx.x;
+    const uint64_t qf = qfix[img];
+    const int Nq = N / 2 + 1;
+    float* co = ctf + img * (int64_t)N * N;
+    for (int e = threadIdx.x; e < Nq * Nq; e += 256) {
+        const int fa = e / Nq, fb = e - fa * Nq;
+        int sg;
+        const float v = ctf_eval(fa * fa + fb * fb, qf, cc, &sg);
+        const int r[2] = {fa, fa ? N - fa : fa}, c[2] = {fb, fb ? N - fb : fb};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (h == 1 && r[1] == r[0]) break;
+            co[r[h] * N + c[0]] = v;
+            if (c[1] != c[0]) co[r[h] * N + c[1]] = v;
+        }
+    }
+}
+
+// 6c. without features (no D asked for): the caller's copy of the spectra, and sign(C) F / N^2 in
+// place for a phase-flip C2R that does not apply the sign itself
+__global__ void __launch_bounds__(256) sign_spectrum_kernel(
+        float2* __restrict__ spec, const uint64_t* __restrict__ qfix,
+        float2* __restrict__ spectrum_out, int N, int Nh, int64_t Kc, CtfConst cc,
+        int write_signed) {
+    const int64_t img = blockIdx.x;
+    const uint64_t qf = qfix[img];
+    const float inv_nn = 1.0f / ((float)N * (float)N);
+    for (int k = threadIdx.x; k < Kc; k += 256) {
+        const float2 F = spec[img * Kc + k];
+        if (spectrum_out) spectrum_out[img * Kc + k] = F;
+        if (write_signed) {
+            const int ka = k / Nh, kb = k - ka * Nh;
+            const int fa = min(ka, N - ka);
+            const float g = (float)ctf_sign(fa * fa + kb * kb, qf, cc) * inv_nn;
+            spec[img * Kc + k] = make_float2(g * F.x, g * F.y);
         }
     }
 }
@@ -1312,13 +1347,15 @@ int pd_finalize(const mem_plan& P, const float* partial, const SumItem* items,
 int features(const mem_plan& P, float2* spec, const uint64_t* qf, const PdDev* pds,
              const int32_t* img_pd, const int32_t* img_row, const FeatTables& ft,
              const float* means, const uint32_t* scale_bits, void* feat_a, void* feat_b,
-             double* pair_norm, float* ctf_out, float* spectrum_out, bool write_signed,
-             cudaStream_t s) {
+             double* pair_norm, float* spectrum_out, bool write_signed, cudaStream_t s) {
     if (P.n_images == 0) return MEM_OK;
     const size_t smem = P.ring_features ? sizeof(float) * P.Kc : 0;
     // 256 threads per image; 1024 when the ring table leaves room for fewer than three CTAs
     // per SM (large boxes: 126 KB at 250 px), so that the SM still holds 32 warps
     const bool wide = smem > 72 * 1024;
+    // paired loads: an even row count keeps every image's slots on 16 bytes if the first are
+    const bool pair_loads = P.Kc % 2 == 0 && (reinterpret_cast<uintptr_t>(spec) & 15) == 0 &&
+                            (reinterpret_cast<uintptr_t>(spectrum_out) & 15) == 0;
 #define MEM_FEATS_NT(MODE, RINGS, NT)                                                          \
     do {                                                                                       \
         MEM_CUDA_TRY(cudaFuncSetAttribute(features_kernel<MODE, RINGS, NT>,                    \
@@ -1326,8 +1363,8 @@ int features(const mem_plan& P, float2* spec, const uint64_t* qf, const PdDev* p
                                           (int)smem));                                         \
         features_kernel<MODE, RINGS, NT><<<(unsigned)P.n_images, NT, smem, s>>>(               \
             spec, qf, pds, img_pd, img_row, ft, means, scale_bits, feat_a, feat_b, pair_norm,  \
-            ctf_out, (float2*)spectrum_out, P.N, P.Nh, P.Kc, P.Kc_pad, P.Kr, P.Kr_pad,         \
-            means_stride(P), P.ctf, write_signed ? 1 : 0, P.Kc % 2 == 0 ? 1 : 0);              \
+            (float2*)spectrum_out, P.N, P.Nh, P.Kc, P.Kc_pad, P.Kr, P.Kr_pad, means_stride(P), \
+            P.ctf, write_signed ? 1 : 0, pair_loads ? 1 : 0);                                  \
     } while (0)
 #define MEM_FEATS(MODE, RINGS)                                                                 \
     do {                                                                                       \
@@ -1344,6 +1381,22 @@ int features(const mem_plan& P, float2* spec, const uint64_t* qf, const PdDev* p
     }
 #undef MEM_FEATS
 #undef MEM_FEATS_NT
+    MEM_LAUNCH_CHECK();
+    return MEM_OK;
+}
+
+int ctf(const mem_plan& P, const uint64_t* qf, float* ctf_out, cudaStream_t s) {
+    if (P.n_images == 0 || !ctf_out) return MEM_OK;
+    ctf_kernel<<<(unsigned)P.n_images, 256, 0, s>>>(qf, P.N, P.ctf, ctf_out);
+    MEM_LAUNCH_CHECK();
+    return MEM_OK;
+}
+
+int sign_spectrum(const mem_plan& P, float2* spec, const uint64_t* qf, float* spectrum_out,
+                  bool write_signed, cudaStream_t s) {
+    if (P.n_images == 0 || (!spectrum_out && !write_signed)) return MEM_OK;
+    sign_spectrum_kernel<<<(unsigned)P.n_images, 256, 0, s>>>(
+            spec, qf, (float2*)spectrum_out, P.N, P.Nh, P.Kc, P.ctf, write_signed ? 1 : 0);
     MEM_LAUNCH_CHECK();
     return MEM_OK;
 }
