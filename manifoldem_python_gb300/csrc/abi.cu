@@ -676,6 +676,8 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     const int32_t* img_row = at<int32_t>(ws, L.img_row);
     float* xbuf = at<float>(ws, L.xbuf);
     float2* spec = at<float2>(ws, L.spec);
+    // the spectra themselves: where the caller wants them, if the transforms leave them unsigned
+    float2* fspec = P.smem_fft && out->spectrum ? reinterpret_cast<float2*>(out->spectrum) : spec;
     uint64_t* qf = at<uint64_t>(ws, L.qfix);
     void* work = at<char>(ws, L.cufft_work);
     const int64_t NN = (int64_t)P.N * P.N;
@@ -734,7 +736,7 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
         MEM_STEP(mark(1));
         MEM_STEP(kern::rot_consts(P, *in, pds, img_pd, at<char>(ws, L.rotc), cs));
         MEM_STEP(kern::image_stage(P, lin, at<float>(ws, L.gtab), at<float2>(ws, L.twid), xbuf,
-                                   img_all, at<char>(ws, L.rotc), spec, status, cs));
+                                   img_all, at<char>(ws, L.rotc), fspec, status, cs));
     } else if (P.smem_fft) {
         // (a2, a3) gather, flip, normalisation and low-pass in one shared-memory pass
         MEM_STEP(mark(1));
@@ -762,13 +764,14 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     // average uses fft2(imgAll) (:355-359): its sums come from the unmasked spectra, then the
     // masked copy (in xbuf; in place when imgAll lives there) replaces them for the rest.
     const float2* twid = at<float2>(ws, L.twid);
-    auto spectrum = [&](const float* images) -> int {
-        if (P.smem_fft) return kern::spectrum_fft(P, P.n_images, images, twid, spec, s);
-        return exec_fft(P, CUFFT_R2C, P.n_images, NN, specN, const_cast<float*>(images), spec,
+    auto spectrum = [&](const float* images, const uint8_t* masks) -> int {
+        if (P.smem_fft)
+            return kern::spectrum_fft(P, P.n_images, images, masks, img_pd, twid, fspec, s);
+        return exec_fft(P, CUFFT_R2C, P.n_images, NN, specN, const_cast<float*>(images), fspec,
                         work, s);
     };
     // (a volume mask's first spectra, those of imgAll itself, serve the Wiener average only)
-    if (!fused && (!in->pd_mask || out->img_avg)) MEM_STEP(spectrum(img_all));
+    if (!fused && (!in->pd_mask || out->img_avg)) MEM_STEP(spectrum(img_all, nullptr));
     MEM_STEP(mark(4));
     MEM_STEP(kern::qfix(P, *in, qf, s));
     float* partial = at<float>(ws, L.partial);
@@ -787,19 +790,23 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
         // the Wiener average from the unmasked spectra, then everything else (centring vectors
         // included, so that they centre the features D is computed from) from the masked ones
         if (out->img_avg) {
-            MEM_STEP(kern::pd_sums(P, spec, qf, items, partial, 1, s));
+            MEM_STEP(kern::pd_sums(P, fspec, qf, items, partial, 1, s));
             MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
                                        avg_spec, pd_max, 1, s));
         }
-        MEM_STEP(kern::apply_pd_mask(P, img_all, xbuf, in->pd_mask, img_pd, s));
-        MEM_STEP(spectrum(xbuf));
+        if (P.smem_fft && kern::spectrum_masks_supported(P)) {
+            MEM_STEP(spectrum(img_all, in->pd_mask));
+        } else {
+            MEM_STEP(kern::apply_pd_mask(P, img_all, xbuf, in->pd_mask, img_pd, s));
+            MEM_STEP(spectrum(xbuf, nullptr));
+        }
         if (want_feat || out->img_avg_flip) {
-            MEM_STEP(kern::pd_sums(P, spec, qf, items, partial, 3, s));
+            MEM_STEP(kern::pd_sums(P, fspec, qf, items, partial, 3, s));
             MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
                                        avg_spec, pd_max, 2, s));
         }
     } else if (want_sums) {
-        MEM_STEP(kern::pd_sums(P, spec, qf, items, partial, 3, s));
+        MEM_STEP(kern::pd_sums(P, fspec, qf, items, partial, 3, s));
         MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
                                    avg_spec, pd_max, 3, s));
     }
@@ -810,11 +817,12 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     double* pair_norm = out->pair_norm ? out->pair_norm : at<double>(ws, L.pair_norm);
     const uint32_t* scale_bits = pd_max;
     const bool write_signed = !P.smem_fft && want_flip;
+    float* spectrum_out = P.smem_fft ? nullptr : out->spectrum;
     if (want_feat)
-        MEM_STEP(kern::features(P, spec, qf, pds, img_pd, img_row, ft, means, scale_bits, feat_a,
-                                feat_b, pair_norm, out->spectrum, write_signed, s));
+        MEM_STEP(kern::features(P, fspec, qf, pds, img_pd, img_row, ft, means, scale_bits, feat_a,
+                                feat_b, pair_norm, spectrum_out, write_signed, s));
     else
-        MEM_STEP(kern::sign_spectrum(P, spec, qf, out->spectrum, write_signed, s));
+        MEM_STEP(kern::sign_spectrum(P, spec, qf, spectrum_out, write_signed, s));
     MEM_STEP(kern::ctf(P, qf, out->ctf, s));
     MEM_STEP(mark(6));
     // averages: one inverse transform per PD (linearity of the reference's per-image sums)
@@ -831,7 +839,7 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     if (want_flip) {
         float* flip_imgs = out->img_all_flip ? out->img_all_flip : xbuf;
         if (P.smem_fft)
-            MEM_STEP(kern::inverse_fft(P, P.n_images, spec, twid, flip_imgs, qf, true, s));
+            MEM_STEP(kern::inverse_fft(P, P.n_images, fspec, twid, flip_imgs, qf, true, s));
         else
             MEM_STEP(exec_fft(P, CUFFT_C2R, P.n_images, specN, NN, spec, flip_imgs, work, s));
         MEM_STEP(kern::intensity(P, flip_imgs, pds, out->img_all_intensity, s));

@@ -612,7 +612,10 @@ int prepare(K kernel, size_t smem) {
 }  // namespace
 
 namespace kern {
-bool smem_fft_supported(const mem_plan& P) { return P.N == 32 || P.N == 64 || P.N == 128; }
+bool smem_fft_supported(const mem_plan& P) {
+    return P.N == 32 || P.N == 64 || P.N == 128 || mixed::supported(P.N);
+}
+bool spectrum_masks_supported(const mem_plan& P) { return mixed::supported(P.N); }
 
 #define MEM_FFT_DISPATCH(CALL)            \
     switch (P.N) {                        \
@@ -625,6 +628,8 @@ bool smem_fft_supported(const mem_plan& P) { return P.N == 32 || P.N == 64 || P.
 int lowpass_fused(const mem_plan& P, const mem_inputs& in, const float* gtab,
                   const float2* twid, float* xbuf, uint32_t* status, cudaStream_t s) {
     if (P.n_images == 0) return MEM_OK;
+    if (mixed::supported(P.N))
+        return mixed::lowpass(P.N, in, P.n_images, gtab, twid, xbuf, status, s);
     const size_t smem = (size_t)(P.N / 2) * P.N * sizeof(float2);
 #define MEM_CALL(NV)                                                                           \
     do {                                                                                       \
@@ -664,9 +669,12 @@ int image_stage(const mem_plan& P, const mem_inputs& in, const float* gtab, cons
     return MEM_OK;
 }
 
-int spectrum_fft(const mem_plan& P, int64_t count, const float* images, const float2* twid,
-                 float2* spec, cudaStream_t s) {
+int spectrum_fft(const mem_plan& P, int64_t count, const float* images, const uint8_t* masks,
+                 const int32_t* img_pd, const float2* twid, float2* spec, cudaStream_t s) {
     if (count == 0) return MEM_OK;
+    if (mixed::supported(P.N))
+        return mixed::spectrum(P.N, count, images, masks, img_pd, twid, spec, s);
+    if (masks) return MEM_ERR_UNSUPPORTED;
     const size_t smem = (size_t)(P.N / 2) * P.N * sizeof(float2);
 #define MEM_CALL(NV)                                                                           \
     do {                                                                                       \
@@ -682,6 +690,8 @@ int spectrum_fft(const mem_plan& P, int64_t count, const float* images, const fl
 int inverse_fft(const mem_plan& P, int64_t count, const float2* spec, const float2* twid,
                 float* images, const uint64_t* qf, bool signed_flip, cudaStream_t s) {
     if (count == 0) return MEM_OK;
+    if (mixed::supported(P.N))
+        return mixed::inverse(P.N, count, spec, twid, images, signed_flip ? qf : nullptr, P.ctf, s);
     const size_t smem = (size_t)(P.N / 2) * P.N * sizeof(float2);
 #define MEM_CALL(NV)                                                                           \
     do {                                                                                       \

@@ -126,7 +126,7 @@ struct mem_plan {
     int tc_group_chunks = 1;        // 64-wide K chunks per TMEM accumulation group (0 = all)
     bool tc_kahan = false;          // compensated register sums across groups
     bool tc_lolo = false;           // add the lo.lo product (4-term split)
-    bool smem_fft = true;           // shared-memory FFT kernels instead of cuFFT (N = 32, 64, 128)
+    bool smem_fft = true;           // shared-memory FFT kernels instead of cuFFT
     // N = 64, 128 without a volume mask: low-pass, rotations and spectrum in one kernel
     // (MEM_FUSED_IMAGE=1; off by default: measured slower than the three kernels, see
     // image_stage_kernel)
@@ -161,6 +161,18 @@ struct mem_plan {
 
 namespace mem {
 
+// ---- mixed-radix shared-memory transforms of even box sizes other than 32, 64, 128
+// (image_fft_mixed.cu); inverse: qf (or null) multiplies element k of image i by sign(C_i(k)) / N^2
+namespace mixed {
+bool supported(int N);
+int lowpass(int N, const mem_inputs& in, int64_t images, const float* gtab, const float2* twid,
+            float* xbuf, uint32_t* status, cudaStream_t s);
+int spectrum(int N, int64_t images, const float* src, const uint8_t* masks, const int32_t* img_pd,
+             const float2* twid, float2* spec, cudaStream_t s);
+int inverse(int N, int64_t images, const float2* spec, const float2* twid, float* dst,
+            const uint64_t* qf, const CtfConst& cc, cudaStream_t s);
+}  // namespace mixed
+
 // ---- batched 2D cuFFT transforms of N x N images (abi.cu): R2C image -> half-plane [N][N/2+1]
 // or C2R back, `count` transforms in chunks of kFftChunk from a per-(device, N, kind, batch) plan
 // cache; work is a caller-owned area of fft_work_bytes(N, type, count) bytes
@@ -177,7 +189,7 @@ int gather_copy(const mem_plan& P, const mem_inputs& in, float* out, uint32_t* s
                 int64_t ctas, cudaStream_t s);
 // multiply the half-plane spectra by the table G/N^2 written by lowpass_table
 int lowpass(const mem_plan& P, float2* spec, float* gtab, cudaStream_t s);
-bool smem_fft_supported(const mem_plan& P);
+bool smem_fft_supported(const mem_plan& P);   // 32, 64, 128 and the mixed-radix sizes
 int lowpass_table(const mem_plan& P, float* gtab, cudaStream_t s);
 int lowpass_fused(const mem_plan& P, const mem_inputs& in, const float* gtab,
                   const float2* twid, float* xbuf, uint32_t* status, cudaStream_t s);
@@ -187,9 +199,11 @@ int apply_pd_mask(const mem_plan& P, const float* src, float* dst, const uint8_t
 // RELION read: shifted images, laid out as SPIDER stack images, into out [n_images][N][N]
 int relion_shift(const mem_plan& P, const mem_inputs& in, float* out, uint32_t* status,
                  cudaStream_t s);
-// shared-memory real 2D FFTs (N = 32, 64, 128) with the layout and scaling of a cuFFT R2C/C2R
-int spectrum_fft(const mem_plan& P, int64_t count, const float* images, const float2* twid,
-                 float2* spec, cudaStream_t s);
+// shared-memory real 2D FFTs with the layout and scaling of a cuFFT R2C/C2R; masks (or null): the
+// images times the volume mask of their PD (spectrum_masks_supported)
+bool spectrum_masks_supported(const mem_plan& P);
+int spectrum_fft(const mem_plan& P, int64_t count, const float* images, const uint8_t* masks,
+                 const int32_t* img_pd, const float2* twid, float2* spec, cudaStream_t s);
 // signed = the phase-flip inverse: element k of image i multiplied by sign(C_i(k)) / N^2 on load
 int inverse_fft(const mem_plan& P, int64_t count, const float2* spec, const float2* twid,
                 float* images, const uint64_t* qf, bool signed_flip, cudaStream_t s);

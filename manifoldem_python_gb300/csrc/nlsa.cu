@@ -357,7 +357,7 @@ int mem_nlsa_snapshots(int32_t N, int32_t num, int32_t c, int32_t n_modes, const
     if (L.smem_fft) {
         twiddle_kernel<<<1, 256, 0, s>>>(N, twid);
         MEM_LAUNCH_CHECK();
-        int st = kern::spectrum_fft(fp, num, images, twid, spec, s);
+        int st = kern::spectrum_fft(fp, num, images, nullptr, nullptr, twid, spec, s);
         if (st != MEM_OK) return st;
     } else {
         int st = fft_exec(fp.device, N, CUFFT_R2C, num, NN, L.K, const_cast<float*>(images), spec,

@@ -199,3 +199,55 @@ def test_sums_of_many_and_of_few_items(cuda_ready, N, n_pd):
         assert torch.equal(out['D'][d:d + counts[k] ** 2], o1['D'])
         a += counts[k]
         d += counts[k] ** 2
+
+
+@pytest.mark.parametrize('N', [36, 42, 54, 66, 78, 100, 130, 150, 160, 200, 224, 234, 250, 256,
+                               324, 350, 400, 512])
+def test_mixed_radix_transforms_match_cufft(cuda_ready, monkeypatch, N):
+    """The shared-memory transforms of every radix family and both forms (whole image per CTA;
+    rows and columns in tiles) against the cuFFT path of the same plan: SPIDER images with
+    conjugate views, a stack on a 4-byte boundary, and volume masks.  Tolerance: both sides are
+    float transforms within 1e-6 of FP64 (normwise), so 4e-6 of the largest value apart."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    rng = np.random.default_rng(N)
+    counts = [3, 2]
+    n = sum(counts)
+    host = (rng.standard_normal((n, N, N)) + 0.7).astype(np.float32)
+    buf = torch.zeros(n * N * N + 4, dtype=torch.float32, device='cuda')
+    odd = buf[1:1 + n * N * N].view(n, N, N)
+    odd.copy_(torch.from_numpy(host))
+    even = torch.from_numpy(host).cuda()
+    idx = torch.from_numpy(rng.permutation(n)).cuda()
+    flip = torch.from_numpy(rng.integers(0, 2, n).astype(np.uint8)).cuda()
+    psi = torch.from_numpy(rng.uniform(-3, 3, n)).cuda()
+    df = torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda()
+    masks = torch.from_numpy((rng.random((2, N, N)) < 0.6).astype(np.uint8)).cuda()
+    names = ('img_all', 'img_all_flip', 'spectrum', 'img_avg', 'img_avg_flip')
+    for m in (None, masks):
+        got = {}
+        for smem in ('1', '0'):
+            monkeypatch.setenv('MEM_SMEM_FFT', smem)
+            plan = Plan(StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1),
+                        counts, [20.0, 250.0])
+            out = plan.allocate_outputs(names)
+            plan.execute(odd if smem == '1' else even, idx, flip, psi, df, out, pd_mask=m)
+            torch.cuda.synchronize()
+            plan.device_status()
+            got[smem] = out
+        for k in names:
+            a, b = got['1'][k].double(), got['0'][k].double()
+            assert float((a - b).abs().max()) <= 4e-6 * float(b.abs().max()), (k, m is None)
+    # an index outside the stack: flagged, the image NaN, the others untouched
+    monkeypatch.setenv('MEM_SMEM_FFT', '1')
+    plan = Plan(StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1), counts,
+                [20.0, 250.0])
+    out = plan.allocate_outputs(('img_all',))
+    bad = idx.clone()
+    bad[1] = n
+    plan.execute(odd, bad, flip, psi, df, out)
+    torch.cuda.synchronize()
+    with pytest.raises(Exception):
+        plan.device_status()
+    assert bool(torch.isnan(out['img_all'][1]).all())
+    assert bool(torch.isfinite(out['img_all'][[0, 2, 3, 4]]).all())
