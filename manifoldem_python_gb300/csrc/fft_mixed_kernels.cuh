@@ -27,6 +27,7 @@
 
 #include "fft_mixed.cuh"
 #include "mem_internal.cuh"
+#include "rotate_whole.cuh"
 
 namespace mem {
 namespace mixed {
@@ -64,6 +65,10 @@ struct Kernels {
     void (*spectrum)(SpectrumArgs);
     void (*inverse)(InverseArgs);
     void (*inverse_signed)(InverseArgs);
+    // rotation of whole images in shared memory (null where a coefficient image does not fit)
+    void (*rotate)(float*, float*, const rot::RotConst*);
+    int rot_threads;
+    size_t rot_smem;
 };
 
 struct KSumM {                    // Kahan-compensated float accumulator
@@ -659,12 +664,24 @@ constexpr Kernels make_kernels() {
         constexpr int NT = whole_threads<Sh>(), MB = whole_blocks<Sh>();
         return Kernels{N, NT, whole_bytes<Sh>(), whole_lowpass_kernel<Sh, NT, MB>,
                        whole_spectrum_kernel<Sh, NT, MB>, whole_inverse_kernel<Sh, NT, MB, false>,
-                       whole_inverse_kernel<Sh, NT, MB, true>};
+                       whole_inverse_kernel<Sh, NT, MB, true>, nullptr, 0, 0};
     } else {
         return Kernels{N, Tile<Sh>::NT, Tile<Sh>::bytes, tiled_lowpass_kernel<Sh>,
                        tiled_spectrum_kernel<Sh>, tiled_inverse_kernel<Sh, false>,
-                       tiled_inverse_kernel<Sh, true>};
+                       tiled_inverse_kernel<Sh, true>, nullptr, 0, 0};
     }
+}
+
+// with the rotation in segments of SEG samples, LPR lines at a time (rotate_whole.cuh); the pair of
+// each size was picked for 512 to 1024 resident threads of 64 registers and few rounds
+template <int N, int R1, int SEG, int LPR>
+constexpr Kernels make_kernels() {
+    using Sh = rot::WholeShape<N, SEG, LPR>;
+    Kernels k = make_kernels<N, R1>();
+    k.rotate = rot::rotate_whole_kernel<Sh>;
+    k.rot_threads = Sh::NT;
+    k.rot_smem = Sh::SMEM;
+    return k;
 }
 
 }  // namespace mixed

@@ -69,5 +69,22 @@ int inverse(int N, int64_t images, const float2* spec, const float2* twid, float
                   images, s);
 }
 
+bool rotate_supported(int N) {
+    const Kernels* k = find(N);
+    return k && k->rotate;
+}
+
+int rotate(int N, int64_t images, float* xbuf, float* img_out, const void* rotc, cudaStream_t s) {
+    const Kernels* k = find(N);
+    if (!k || !k->rotate) return MEM_ERR_UNSUPPORTED;
+    if (images == 0) return MEM_OK;
+    MEM_CUDA_TRY(cudaFuncSetAttribute(k->rotate, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)k->rot_smem));
+    k->rotate<<<(unsigned)images, k->rot_threads, k->rot_smem, s>>>(
+            xbuf, img_out, static_cast<const rot::RotConst*>(rotc));
+    MEM_LAUNCH_CHECK();
+    return MEM_OK;
+}
+
 }  // namespace mixed
 }  // namespace mem

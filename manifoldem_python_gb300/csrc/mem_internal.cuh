@@ -132,8 +132,11 @@ struct mem_plan {
     // image_stage_kernel)
     bool fused_image = false;
     // boxes rotated by rotate_band: 1 = N > 236 (no whole-image shared-memory kernel), 2 = also
-    // N <= 236 without a compile-time kernel, 0 = never (MEM_ROT_BAND)
+    // N <= 236 other than 64 and 128, 0 = never (MEM_ROT_BAND)
     int rot_band = 1;
+    // compile-time whole-image rotation of the mixed-radix sizes (MEM_ROT_WHOLE=0: the
+    // runtime-size kernel, for comparison)
+    bool rot_whole = true;
     int rot_band_variant = 2;       // rotate_band's sampling / occupancy form (MEM_ROT_BAND_VARIANT)
     // host-to-device image copy of a split execute: the fewer SMs it occupies the less it slows
     // the concurrent computation; 8 x 1024 threads, two images per step, keep ~1 MB of loads in
@@ -171,6 +174,10 @@ int spectrum(int N, int64_t images, const float* src, const uint8_t* masks, cons
              const float2* twid, float2* spec, cudaStream_t s);
 int inverse(int N, int64_t images, const float2* spec, const float2* twid, float* dst,
             const uint64_t* qf, const CtfConst& cc, cudaStream_t s);
+// the two rotations of whole images in shared memory (sizes up to 224 of the table); rotc: the
+// constants that rot_consts writes
+bool rotate_supported(int N);
+int rotate(int N, int64_t images, float* xbuf, float* img_out, const void* rotc, cudaStream_t s);
 }  // namespace mixed
 
 // ---- batched 2D cuFFT transforms of N x N images (abi.cu): R2C image -> half-plane [N][N/2+1]

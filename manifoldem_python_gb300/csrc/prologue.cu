@@ -1247,6 +1247,8 @@ int rotate(const mem_plan& P, const mem_inputs& in, float* xbuf, float* img_out,
     if (kern::rotate_band_supported(N) &&
         ((P.rot_band >= 1 && N > kMaxSmemN) || (P.rot_band >= 2 && !fixed_n)))
         return kern::rotate_band(P, xbuf, spec, img_out, rotc, s);
+    if (P.rot_whole && mixed::rotate_supported(N))
+        return mixed::rotate(N, P.n_images, xbuf, img_out, rotc, s);
     if (N > kMaxSmemN) {
         constexpr int NT = 512;
         const int nseg = std::max(1, std::min(NT / N, N / 16));

@@ -251,3 +251,36 @@ def test_mixed_radix_transforms_match_cufft(cuda_ready, monkeypatch, N):
         plan.device_status()
     assert bool(torch.isnan(out['img_all'][1]).all())
     assert bool(torch.isfinite(out['img_all'][[0, 2, 3, 4]]).all())
+
+
+@pytest.mark.parametrize('N', [36, 42, 50, 54, 70, 88, 96, 100, 144, 150, 162, 182, 192, 200, 220,
+                               224])
+def test_whole_image_rotation_matches_runtime_kernel(cuda_ready, monkeypatch, N):
+    """The compile-time rotation of the mixed-radix sizes (segments of every length, several
+    rounds, odd segments, the odd row stride of 224 px) against the runtime-size kernel, at angles
+    that take both lane orientations, a right angle and zero, with imgAll in its own buffer and in
+    the workspace.  Tolerance: two float evaluations of the same splines, as for the banded
+    kernel: 2e-6 of the largest value."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    rng = np.random.default_rng(N)
+    n = 8
+    stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
+    idx = torch.arange(n, device='cuda')
+    flip = torch.zeros(n, dtype=torch.uint8, device='cuda')
+    psi = torch.tensor([0.0, 0.3, -0.3, 1.5707963267948966, 2.2, -2.2, 3.1, -1.0],
+                       dtype=torch.float64, device='cuda')
+    df = torch.full((n,), 2e4, dtype=torch.float64, device='cuda')
+    got = {}
+    for whole in ('1', '0'):
+        monkeypatch.setenv('MEM_ROT_WHOLE', whole)
+        plan = Plan(StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1),
+                    [3, 1, 4], [0.0, 37.0, 290.0])
+        for names in (('img_all', 'spectrum'), ('spectrum',)):
+            out = plan.allocate_outputs(names)
+            plan.execute(stack, idx, flip, psi, df, out)
+            torch.cuda.synchronize()
+            got[whole, len(names)] = out
+    for m, k in ((2, 'img_all'), (2, 'spectrum'), (1, 'spectrum')):
+        a, b = got['1', m][k].double(), got['0', m][k].double()
+        assert float((a - b).abs().max()) <= 2e-6 * float(b.abs().max()), (m, k)
