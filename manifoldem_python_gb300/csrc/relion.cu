@@ -7,13 +7,22 @@
 //     signal extended symmetrically, period 2N-2) along each axis;
 //   * sample coordinate u = i - s is wrapped with period N-1 into [0, N-1] when it falls outside;
 //   * four taps floor(u)-1 .. floor(u)+2 take mirrored indices (k -> -k, N-1+k -> N-1-k).
-// A shift has one fractional offset per axis, so the 2D interpolation is two separable 4-tap
-// passes.  The mirror prefilter uses the closed-form start values of the causal and anticausal
-// recursions (exact for the symmetric extension).
+// A shift has one fractional offset per axis, so the 2D interpolation is two separable passes,
+// each a prefilter and 4 taps of constant weight.
 //
 // Output: the shifted image transposed (out[a][b] = I[b][a]), i.e. laid out as a SPIDER stack
 // image is, so the rest of the stage (conjugate flip, normalisation, low-pass, ...) reads it
-// unchanged.  One CTA per image, the image in shared memory (row stride N + 1), N <= 236.
+// unchanged.  One CTA per image, the image in shared memory, N <= 236.
+//
+// relion_shift_kernel (N >= 40): a line is split into nseg segments of L <= 32 samples, one thread
+// per segment holding it in registers; the states between segments go through shared memory.
+// Axis 0 comes first, its lines read from global memory (lanes on consecutive columns), and
+// axis 1 last, its results written to global memory (lanes on consecutive rows of the transposed
+// output): an image is read and written once, coalesced.  Bound by latency: 800 images of
+// 100 px take 111 us; with a whole line per thread (serial chains of 3 N) and the taps of every
+// output in FP64 it was 209 us.  Smaller boxes keep that form, whose start values are exact for
+// any length (relion_small_kernel).
+#include <algorithm>
 #include <cmath>
 
 #include "mem_internal.cuh"
@@ -75,13 +84,17 @@ __device__ __forceinline__ void bspline4(float t, float w[4]) {
 __device__ __forceinline__ void wrap_coord(int i, double s, int N, int* f, float* t) {
     double u = (double)i - s;
     const double per = (double)(N - 1);
-    if (per > 0.0 && (u < 0.0 || u > per)) u -= per * floor(u / per);
+    if (per > 0.0 && (u < 0.0 || u > per)) {
+        const bool below = u < 0.0;
+        u -= per * floor(u / per);
+        if (below && u == 0.0) u = per;            // a negative whole period lands on the far end
+    }
     const double fu = floor(u);
     *f = (int)fu;
     *t = (float)(u - fu);
 }
 
-constexpr int kMaxPer = 8;                         // N <= 256: outputs per lane and line
+constexpr int kMaxPer = 2;                         // N < 40: outputs per lane and line
 
 // Interpolation along one axis, one warp per line, in place: lane l computes the outputs
 // j = l + 32 q of its line into registers, then writes them (taps and weights per j are the
@@ -123,7 +136,7 @@ __device__ __forceinline__ void shift_lines(float* A, int N, int P, double sh, i
 }
 
 template <int NT>
-__global__ void __launch_bounds__(NT) relion_shift_kernel(
+__global__ void __launch_bounds__(NT) relion_small_kernel(
         const float* __restrict__ stack, int64_t num_stack, const int64_t* __restrict__ sidx,
         const double* __restrict__ shift_yx, int N, float* __restrict__ out,
         uint32_t* __restrict__ status) {
@@ -160,6 +173,180 @@ __global__ void __launch_bounds__(NT) relion_shift_kernel(
     }
 }
 
+// Segments of one axis of one image (see above): line l, segment g of L samples (the last one
+// shorter).
+constexpr int kSeg = 32;
+struct ShiftAxis {
+    int N, L, nseg, lpr;
+    float zL;                              // kPole^L
+};
+
+// prefilter and shift along one axis.  GLOBAL_IN: sample k of line l is src[k N + l], else
+// s[l SL + k SK]; the coefficients go to s; the result to s, or (GLOBAL_OUT) to dst[k N + l].
+template <int NT, bool GLOBAL_IN, bool GLOBAL_OUT>
+__device__ __forceinline__ void shift_axis(float* s, float* carry, const float* __restrict__ src,
+                                           float* __restrict__ dst, double shift, int SL, int SK,
+                                           const ShiftAxis& ax) {
+    const float z = kPole;
+    const int N = ax.N, L = ax.L;
+    const int lw = threadIdx.x % ax.lpr, g = threadIdx.x / ax.lpr;
+    const int k0 = g * L, len = min(L, N - k0);
+    // output k samples at k - shift = k + i0 + t
+    const double fl = floor(-shift);
+    // far outside, where every sample wraps, the whole part is first reduced by whole periods
+    const double per = (double)(N - 1);
+    const double fr = fabs(fl) > 1.0e6 ? fl - per * floor(fl / per) - 16.0 * per : fl;
+    const int i0 = (int)fmin(fmax(fr, -1.0e9), 1.0e9);       // in range for a NaN or inf shift too
+    const float t = (float)(-shift - fl);
+    float w[4];
+    bspline4(t, w);
+    float* carry_c = carry;                // [nseg][lpr] causal, then anticausal end states
+    float* carry_a = carry + NT;
+    for (int l0 = 0; l0 < N; l0 += ax.lpr) {
+        const int line = l0 + lw;
+        const bool on = g < ax.nseg && line < N;
+        float* x = s + line * SL;
+        float v[kSeg];
+        if (on) {
+            float e = 0.f;
+#pragma unroll
+            for (int k = 0; k < kSeg; ++k)
+                if (k < len) {
+                    v[k] = GLOBAL_IN ? __ldg(src + (int64_t)(k0 + k) * N + line)
+                                     : x[(k0 + k) * SK];
+                    e = fmaf(z, e, v[k]);
+                }
+            carry_c[g * ax.lpr + lw] = e;
+        }
+        __syncthreads();
+        if (on) {
+            // the state before the segment: the two previous end states, or for the first
+            // segment the mirrored samples themselves, sum_{j >= 1} z^(j-1) x[j]
+            float c;
+            if (g == 0) {
+                c = 0.f;
+#pragma unroll
+                for (int k = kSeg - 1; k >= 1; --k)
+                    if (k < len) c = fmaf(z, c, v[k]);
+            } else {
+                c = carry_c[(g - 1) * ax.lpr + lw];
+                if (g > 1) c = fmaf(ax.zL, carry_c[(g - 2) * ax.lpr + lw], c);
+            }
+            float last = 0.f, before = 0.f;            // c+ of the line's last two samples
+#pragma unroll
+            for (int k = 0; k < kSeg; ++k)
+                if (k < len) {
+                    c = fmaf(z, c, v[k]);
+                    v[k] = c;
+                    before = last;
+                    last = c;
+                }
+            float e = 0.f;
+            if (g == ax.nseg - 1) {                    // the mirror's closed form at the end
+                e = (z / (z * z - 1.f)) * (last + z * before);
+#pragma unroll
+                for (int k = kSeg - 1; k >= 0; --k)
+                    if (k < len - 1) e = z * (e - v[k]);
+            } else {
+#pragma unroll
+                for (int k = kSeg - 1; k >= 0; --k)
+                    if (k < len) e = z * (e - v[k]);
+            }
+            carry_a[g * ax.lpr + lw] = e;
+        }
+        __syncthreads();
+        if (on) {
+            if (g == ax.nseg - 1) {
+                float last = 0.f, before = 0.f;
+#pragma unroll
+                for (int k = 0; k < kSeg; ++k)
+                    if (k < len) {
+                        before = last;
+                        last = v[k];
+                    }
+                float c = (z / (z * z - 1.f)) * (last + z * before);
+#pragma unroll
+                for (int k = kSeg - 1; k >= 0; --k)
+                    if (k < len) {
+                        if (k < len - 1) c = z * (c - v[k]);
+                        x[(k0 + k) * SK] = 6.f * c;
+                    }
+            } else {
+                float c = carry_a[(g + 1) * ax.lpr + lw];
+                if (g + 2 < ax.nseg) {
+                    // the end state of a segment of L, carried over the one between
+                    c = fmaf(ax.zL, carry_a[(g + 2) * ax.lpr + lw], c);
+                }
+#pragma unroll
+                for (int k = kSeg - 1; k >= 0; --k)
+                    if (k < len) {
+                        c = z * (c - v[k]);
+                        x[(k0 + k) * SK] = 6.f * c;
+                    }
+            }
+        }
+        __syncthreads();
+        if (on) {
+#pragma unroll
+            for (int k = 0; k < kSeg; ++k)
+                if (k < len) {
+                    // wrapped with period N - 1 where the sample point lies outside [0, N - 1]
+                    int f = k0 + k + i0;
+                    if (f < 0 || f > N - 1 || (f == N - 1 && t > 0.f)) {
+                        const bool below = f < 0;
+                        f %= N - 1;
+                        f += f < 0 ? N - 1 : 0;
+                        f = below && f == 0 && t == 0.f ? N - 1 : f;     // as scipy wraps
+                    }
+                    float acc = 0.f;
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        int q = f - 1 + b;             // -1 .. N + 1, mirrored
+                        q = q < 0 ? -q : q;
+                        q = q > N - 1 ? 2 * (N - 1) - q : q;
+                        acc = fmaf(w[b], x[q * SK], acc);
+                    }
+                    v[k] = acc;
+                }
+        }
+        if (!GLOBAL_OUT) __syncthreads();              // every tap of the lines is read
+        if (on) {
+#pragma unroll
+            for (int k = 0; k < kSeg; ++k)
+                if (k < len) {
+                    if (GLOBAL_OUT)
+                        dst[(int64_t)(k0 + k) * N + line] = v[k];
+                    else
+                        x[(k0 + k) * SK] = v[k];
+                }
+        }
+    }
+    __syncthreads();
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT, 3) relion_shift_kernel(
+        const float* __restrict__ stack, int64_t num_stack, const int64_t* __restrict__ sidx,
+        const double* __restrict__ shift_yx, ShiftAxis ax, float* __restrict__ out,
+        uint32_t* __restrict__ status) {
+    extern __shared__ float smem[];        // carries [2 NT], the image [N][N | 1]
+    const int N = ax.N, P = N | 1, NN = N * N;
+    const int64_t img = blockIdx.x;
+    const int64_t s = sidx[img];
+    float* dst = out + img * (int64_t)NN;
+    if (s < 0 || s >= num_stack) {
+        if (threadIdx.x == 0) atomicOr(status, 2u);
+        for (int p = threadIdx.x; p < NN; p += NT) dst[p] = __int_as_float(0x7fc00000);
+        return;
+    }
+    float* A = smem + 2 * NT;
+    // axis 0 (rows r of column l): shift sh_y - 0.5; axis 1 (columns c of row l): sh_x - 0.5,
+    // written to out[c][r]
+    shift_axis<NT, true, false>(A, smem, stack + s * (int64_t)NN, nullptr, shift_yx[2 * img], 1, P,
+                                ax);
+    shift_axis<NT, false, true>(A, smem, nullptr, dst, shift_yx[2 * img + 1], P, 1, ax);
+}
+
 }  // namespace
 
 namespace kern {
@@ -168,12 +355,26 @@ int relion_shift(const mem_plan& P, const mem_inputs& in, float* out, uint32_t* 
     if (P.n_images == 0) return MEM_OK;
     const int N = P.N;
     if (N > kMaxSmemN) return MEM_ERR_UNSUPPORTED;         // one image in shared memory
-    const size_t smem = (size_t)N * (N + 1) * sizeof(float);
-    constexpr int NT = 256;
-    MEM_CUDA_TRY(cudaFuncSetAttribute(relion_shift_kernel<NT>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    relion_shift_kernel<NT><<<(unsigned)P.n_images, NT, smem, s>>>(
-            in.stack, in.num_stack, in.stack_index, in.shift_yx, N, out, status);
+    if (N >= 40) {
+        constexpr int NT = 256;
+        ShiftAxis ax;
+        ax.N = N;
+        ax.nseg = (N + kSeg - 1) / kSeg;
+        ax.L = (N + ax.nseg - 1) / ax.nseg;            // >= 20: the last segment has >= 13 samples
+        ax.lpr = std::min(N, NT / ax.nseg);
+        ax.zL = (float)std::pow((double)kPole, (double)ax.L);
+        const size_t smem = (2 * NT + (size_t)N * (N | 1)) * sizeof(float);
+        MEM_CUDA_TRY(cudaFuncSetAttribute(relion_shift_kernel<NT>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem));
+        relion_shift_kernel<NT><<<(unsigned)P.n_images, NT, smem, s>>>(
+                in.stack, in.num_stack, in.stack_index, in.shift_yx, ax, out, status);
+    } else {
+        const size_t smem = (size_t)N * (N + 1) * sizeof(float);
+        constexpr int NT = 256;
+        relion_small_kernel<NT><<<(unsigned)P.n_images, NT, smem, s>>>(
+                in.stack, in.num_stack, in.stack_index, in.shift_yx, N, out, status);
+    }
     MEM_LAUNCH_CHECK();
     return MEM_OK;
 }

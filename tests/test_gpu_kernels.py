@@ -284,3 +284,35 @@ def test_whole_image_rotation_matches_runtime_kernel(cuda_ready, monkeypatch, N)
     for m, k in ((2, 'img_all'), (2, 'spectrum'), (1, 'spectrum')):
         a, b = got['1', m][k].double(), got['0', m][k].double()
         assert float((a - b).abs().max()) <= 2e-6 * float(b.abs().max()), (m, k)
+
+
+@pytest.mark.parametrize('N', [8, 39, 40, 63, 64, 65, 97, 100, 128, 200, 235, 236])
+def test_relion_shift(cuda_ready, N):
+    """The RELION read against scipy's shift (order 3, 'wrap') at fractional, whole, zero and large
+    shifts of both signs, through the normalised images of an avg_only plan with an all-pass
+    filter.  Tolerance: float prefilter and taps, 1e-5 of the largest value as for every image
+    output."""
+    torch = cuda_ready
+    from scipy.ndimage import shift
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    rng = np.random.default_rng(N)
+    sh = np.array([[0.0, 0.0], [2.0, -3.0], [0.25, 0.75], [-1.6, 3.4], [N - 1.0, -(N - 1.0)],
+                   [N + 7.3, -2.0 * N - 0.4], [-0.5, -0.5], [1.5e6 + 0.25, -1.5e6 - 0.75]])
+    n = len(sh)
+    stack = rng.standard_normal((n, N, N)).astype(np.float32)
+    psi = torch.zeros(n, dtype=torch.float64, device='cuda')
+    plan = Plan(StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1,
+                            filter_Qc=1e9, avg_only=True), [n], [0.0])
+    out = plan.allocate_outputs(('img_all',))
+    plan.execute(torch.from_numpy(stack).cuda(), torch.arange(n, device='cuda'),
+                 torch.zeros(n, dtype=torch.uint8, device='cuda'), psi,
+                 torch.full((n,), 2e4, dtype=torch.float64, device='cuda'), out,
+                 shift_yx=torch.from_numpy(sh).cuda())
+    got = out['img_all'].cpu().numpy()
+    r, c = np.mgrid[0:N, 0:N]
+    msk = ((r - N / 2 + 1) ** 2 + (c - N / 2) ** 2 < (N / 2) ** 2)
+    for i in range(n):
+        x = shift(stack[i].astype(np.float64), sh[i], order=3, mode='wrap')
+        b = x * (1 - msk)
+        ref = (x - b.mean()) / b.std() * msk
+        assert np.abs(got[i] - ref).max() <= 1e-5 * np.abs(ref).max(), (i, sh[i])
