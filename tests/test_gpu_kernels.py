@@ -316,3 +316,38 @@ def test_relion_shift(cuda_ready, N):
         b = x * (1 - msk)
         ref = (x - b.mean()) / b.std() * msk
         assert np.abs(got[i] - ref).max() <= 1e-5 * np.abs(ref).max(), (i, sh[i])
+
+
+@pytest.mark.parametrize('counts', [[1], [31], [33, 2], [128, 129], [600], [700], [1900]])
+def test_fp32_contraction_tiles(cuda_ready, counts):
+    """The FP32 contraction in every tile size (32, 64 and 128, by the number of tiles): exactly
+    symmetric, zero on the diagonal, and the same bits as the PD has in a plan of many PDs (each
+    element is one sum over k in order in all of them)."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    N = 32
+    rng = np.random.default_rng(len(counts) + counts[0])
+    extra = [300] * 34                                     # 34 x 6 tiles: the 128-wide form
+    n = sum(counts) + sum(extra)
+    stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
+    idx = torch.arange(n, device='cuda')
+    flip = torch.zeros(n, dtype=torch.uint8, device='cuda')
+    psi = torch.from_numpy(rng.uniform(-3, 3, n)).cuda()
+    df = torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda()
+    params = StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1)
+    got = []
+    for cs in (counts, counts + extra):
+        m = sum(cs)
+        plan = Plan(params, cs, [30.0 * (i % 12) for i in range(len(cs))])
+        out = plan.allocate_outputs(('D',))
+        out['D'].fill_(float('nan'))
+        plan.execute(stack, idx[:m], flip[:m], psi[:m], df[:m], out)
+        torch.cuda.synchronize()
+        got.append(out['D'])
+    off = 0
+    for c in counts:
+        d = got[0][off:off + c * c].view(c, c)
+        assert bool(torch.isfinite(d).all())
+        assert torch.equal(d, d.t()) and float(d.diagonal().abs().max()) == 0.0
+        off += c * c
+    assert torch.equal(got[0], got[1][:off])
