@@ -519,6 +519,13 @@ int mem_plan_create(const mem_params* params, int32_t n_pd, const int32_t* pd_co
     L.avg_spec = take(sizeof(float) * 2 * 2 * P->Kc * n_pd);
     L.avg_real = take(sizeof(float) * 2 * NN * n_pd);
     L.cufft_work = take(P->cufft_work_bytes);
+    // up to 64 MB for the contraction of few tiles
+    P->tc_part_units = (p.precision == MEM_PREC_FP32 || p.avg_only)
+                           ? 0
+                           : tc_split_units((int64_t)P->tiles.size(), P->n_chunks, 1024);
+    L.tc_part = take(P->tc_part_units
+                         ? (size_t)(P->tc_part_units + (int64_t)P->tiles.size()) * kTcUnitBytes
+                         : 0);
     L.total = off;
     *out_plan = P;
     return MEM_OK;
@@ -855,7 +862,7 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
         else
             MEM_STEP(kern::gemm_split_bf16(P, feat_a, feat_b, pair_norm, scale_bits,
                                            at<Tile>(ws, L.tc_tiles), pds, ft.chunks, out->D,
-                                           status, s));
+                                           status, at<float>(ws, L.tc_part), P.tc_part_units, s));
     }
     MEM_STEP(mark(9));
 #undef MEM_STEP

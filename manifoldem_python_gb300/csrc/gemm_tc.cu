@@ -605,13 +605,184 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TC_THREADS, 1) gemm_
     }
 }
 
+// ---- few tiles: every K chunk its own CTA ---------------------------------------------------
+// One CTA walks a tile's chunks in about 1 us each (the MMA and its shared-memory traffic), so a
+// plan of few tiles leaves most SMs idle: 102 us for the 6 tiles of 300 images of 70 px.  Here unit
+// (tile, chunk) is a CTA of its own, which stores the chunk's accumulator -- the very value that the
+// epilogue of gemm_tc_kernel adds for the chunk -- and gemm_tc_join_kernel adds a tile's chunks in
+// their order: D is bit-identical.  Units go in rounds of what the scratch holds, the running sums
+// between rounds in the scratch too.  Bound by writing and reading the 64 KB of a unit in L2.
+// 300 images of 70 px: 28 us; 100 of 128 px: 17 us, was 268; see tc_split_units for the line between the two.
+constexpr int TS_THREADS = 128;
+constexpr int TS_ELEMS = TC_M * 128;
+constexpr size_t TS_SMEM = (size_t)4 * TC_OPB + 1024;
+
+template <bool LOLO>
+__global__ void __launch_bounds__(TS_THREADS) gemm_tc_chunk_kernel(
+        const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
+        const Tile* __restrict__ tiles, const PdDev* __restrict__ pds, float* __restrict__ part,
+        uint32_t* __restrict__ status, const int4* __restrict__ chunks, int c_begin, int c_count,
+        long long wait_limit, int withhold) {
+    constexpr uint32_t IDESC = idesc_f16<128>(), IDESC_NEG = IDESC | (1u << 14);
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* sb = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t full, done;
+    __shared__ uint32_t tmem_base;
+    __shared__ int abort_word;
+    volatile int* abort_flag = &abort_word;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const Tile t = tiles[blockIdx.x / c_count];
+    const int c = c_begin + (int)(blockIdx.x % c_count);
+    if (threadIdx.x == 0) {
+        mbar_init(&full, 1);
+        mbar_init(&done, 1);
+        abort_word = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(&tmem_base)),
+                     "r"(128u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+    if (threadIdx.x == 0) {
+        const int4 ch = chunks[c];
+        const bool load = c != withhold;           // a withheld chunk: test of the timeout path
+        if (load) {
+            const PdDev pd = pds[t.pd];
+            const int rowA = (int)(pd.row_off + (int64_t)t.I * TC_M);
+            const int rowB = (int)(pd.row_off + (int64_t)t.J * 128);
+            mbar_expect_tx(&full, 4 * TC_OPB);
+            tma_load_2d(sb + 0 * TC_OPB, &map_hi, &full, ch.x, rowA);
+            tma_load_2d(sb + 1 * TC_OPB, &map_lo, &full, ch.x, rowA);
+            tma_load_2d(sb + 2 * TC_OPB, &map_hi, &full, ch.y, rowB);
+            tma_load_2d(sb + 3 * TC_OPB, &map_lo, &full, ch.y, rowB);
+        }
+        if (mbar_wait(&full, 0, abort_flag, status, wait_limit)) {
+            tc_fence_after();
+            const uint32_t idesc = ch.z != 0 ? IDESC_NEG : IDESC;
+            const uint32_t sa = smem_u32(sb);
+            const bool four = LOLO || ch.w != 0;
+#pragma unroll
+            for (int k = 0; k < TC_BK / 16; ++k) {
+                const uint64_t ahi = sdesc_sw128(sa + 0 * TC_OPB + k * 32);
+                const uint64_t alo = sdesc_sw128(sa + 1 * TC_OPB + k * 32);
+                const uint64_t bhi = sdesc_sw128(sa + 2 * TC_OPB + k * 32);
+                const uint64_t blo = sdesc_sw128(sa + 3 * TC_OPB + k * 32);
+                umma_bf16(tmem, ahi, bhi, idesc, k == 0 ? 0u : 1u);
+                umma_bf16(tmem, ahi, blo, idesc, 1u);
+                umma_bf16(tmem, alo, bhi, idesc, 1u);
+                if (four) umma_bf16(tmem, alo, blo, idesc, 1u);
+            }
+            umma_commit(&done);
+            // an expired wait below does not end before the MMAs have
+            if (!mbar_wait(&done, 0, abort_flag, status, wait_limit))
+                mbar_drain(&done, 0, wait_limit);
+        } else if (load) {
+            mbar_drain(&full, 0, wait_limit);      // the copies land before the CTA exits
+        }
+    }
+    __syncwarp();
+    const bool ok = __all_sync(0xffffffffu,
+                               mbar_wait(&done, 0, abort_flag, status, wait_limit));
+    if (ok) {
+        tc_fence_after();
+        // [column][row]: a column's 32 lanes store 128 consecutive bytes
+        float* out = part + (int64_t)blockIdx.x * TS_ELEMS + warp * 32 + lane;
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+            uint32_t r[32];
+            tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(q * 32), r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) out[(q * 32 + j) * TC_M] = __uint_as_float(r[j]);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                     "r"(128u)
+                     : "memory");
+    }
+}
+
+// adds the round's chunks to the tiles' running sums; the last round stores D
+__global__ void __launch_bounds__(TS_THREADS) gemm_tc_join_kernel(
+        const float* __restrict__ part, float* __restrict__ run, int c_count, int first, int last,
+        const double* __restrict__ pair_norm, const uint32_t* __restrict__ scale_bits,
+        const Tile* __restrict__ tiles, const PdDev* __restrict__ pds, double* __restrict__ D) {
+    constexpr int kPerTile = TS_ELEMS / TS_THREADS;
+    const int tile = blockIdx.x / kPerTile;
+    const int e = (int)(blockIdx.x % kPerTile) * TS_THREADS + (int)threadIdx.x;
+    const Tile t = tiles[tile];
+    const PdDev pd = pds[t.pd];
+    const int gi = t.I * TC_M + e % TC_M, gj = t.J * 128 + e / TC_M, n = pd.n;
+    if (gi >= n || gj >= n || gj < gi) return;
+    float* r = run + (int64_t)tile * TS_ELEMS + e;
+    float acc = first ? 0.f : *r;
+    const float* p = part + (int64_t)tile * c_count * TS_ELEMS + e;
+    constexpr int B = 16;                          // loads in flight per element
+    float v[B];
+    auto load = [&](int c0) {
+#pragma unroll
+        for (int u = 0; u < B; ++u) v[u] = p[(int64_t)min(c0 + u, c_count - 1) * TS_ELEMS];
+    };
+    load(0);
+    int c = 0;
+    for (; c + B <= c_count; c += B) {
+        float w[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) w[u] = v[u];
+        load(c + B);
+#pragma unroll
+        for (int u = 0; u < B; ++u) acc += w[u];
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+        if (c + u < c_count) acc += v[u];
+    if (!last) {
+        *r = acc;
+        return;
+    }
+    double* Dp = D + pd.d_off;
+    if (gj == gi) {
+        Dp[(int64_t)gi * n + gi] = 0.0;
+        return;
+    }
+    const double sc = (double)feature_scale_from_bits(scale_bits[t.pd]);
+    const double inv_sc2 = 1.0 / (sc * sc);
+    const double* an = pair_norm + pd.img_off;
+    const double d = an[gi] + an[gj] + (double)acc * inv_sc2;
+    Dp[(int64_t)gi * n + gj] = d;
+    Dp[(int64_t)gj * n + gi] = d;
+}
+
 }  // namespace
+
+// Scratch units (64 KB each) with which the contraction of `tiles` tiles is split by chunks, at most
+// `most`; 0: one CTA per tile is the faster.  Measured: about 1 us per chunk for a tile of its own
+// CTA whatever the number of tiles up to one per SM, against 20 to 27 ns per unit and 8 us per round.
+int64_t tc_split_units(int64_t tiles, int64_t chunks, int64_t most) {
+    if (tiles < 1 || tiles > 64) return 0;
+    const int64_t per_round = std::min(chunks, most / tiles);    // chunks
+    if (per_round < 1) return 0;
+    const int64_t rounds = (chunks + per_round - 1) / per_round;
+    if (8.0 * rounds + 0.02 * (double)(tiles * chunks) > 0.7 * (double)chunks) return 0;
+    return per_round * tiles;
+}
 
 namespace kern {
 int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
                     const double* pair_norm, const uint32_t* scale_bits, const Tile* tiles,
                     const PdDev* pds, const int4* chunks, double* D, uint32_t* status,
-                    cudaStream_t s) {
+                    float* part, int64_t part_units, cudaStream_t s) {
     if (P.tiles.empty() || !D) return MEM_OK;
     // every chunk starts on a 64-column boundary: TMA x offsets are multiples of 8 bf16
     if (P.Kf % TC_BK != 0 || P.n_rows % TC_M != 0 || (int64_t)P.n_chunks * TC_BK != P.Kf)
@@ -621,6 +792,29 @@ int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
     if (st != MEM_OK) return st;
     st = tc::make_map(&mlo, feat_lo, P.Kf, P.n_rows);
     if (st != MEM_OK) return st;
+    // the default schedule of a plan of few tiles: chunks spread over the SMs
+    const mem_contraction_config& c0 = P.tc_classes[0];
+    const int T = (int)P.tc_tiles.size();
+    if (part_units >= T && P.tc_ranges.size() == 1 && !c0.persistent && c0.accumulators == 2 &&
+        c0.tile_n == 128 && c0.tile_m == 128 && P.tc_group_chunks == 1 && !P.tc_kahan) {
+        float* run = part + part_units * TS_ELEMS;
+        const int per_round = (int)std::min<int64_t>(P.n_chunks, part_units / T);
+        auto kfn = P.tc_lolo ? gemm_tc_chunk_kernel<true> : gemm_tc_chunk_kernel<false>;
+        MEM_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)TS_SMEM));
+        for (int c = 0; c < P.n_chunks; c += per_round) {
+            const int count = std::min(per_round, P.n_chunks - c);
+            kfn<<<(unsigned)(T * count), TS_THREADS, TS_SMEM, s>>>(
+                    mhi, mlo, tiles, pds, part, status, chunks, c, count, P.wait_cycles,
+                    P.test_withhold_chunk);
+            MEM_LAUNCH_CHECK();
+            gemm_tc_join_kernel<<<(unsigned)(T * (TS_ELEMS / TS_THREADS)), TS_THREADS, 0, s>>>(
+                    part, run, count, c == 0 ? 1 : 0, c + count == P.n_chunks ? 1 : 0, pair_norm,
+                    scale_bits, tiles, pds, D);
+            MEM_LAUNCH_CHECK();
+        }
+        return MEM_OK;
+    }
     const int sms = P.num_sms > 0 ? P.num_sms : 1;
     CUtensorMap bhi, blo;                // 64-row boxes: the CTA pairs' halves of B
     bool have_b64 = false;

@@ -86,7 +86,7 @@ struct Layout {
     size_t status, pd_table, sum_items, img_pd, img_row, tiles, tc_tiles;
     size_t item_off, qfix, rotc, gtab, pd_max, colmap, twid, ident;
     size_t xbuf, spec, feat_a, feat_b, pair_norm, partial, means, avg_spec, avg_real, cufft_work;
-    size_t total;
+    size_t tc_part, total;
 };
 
 }  // namespace mem
@@ -123,6 +123,7 @@ struct mem_plan {
     std::vector<std::pair<int, int>> tc_ranges;
     std::vector<mem::Tile> tc_tiles;   // the split-BF16 contraction's tiles (J in tile_n units)
     bool uploaded = false;
+    int64_t tc_part_units = 0;      // scratch of the chunk-split contraction
     int tc_group_chunks = 1;        // 64-wide K chunks per TMEM accumulation group (0 = all)
     bool tc_kahan = false;          // compensated register sums across groups
     bool tc_lolo = false;           // add the lo.lo product (4-term split)
@@ -262,8 +263,13 @@ int gemm_fp32(const mem_plan& P, const float* feat, const double* pair_norm,
 int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
                     const double* pair_norm, const uint32_t* scale_bits, const Tile* tiles,
                     const PdDev* pds, const int4* chunks, double* D, uint32_t* status,
-                    cudaStream_t s);
+                    float* part, int64_t part_units, cudaStream_t s);
 }  // namespace kern
+
+// scratch of the split-BF16 contraction of few tiles (gemm_tc.cu): units of 64 KB to use, of at most
+// `most`, 0 for none; the buffer holds the units and one more per tile
+constexpr size_t kTcUnitBytes = 128 * 128 * sizeof(float);
+int64_t tc_split_units(int64_t tiles, int64_t chunks, int64_t most);
 
 std::vector<int32_t> radius_descending_columns(int N, int64_t Kc, int64_t Kc_pad);
 

@@ -61,7 +61,7 @@ size_t a256(size_t x) { return (x + 255) / 256 * 256; }
 // then the per-call tables and buffers.
 struct NoallocLayout {
     size_t status, colmap, pd_table, items, item_off, img_pd, img_row, tiles, qfix, partial, means,
-        avg_spec, pd_max, spec, feat_a, feat_b, pair_norm, total;
+        avg_spec, pd_max, spec, feat_a, feat_b, pair_norm, total;   // the rest: scratch units
 };
 
 NoallocLayout layout_for(const mem_plan& P) {
@@ -274,10 +274,17 @@ extern "C" int mem_pd_distances_noalloc(const mem_params* params, int32_t n, con
     if (P.params.precision == MEM_PREC_FP32)
         NA_STEP(kern::gemm_fp32(P, at<float>(ws, L.feat_a), pair_norm, scale_bits,
                                 at<Tile>(ws, L.tiles), pds, ft.chunks, D, s));
-    else
+    else {
+        // what the layout leaves of the array is scratch for the contraction of few tiles
+        const int64_t T = (int64_t)P.tiles.size();
+        const int64_t room =
+            (int64_t)(((size_t)MEM_NOALLOC_SCRATCH_BYTES - L.total) / kTcUnitBytes) - T;
+        const int64_t units = room > 0 ? tc_split_units(T, P.n_chunks, room) : 0;
         NA_STEP(kern::gemm_split_bf16(P, at<char>(ws, L.feat_a), at<char>(ws, L.feat_b),
                                       pair_norm, scale_bits, at<Tile>(ws, L.tiles), pds,
-                                      ft.chunks, D, at<uint32_t>(ws, L.status), s));
+                                      ft.chunks, D, at<uint32_t>(ws, L.status),
+                                      at<float>(ws, L.total), units, s));
+    }
 #undef NA_STEP
     return MEM_OK;
 }

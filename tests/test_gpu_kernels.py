@@ -351,3 +351,35 @@ def test_fp32_contraction_tiles(cuda_ready, counts):
         assert torch.equal(d, d.t()) and float(d.diagonal().abs().max()) == 0.0
         off += c * c
     assert torch.equal(got[0], got[1][:off])
+
+
+@pytest.mark.parametrize('N,counts', [(32, [1]), (32, [24, 3]), (64, [128]), (64, [129, 300]),
+                                      (70, [300]), (128, [60]), (128, [400])])
+def test_contraction_split_by_chunks(cuda_ready, N, counts):
+    """The split-BF16 contraction of few tiles, every K chunk a CTA of its own and the chunks added
+    in order (one round or several), gives the same bits as a persistent CTA per tile."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    rng = np.random.default_rng(N + counts[0])
+    n = sum(counts)
+    stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
+    idx = torch.arange(n, device='cuda')
+    flip = torch.zeros(n, dtype=torch.uint8, device='cuda')
+    psi = torch.from_numpy(rng.uniform(-3, 3, n)).cuda()
+    df = torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda()
+    params = StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1,
+                         precision='bf16x3')
+    got = []
+    for contraction in ([dict(max_n=2 ** 31 - 1, persistent=0, accumulators=2)],
+                        [dict(max_n=2 ** 31 - 1, persistent=1, accumulators=2)]):
+        plan = Plan(params, counts, [40.0 * i for i in range(len(counts))],
+                    contraction=contraction)
+        out = plan.allocate_outputs(('D',))
+        out['D'].fill_(float('nan'))
+        for _ in range(2):
+            plan.execute(stack, idx, flip, psi, df, out)
+        torch.cuda.synchronize()
+        plan.device_status()
+        got.append(out['D'])
+    assert bool(torch.isfinite(got[0]).all())
+    assert torch.equal(got[0], got[1])
