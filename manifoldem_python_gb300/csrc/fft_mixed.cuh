@@ -104,7 +104,7 @@ MEM_HD void dft_odd_prime(float2* v) {
     v[0] = t;
 }
 
-constexpr int first_factor(int R) {                // the pass-1 length of a composite R
+MEM_HD constexpr int first_factor(int R) {                // the pass-1 length of a composite R
     return R % 8 == 0 && R > 8 && R != 16 ? 8
            : R % 4 == 0 && R > 4 ? 4
            : R % 2 == 0 && R > 2 ? 2

@@ -7,22 +7,19 @@
 //
 // Whole (N <= 224): one image per CTA, the N x N / 2 complex buffer in shared memory; an image is
 // read and written once.  Bound by the latency of its 8 (low-pass 12) shared-memory passes at the
-// 16 to 20 warps that the buffer and 102 to 128 registers per thread leave on an SM: 512 threads
-// where the buffer lets only one or two CTAs on an SM, 128 where it is small.
+// 12 to 20 warps that the buffer and about 100 registers per thread leave on an SM.
 //
 // Tiled (larger N): one image per CTA too, rows in chunks of PC pair-rows and columns in tiles of
-// CT columns through a buffer of about 50 KB, four CTAs per SM.  Between rows and columns the
-// spectra go through the image's own output slot (in L2: the slots of all resident CTAs are 152
-// x 4 x 250 KB at most, and a slot is read back right after it is written).  Keeping the rows
-// of an image in the shared memories of a cluster of two CTAs instead measured 1758 us for the
-// low-pass of 1160 images of 250 px, against 706 us for this form: the column passes' 8-byte
-// accesses are slow over distributed shared memory.
+// CT columns through a buffer of up to 108 KB, two CTAs per SM.  Between rows and columns the
+// spectra go through the image's own output slot (in L2: 304 slots of 250 KB at 250 px, read back
+// right after they are written).  Keeping the rows of an image in the shared memories of a
+// cluster of two CTAs instead measured 1758 us for the low-pass of 1160 images of 250 px, against
+// 583 us for this form: the column passes' 8-byte accesses are slow over distributed shared memory.
 //
 // Against cuFFT (a row pass and a column pass over HBM for every transform, the gather and the
 // filter in passes of their own):
-//   1000 images of 192 px:  low-pass 234 us, was 465; spectrum 104, was 150; flip 102, was 153
-//   1160 images of 250 px:  low-pass 706 us, was 1240; spectrum 282, was 434; flip 354, was
-//   451
+//   1000 images of 192 px:  low-pass 217 us, was 465; spectrum 108, was 150; flip 103, was 153
+//   1160 images of 250 px:  low-pass 583 us, was 1240; spectrum 252, was 434; flip 289, was 451
 #pragma once
 
 #include "fft_mixed.cuh"
@@ -140,13 +137,17 @@ template <class Sh>
 constexpr size_t whole_bytes() {
     return (size_t)Sh::H * Sh::S * sizeof(float2);
 }
+// Threads and CTAs per SM: 128 x 5 while five buffers fit, 320 x 2 while two do (the load of one
+// image then overlaps the passes of another), else 384 threads alone; measured against 256 x 2,
+// 256 x 3, 512 x 1, 768 x 1 (low-pass of 1000 images: 120 px 97 us, 256 x 2 the same; 150 px 137,
+// 512 x 1 190; 192 px 217, 512 x 1 235; 800 of 100 px 53, 256 x 2 60)
 template <class Sh>
-constexpr int whole_threads() {
-    return whole_bytes<Sh>() > 75 * 1024 ? 512 : whole_bytes<Sh>() > 30 * 1024 ? 256 : 128;
+constexpr int whole_blocks() {
+    return whole_bytes<Sh>() <= 44 * 1024 ? 5 : whole_bytes<Sh>() <= 108 * 1024 ? 2 : 1;
 }
 template <class Sh>
-constexpr int whole_blocks() {                    // at least 102 registers per thread
-    return whole_threads<Sh>() == 512 ? 1 : whole_threads<Sh>() == 256 ? 2 : 5;
+constexpr int whole_threads() {
+    return whole_blocks<Sh>() == 5 ? 128 : whole_blocks<Sh>() == 2 ? 320 : 384;
 }
 
 template <class Sh, int NT>
@@ -360,17 +361,24 @@ __global__ void __launch_bounds__(NT, MINB) whole_inverse_kernel(InverseArgs a) 
 // column c at [i][c] of the buffer; pass 1 reads its elements straight from global memory (lanes
 // on consecutive columns), pass 2 the buffer.  The columns 0 and N/2 of the row spectra are real;
 // between rows and columns a slot [N][H] keeps their real parts in one element.
+// Up to 42 pair-rows and columns at a time, fewer where two buffers of that would not fit an SM:
+// wide tiles keep the columns' global accesses long (1160 images of 250 px, low-pass / spectrum /
+// flip: 583 / 252 / 289 us; 25 at a time with 128 threads, three CTAs per SM: 707 / 289 / 360;
+// 16 with five CTAs: 578 / 291 / 346; 63 with one: 755 / 287 / 317).
 template <class Sh>
 struct Tile {
-    static constexpr int NT = 128;
-    static constexpr int kChunks = (Sh::H + 24) / 25, PC = (Sh::H + kChunks - 1) / kChunks;
-    static constexpr int kTiles = (Sh::HS + 24) / 25, CT = (Sh::HS + kTiles - 1) / kTiles;
+    static constexpr int NT = 288, MINB = 2;
+    static constexpr size_t kRoom = 108 * 1024;
+    static constexpr int cut(int lines, size_t line_bytes) {           // lines per buffer
+        const int most = (int)(kRoom / line_bytes) < 42 ? (int)(kRoom / line_bytes) : 42;
+        const int parts = (lines + most - 1) / most;
+        return (lines + parts - 1) / parts;
+    }
+    static constexpr int PC = cut(Sh::H, Sh::S * sizeof(float2));
+    static constexpr int CT = cut(Sh::HS, Sh::N * sizeof(float2));
     static constexpr size_t kRowBytes = (size_t)PC * Sh::S * sizeof(float2);
     static constexpr size_t kColBytes = (size_t)Sh::N * CT * sizeof(float2);
     static constexpr size_t bytes = kRowBytes > kColBytes ? kRowBytes : kColBytes;
-    static constexpr int MINB = 4 * (bytes + sizeof(float2) * Sh::N + 1280) <= 227 * 1024   ? 4
-                                : 3 * (bytes + sizeof(float2) * Sh::N + 1280) <= 227 * 1024 ? 3
-                                                                                            : 2;
 };
 
 // the chunk's row spectra (Z in the buffer, pass 1 done) split and handed to put(row, c, value),
