@@ -132,13 +132,12 @@ struct mem_plan {
     // (MEM_FUSED_IMAGE=1; off by default: measured slower than the three kernels, see
     // image_stage_kernel)
     bool fused_image = false;
-    // boxes rotated by rotate_band: 1 = N > 236 (no whole-image shared-memory kernel), 2 = also
-    // N <= 236 other than 64 and 128, 0 = never (MEM_ROT_BAND)
+    // boxes rotated by rotate_band: 1 = N > 236 (no whole-image shared-memory kernel) and N >= 180
+    // without a compile-time kernel, 2 = all but 64 and 128, 0 = never (MEM_ROT_BAND)
     int rot_band = 1;
     // compile-time whole-image rotation of the mixed-radix sizes (MEM_ROT_WHOLE=0: the
     // runtime-size kernel, for comparison)
     bool rot_whole = true;
-    int rot_band_variant = 2;       // rotate_band's sampling / occupancy form (MEM_ROT_BAND_VARIANT)
     // host-to-device image copy of a split execute: the fewer SMs it occupies the less it slows
     // the concurrent computation; 8 x 1024 threads, two images per step, keep ~1 MB of loads in
     // flight, enough for the host link
@@ -228,8 +227,8 @@ int image_stage(const mem_plan& P, const mem_inputs& in, const float* gtab, cons
 int rotate(const mem_plan& P, const mem_inputs& in, float* xbuf, float* img_out,
            const PdDev* pd_table, const int32_t* img_pd, float2* spec, void* rot_scratch,
            cudaStream_t s);
-// the two rotations with the coefficient image in bands of rows (64 <= N <= 512; rotate calls it
-// for boxes without a shared-memory kernel); spec is the coefficient scratch
+// the two rotations with the coefficient image in bands of rows (64 <= N <= 512); spec holds the
+// first one's results
 bool rotate_band_supported(int N);
 int rotate_band(const mem_plan& P, float* xbuf, float2* spec, float* img_out, const void* rotc,
                 cudaStream_t s);

@@ -1243,12 +1243,16 @@ int rotate(const mem_plan& P, const mem_inputs& in, float* xbuf, float* img_out,
     RotConst* rotc = static_cast<RotConst*>(rot_scratch);
     const int st = rot_consts(P, in, pd_table, img_pd, rot_scratch, s);
     if (st != MEM_OK) return st;
+    // the banded kernel where no whole image fits, and for large boxes without a compile-time
+    // kernel (800 images of 190 px: 432 us, 456 with the runtime-size kernel; 1000 of 142 px: 327
+    // against 277)
     const bool fixed_n = N == 64 || N == 128;
+    const bool whole = P.rot_whole && mixed::rotate_supported(N);
     if (kern::rotate_band_supported(N) &&
-        ((P.rot_band >= 1 && N > kMaxSmemN) || (P.rot_band >= 2 && !fixed_n)))
+        ((P.rot_band >= 1 && (N > kMaxSmemN || (N >= 180 && !whole && P.rot_whole))) ||
+         (P.rot_band >= 2 && !fixed_n)))
         return kern::rotate_band(P, xbuf, spec, img_out, rotc, s);
-    if (P.rot_whole && mixed::rotate_supported(N))
-        return mixed::rotate(N, P.n_images, xbuf, img_out, rotc, s);
+    if (whole) return mixed::rotate(N, P.n_images, xbuf, img_out, rotc, s);
     if (N > kMaxSmemN) {
         constexpr int NT = 512;
         const int nseg = std::max(1, std::min(NT / N, N / 16));

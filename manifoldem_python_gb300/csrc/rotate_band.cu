@@ -1,22 +1,30 @@
 // The two periodic cubic B-spline rotations of rotatefill.op (modules/rotatefill.py:21-41,
 // called at modules/getDistanceCTF_local_Conj9combinedS2.py:328-330) for boxes whose
-// coefficient image does not fit one CTA's shared memory (64 < N <= 512 without a compile-time
-// kernel; N = 250 is the 1500-PD workload's box).  One CTA per image (512 threads, one CTA per
-// SM, by default; the launcher's variants are described at rotate_band).
+// coefficient image does not fit one CTA's shared memory (64 <= N <= 512).
 //
-// Each rotation is split where the separable prefilter splits:
-//   1. the prefilter along layout columns (every line runs across all N layout rows), from the
-//      input image in global memory to the image's scratch slot A: lanes on 32 consecutive
-//      columns, each thread's 32-sample segment of a column in registers (coalesced loads and
-//      stores, one L2 round trip per sample);
-//   2. for each band of H0 consecutive layout rows (plus the 3-row periodic halo of the 4x4
-//      window): the band's rows from A into shared memory, the prefilter along each row there
-//      (complete lines), the 3-column periodic halo, and every output sample whose window
-//      starts in the band, written straight to its output pixel.
+// One launch per rotation, one CTA per image and band of h consecutive layout rows:
+//   1. the prefilter along layout columns for the band's rows and the 3 below them (the 4x4
+//      window), straight from the input image in global memory: the recursions start kWarm rows
+//      outside (periodic; z1^20 = 4e-12 of a state is left out), so a band needs no other
+//      band's coefficients and no scratch; lanes on consecutive columns, segments of up to 32
+//      rows in registers;
+//   2. the prefilter along each of the band's rows in shared memory, and the 3-column halo;
+//   3. every output sample whose window starts in the band: along an output row the window's
+//      first layout row is linear in the column, so the samples in the band are up to three
+//      intervals of columns (the band and its periodic copies).  A warp owns every 16th output
+//      row; its lanes find the intervals of one row each, then walk those of two rows at a time
+//      together, 32 columns of each (paired FP32): stores are coalesced and few lanes idle.
 // The first rotation reads the low-passed image in its storage orientation (transposed), so its
 // layout rows are reference columns: it samples at (Y, X) and filters the reference rows first,
-// as the other rotation kernels do.  The second rotation reads the first one's output in the
-// reference orientation.  Outputs (and the second rotation's input) are reference-oriented.
+// as the other rotation kernels do; its result goes to the image's spectrum slot (free at this
+// point) in the reference orientation, where the second rotation reads it.
+//
+// Bound by shared-memory wavefronts (16 tap loads per sample, about two-way conflicts).  Three
+// bands of 84 rows at 250 px, two CTAs of 512 threads per SM.  1160 images of 250 px: 1032 us;
+// 1453 with one CTA per image working through the bands of both rotations, which was bound
+// by its barriers (one CTA per SM, the column coefficients through global scratch) and by the
+// sampling loops' idle lanes (611 K warp instructions per image).
+#include <algorithm>
 #include <cmath>
 
 #include "mem_internal.cuh"
@@ -26,152 +34,66 @@ namespace mem {
 namespace {
 
 using rot::kZ1;
-using rot::mask_ref;
 using rot::RotConst;
 
-constexpr int kBandThreads = 512;
+constexpr int kBandThreads = 512, kBandWarps = kBandThreads / 32;
 constexpr int kBandSeg = 32;                  // prefilter segment held in registers
-constexpr int kMaxBandN = kBandThreads;       // one output row per thread per pass at most
+constexpr int kWarm = 20;                     // rows before and after a band in the column pass
+constexpr int kMaxBandN = 512;                // a lane per output row of a warp: 16 x 32
+
+struct BandShape {
+    int N, P1, Pm1;                           // row strides = 1 and -1 mod 32
+    int H0, nb;                               // rows per band, bands
+    int cseg;                                 // column pass: segments of kBandSeg rows
+    int rseg;                                 // row pass: segments, the last one shorter
+    float zrlast;                             // z1^(length of the last row segment)
+};
 
 __device__ __forceinline__ int wrap_n(int i, int N) {      // i in [-N, 2N) -> [0, N)
     i += (i < 0) ? N : 0;
     return i - ((i >= N) ? N : 0);
 }
 
-// The three phases of one segment's prefilter (see prefilter_lines).  FULL: the segment has
-// kBandSeg samples (no per-sample length checks), else len < kBandSeg.  Sample k of the
-// segment is in[k * ks] (times the annular mask at (mrow, mcol0 + k) when MASK); GLOBAL: `in`
-// is global memory written earlier in this kernel (read through L2), else shared memory.
-template <bool FULL, bool GLOBAL, bool MASK>
-__device__ __forceinline__ float seg_causal_end(float* v, int len, const float* in, int ks,
-                                                int N, int mrow, int mcol0) {
+// The phases of one segment's prefilter in registers: the end state of the causal recursion
+// from zero; the causal recursion from state c and the anticausal end state from zero; the
+// anticausal recursion from state c.  FULL: kBandSeg samples, else len of them.
+template <bool FULL>
+__device__ __forceinline__ float seg_end(const float* v, int len) {
     float e = 0.f;
 #pragma unroll
-    for (int k = 0; k < kBandSeg; ++k) {
-        if (FULL || k < len) {
-            const float x = GLOBAL ? __ldcg(in) : *in;
-            v[k] = MASK ? x * mask_ref(mrow, mcol0 + k, N) : x;
-            e = fmaf(kZ1, e, v[k]);
-            in += ks;
-        }
-    }
+    for (int k = 0; k < kBandSeg; ++k)
+        if (FULL || k < len) e = fmaf(kZ1, e, v[k]);
     return e;
 }
-
 template <bool FULL>
 __device__ __forceinline__ float seg_causal(float* v, int len, float c) {
 #pragma unroll
-    for (int k = 0; k < kBandSeg; ++k) {
+    for (int k = 0; k < kBandSeg; ++k)
         if (FULL || k < len) {
             c = fmaf(kZ1, c, v[k]);
             v[k] = c;
         }
-    }
     float e = 0.f;
 #pragma unroll
     for (int k = kBandSeg - 1; k >= 0; --k)
         if (FULL || k < len) e = fmaf(kZ1, e, v[k]);
     return e;
 }
-
-// out points at sample len - 1 of the segment's output (stride ks)
+// sample k goes to x[k]
 template <bool FULL>
-__device__ __forceinline__ void seg_anticausal(const float* v, int len, float c, float* out,
-                                               int ks) {
+__device__ __forceinline__ void seg_anticausal(const float* v, int len, float c, float* x) {
     constexpr float gain = -6.0f * kZ1;
 #pragma unroll
-    for (int k = kBandSeg - 1; k >= 0; --k) {
+    for (int k = kBandSeg - 1; k >= 0; --k)
         if (FULL || k < len) {
             c = fmaf(kZ1, c, v[k]);
-            *out = gain * c;
-            out -= ks;
+            x[k] = gain * c;
         }
-    }
 }
 
-// One periodic prefilter pass over `lines` lines of N samples: sample k of line l is
-// in[l * ls + k * ks] (times the annular mask at (l, k) when MASK), its result goes to
-// out[l * ls + k * ks] (out may be in); GLOBAL: in and out are global memory, else shared.  Each line is split into nsg segments of kBandSeg
-// samples (the last one N - 32 (nsg - 1) long), one thread per segment with the segment in
-// registers.  Lines go in rounds of LPR = 32 floor(NT / (32 nsg)), a warp holding one segment
-// of 32 consecutive lines (so a warp's segments have one length).  Causal pass
-// c+[k] = x[k] + z1 c+[k-1]: each thread forms its segment's end state from zero,
-// E_g = sum_k z1^(L_g - 1 - k) x[k], and starts its recursion from E_{g-1} + z1^L_{g-1} E_{g-2}
-// (periodic in g; the omitted terms are below z1^58 = 6e-34 of the state).  The anticausal pass
-// c-[k] = c+[k] + z1 c-[k+1] does the same from the right, and the output is -6 z1 c-[k].
-// carry holds 2 NT floats.  Ends with a barrier.
-template <int NT, bool GLOBAL, bool MASK>
-__device__ __forceinline__ void prefilter_lines(int lines, int N, int nsg, float zlast,
-                                                float* carry, const float* in, float* out,
-                                                int ls, int ks) {
-    constexpr float zseg = rot::z1_pow<kBandSeg>();
-    const int lpr = 32 * (NT / (32 * nsg));
-    const int t = threadIdx.x;
-    const int lw = t % lpr, g = t / lpr;
-    const bool has_seg = g < nsg;
-    const int k0 = g * kBandSeg;
-    const int len = has_seg ? min(kBandSeg, N - k0) : 0;
-    const bool full = len == kBandSeg;               // the same for a whole warp
-    float* carry_c = carry;              // [nsg][lpr] causal end states
-    float* carry_a = carry + NT;         // [nsg][lpr] anticausal start states
-    const int g1 = g == 0 ? nsg - 1 : g - 1, g2 = g1 == 0 ? nsg - 1 : g1 - 1;
-    const int h1 = g == nsg - 1 ? 0 : g + 1, h2 = h1 == nsg - 1 ? 0 : h1 + 1;
-    const float zg1 = g1 == nsg - 1 ? zlast : zseg;
-    const float zh1 = h1 == nsg - 1 ? zlast : zseg;
-    for (int l0 = 0; l0 < lines; l0 += lpr) {
-        const int l = l0 + lw;
-        const bool active = has_seg && l < lines;
-        const int off = l * ls + k0 * ks;
-        float v[kBandSeg];
-        if (active)
-            carry_c[g * lpr + lw] =
-                    full ? seg_causal_end<true, GLOBAL, MASK>(v, len, in + off, ks, N, l, k0)
-                         : seg_causal_end<false, GLOBAL, MASK>(v, len, in + off, ks, N, l, k0);
-        __syncthreads();
-        if (active) {
-            const float c = fmaf(zg1, carry_c[g2 * lpr + lw], carry_c[g1 * lpr + lw]);
-            carry_a[g * lpr + lw] = full ? seg_causal<true>(v, len, c)
-                                         : seg_causal<false>(v, len, c);
-        }
-        __syncthreads();
-        if (active) {
-            const float c = fmaf(zh1, carry_a[h2 * lpr + lw], carry_a[h1 * lpr + lw]);
-            float* o = out + off + (len - 1) * ks;
-            if (full)
-                seg_anticausal<true>(v, len, c, o, ks);
-            else
-                seg_anticausal<false>(v, len, c, o, ks);
-        }
-        __syncthreads();
-    }
-}
-
-// One output sample from the band: layout coordinates (U, V) in 32.32 fixed point with the
-// window's -1 folded in, band row rho = the window's first layout row - b0, iv its first
-// layout column.
-__device__ __forceinline__ float sample_band(const float* s, int P, int rho, int iv, int64_t U,
-                                             int64_t V) {
-    const float tu = (float)(uint32_t)(U & 0xffffffffll) * 2.3283064365386963e-10f;
-    const float tv = (float)(uint32_t)(V & 0xffffffffll) * 2.3283064365386963e-10f;
-    float wu[4], wv[4];
-    rot::bspline_w(tu, wu);
-    rot::bspline_w(tv, wv);
-    const float* b = s + rho * P + iv;
-    float acc = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float r = wv[0] * b[i * P];
-        r = fmaf(wv[1], b[i * P + 1], r);
-        r = fmaf(wv[2], b[i * P + 2], r);
-        r = fmaf(wv[3], b[i * P + 3], r);
-        acc = fmaf(wu[i], r, acc);
-    }
-    return acc;
-}
-
-// Two output samples a, b from the band with paired FP32 instructions (as sample_fixed2 does
-// for the whole-image kernel): layout coordinates (U, V) in 32.32 fixed point with the window's
-// -1 folded in (see sample_band).
+// Two output samples a, b from the band with paired FP32 instructions: layout coordinates (U, V)
+// in 32.32 fixed point with the window's -1 folded in, band row rho = the window's first layout
+// row - b0, iv its first layout column.
 __device__ __forceinline__ float2 sample_band2(const float* s, int P, int rho_a, int iv_a,
                                                int64_t Ua, int64_t Va, int rho_b, int iv_b,
                                                int64_t Ub, int64_t Vb) {
@@ -197,137 +119,206 @@ __device__ __forceinline__ float2 sample_band2(const float* s, int P, int rho_a,
     return acc;
 }
 
-// One rotation: the layout-column prefilter from `in` to A, then the bands.  TRANS: `in` is
-// transposed (layout row u = reference column), masked with the annular mask on load.
-template <int NT, bool TRANS, bool PAIRED>
-__device__ __forceinline__ void rotate_banded(const float* in, float* A, float* out, float* s,
-                                              float* carry, const RotConst* Qp, int N, int P1,
-                                              int Pm1, int H0, int nb, int nsg, float zlast) {
-    // 1. along layout columns: line = column v, sample k = row u
-    // (TRANS: layout (u, v) is reference (v, u), masked by mask_ref(v, u))
-    prefilter_lines<NT, true, TRANS>(N, N, nsg, zlast, carry, in, A, 1, N);
-    // The band's row stride: a warp's lanes sample along an output row, a layout step of
-    // (rc, rs) (TRANS) or (rs, rc) per lane; tap (rho, iv) sits in bank (rho P + iv) mod 32, so
-    // P = 1 mod 32 keeps the bank index monotone across the lanes when the two components have
-    // one sign and P = -1 mod 32 when they have opposite signs (about two wavefronts per tap
-    // instruction either way, as in the whole-image kernels).  Qp is in shared memory, written
-    // before the column pass's barriers.
-    const int P = (Qp->rc > 0) == (Qp->rs > 0) ? P1 : Pm1;
-    constexpr int64_t kOne = 1ll << 32;
-    const int R = NT / N;
-    const int c = threadIdx.x % N, r0 = threadIdx.x / N;
-#pragma unroll 1
-    for (int b = 0; b < nb; ++b) {
-        const int b0 = b * H0, h = min(H0, N - b0), rows = h + 3;
-        // 2a. band rows b0 .. b0 + h + 2 (mod N) of A, a warp per row
-        for (int rho = threadIdx.x >> 5; rho < rows; rho += NT / 32) {
-            const float* src = A + (int64_t)wrap_n(b0 + rho, N) * N;
-            float* dst = s + rho * P;
-            for (int v = threadIdx.x & 31; v < N; v += 32) dst[v] = __ldcg(src + v);
-        }
-        __syncthreads();
-        // 2b. along layout rows, in shared memory (lanes on consecutive rows: the row stride is
-        // +-1 mod 32, so a warp's 32 accesses fall in 32 banks)
-        prefilter_lines<NT, false, false>(rows, N, nsg, zlast, carry, s, s, P, 1);
-        for (int p = threadIdx.x; p < rows * 3; p += NT) {
-            const int rho = p / 3, j = p - rho * 3;
-            s[rho * P + N + j] = s[rho * P + j];
-        }
-        __syncthreads();
-        // 2c. every output whose window starts in the band.  Thread (c, r0) owns rows
-        // r0 + j R, j < J; along them the window's first layout row U_j = U_0 + j dU is linear,
-        // so the rows in the band (its rows b0 .. b0 + h - 1, met as U in [b0, b0 + h) + k N,
-        // k = -1, 0, 1, since U stays within (-N, 2N)) are up to three ranges of j, found from
-        // U_0 and dU and widened by one step each way.  A warp walks the union of its lanes'
-        // ranges in step (its samples then lie along output rows, as in the whole-image
-        // kernels), two rows per iteration, and each sample checks its own row.
-        {
-            // the constants are read from shared memory after the band's barriers, so that
-            // nothing of the sampling stays live in registers through the prefilter
-            const RotConst Q = *Qp;
-            const bool lane_ok = r0 < R;
-            const int64_t X0 = Q.bx - kOne + (int64_t)r0 * Q.rc + (int64_t)c * Q.rs;
-            const int64_t Y0 = Q.by - kOne - (int64_t)r0 * Q.rs + (int64_t)c * Q.rc;
-            const int64_t dX = (int64_t)R * Q.rc, dY = -(int64_t)R * Q.rs;
-            const int64_t U0 = TRANS ? Y0 : X0, dU = TRANS ? dY : dX;
-            const int J = lane_ok ? (N - r0 + R - 1) / R : 0;
-#pragma unroll 1
-            for (int k = -1; k <= 1; ++k) {
-                int j0 = 0, j1 = J;
-                if (dU != 0) {
-                    // in layout rows: U_0 / 2^32 and dU / 2^32 (float is exact enough here:
-                    // the range is widened by a step each way)
-                    const float u0 = (float)U0 * 2.3283064365386963e-10f;
-                    const float inv = 4294967296.0f / (float)dU;
-                    const float ea = ((float)(b0 + k * N) - u0) * inv;
-                    const float eb = ((float)(b0 + h + k * N) - u0) * inv;
-                    const float lo = fminf(fmaxf(fminf(ea, eb), -2.f), (float)J + 2.f);
-                    const float hi = fminf(fmaxf(fmaxf(ea, eb), -2.f), (float)J + 2.f);
-                    j0 = max(0, (int)floorf(lo) - 1);
-                    j1 = min(J, (int)ceilf(hi) + 1);
-                } else if (k != 0) {
-                    j1 = 0;                        // a constant U: one pass (k = 0) over all rows
-                }
-                const bool some = j0 < j1;
-                const int w0 = __reduce_min_sync(0xffffffffu, some ? j0 : 0x7fffffff);
-                const int w1 = __reduce_max_sync(0xffffffffu, some ? j1 : 0);
-                if (w0 >= w1) continue;            // warp-uniform
-                int64_t X = X0 + (int64_t)w0 * dX, Y = Y0 + (int64_t)w0 * dY;
-                if constexpr (!PAIRED) {
-#pragma unroll 1
-                    for (int j = w0; j < w1; ++j, X += dX, Y += dY) {
-                        const int64_t U = TRANS ? Y : X, V = TRANS ? X : Y;
-                        const int f = (int)(U >> 32);
-                        const int rho = (dU == 0 ? wrap_n(f, N) : f - k * N) - b0;
-                        if (j >= J || (unsigned)rho >= (unsigned)h) continue;
-                        out[(int64_t)(r0 + j * R) * N + c] =
-                                sample_band(s, P, rho, wrap_n((int)(V >> 32), N), U, V);
+// TRANS: the first rotation (input transposed and masked on load, see above)
+template <bool TRANS>
+__global__ void __launch_bounds__(kBandThreads, 2) rotate_band_kernel(
+        const float* __restrict__ in, int64_t in_stride, float* __restrict__ out,
+        int64_t out_stride, const RotConst* __restrict__ rotc, const BandShape B) {
+    extern __shared__ float sm[];
+    float* carry_c = sm;                          // causal / anticausal segment end states
+    float* carry_a = sm + kBandThreads;
+    float* s = sm + 2 * kBandThreads;             // (H0 + 3) x P band
+    const int N = B.N, t = threadIdx.x;
+    const int64_t img = blockIdx.x / B.nb;
+    const int b0 = (int)(blockIdx.x % B.nb) * B.H0;
+    const int h = min(B.H0, N - b0), rows = h + 3;
+    const RotConst Q = rotc[2 * img + (TRANS ? 0 : 1)];
+    // A warp's lanes sample along an output row, a layout step of (rc, rs) (TRANS) or (rs, rc)
+    // per lane; tap (rho, iv) sits in bank (rho P + iv) mod 32, so P = 1 mod 32 keeps the bank
+    // index monotone across the lanes when the two components have one sign and P = -1 mod 32
+    // when they have opposite signs (about two wavefronts per tap instruction).
+    const int P = (Q.rc > 0) == (Q.rs > 0) ? B.P1 : B.Pm1;
+    const float* src = in + img * in_stride;
+    constexpr float zseg = rot::z1_pow<kBandSeg>();
+    // 1. layout columns: line v, sample i = layout row b0 - kWarm + i, cseg whole segments (the
+    // rows after the band's last warm the anticausal recursion up)
+    {
+        const int lpr = 32 * (kBandThreads / (32 * B.cseg));
+        const int lw = t % lpr, g = t / lpr;
+        const int i0 = g * kBandSeg - kWarm;                   // first row, counted from b0
+        const int u0 = wrap_n(b0 + i0, N);
+        const bool wraps = u0 + kBandSeg > N;                  // the same in a whole warp
+        for (int l0 = 0; l0 < N; l0 += lpr) {
+            const int line = l0 + lw;
+            const bool on = g < B.cseg && line < N;
+            float v[kBandSeg];
+            if (on) {
+                const float* p = src + u0 * N + line;
+                if (!wraps) {
+#pragma unroll
+                    for (int k = 0; k < kBandSeg; ++k, p += N) v[k] = __ldg(p);
+                } else {
+                    int u = u0;
+#pragma unroll
+                    for (int k = 0; k < kBandSeg; ++k) {
+                        v[k] = __ldg(p);
+                        const bool end = ++u == N;
+                        u = end ? 0 : u;
+                        p += end ? N - N * N : N;
                     }
-                    continue;
                 }
-#pragma unroll 1
-                for (int j = w0; j < w1; j += 2, X += 2 * dX, Y += 2 * dY) {
-                    const int64_t Ua = TRANS ? Y : X, Va = TRANS ? X : Y;
-                    const int64_t Ub = Ua + dU, Vb = Va + (TRANS ? dX : dY);
-                    const int fa = (int)(Ua >> 32), fb = (int)(Ub >> 32);
-                    int ra = (dU == 0 ? wrap_n(fa, N) : fa - k * N) - b0;
-                    int rb = (dU == 0 ? wrap_n(fb, N) : fb - k * N) - b0;
-                    const bool in_a = j < J && (unsigned)ra < (unsigned)h;
-                    const bool in_b = j + 1 < J && (unsigned)rb < (unsigned)h;
-                    if (!(in_a || in_b)) continue;
-                    ra = in_a ? ra : 0;            // a valid address for the unused half
-                    rb = in_b ? rb : 0;
-                    const float2 v = sample_band2(s, P, ra, wrap_n((int)(Va >> 32), N), Ua, Va,
-                                                  rb, wrap_n((int)(Vb >> 32), N), Ub, Vb);
-                    if (in_a) out[(int64_t)(r0 + j * R) * N + c] = v.x;
-                    if (in_b) out[(int64_t)(r0 + (j + 1) * R) * N + c] = v.y;
+                if (TRANS) {
+                    // mask_ref(line, u): (line - N/2 + 1)^2 + (u - N/2)^2 < (N/2)^2, exact in float
+                    const float hf = 0.5f * (float)N, x = (float)line - hf + 1.0f;
+                    const float d = hf * hf - x * x;
+                    float y = (float)u0 - hf;
+#pragma unroll
+                    for (int k = 0; k < kBandSeg; ++k) {
+                        v[k] = y * y < d ? v[k] : 0.f * v[k];
+                        y += 1.0f;
+                        if (wraps && y >= hf) y -= (float)N;
+                    }
+                }
+                carry_c[g * lpr + lw] = seg_end<true>(v, kBandSeg);
+            }
+            __syncthreads();
+            if (on) {
+                float c = g > 0 ? carry_c[(g - 1) * lpr + lw] : 0.f;
+                if (g > 1) c = fmaf(zseg, carry_c[(g - 2) * lpr + lw], c);
+                carry_a[g * lpr + lw] = seg_causal<true>(v, kBandSeg, c);
+            }
+            __syncthreads();
+            if (on) {
+                float c = g + 1 < B.cseg ? carry_a[(g + 1) * lpr + lw] : 0.f;
+                if (g + 2 < B.cseg) c = fmaf(zseg, carry_a[(g + 2) * lpr + lw], c);
+                constexpr float gain = -6.0f * kZ1;
+                float* x = s + (i0 + kBandSeg - 1) * P + line;
+#pragma unroll
+                for (int k = kBandSeg - 1; k >= 0; --k, x -= P) {
+                    c = fmaf(kZ1, c, v[k]);
+                    if ((unsigned)(i0 + k) < (unsigned)rows) *x = gain * c;
                 }
             }
         }
         __syncthreads();
     }
-}
-
-// xbuf: the low-passed image (storage orientation), then the first rotation's output; A: the
-// image's spectrum slot (>= N^2 floats, free at this point) as coefficient scratch.
-template <int NT, int MINB, bool PAIRED>
-__global__ void __launch_bounds__(NT, MINB) rotate_band_kernel(
-        float* xbuf, float2* spec, int64_t Kc, float* img_out, const RotConst* __restrict__ rotc,
-        int N, int P1, int Pm1, int H0, int nb, int nsg, float zlast) {
-    extern __shared__ float sm[];
-    float* carry = sm;                   // 2 NT floats
-    float* s = sm + 2 * NT;              // (H0 + 3) x max(P1, Pm1) band
-    const int64_t img = blockIdx.x;
-    const int64_t NN = (int64_t)N * N;
-    float* B = xbuf + img * NN;
-    float* A = reinterpret_cast<float*>(spec + img * Kc);
-    __shared__ RotConst rq[2];
-    if (threadIdx.x < 2) rq[threadIdx.x] = rotc[2 * img + threadIdx.x];
-    // rq is read after the first column pass's barriers; B is read by that pass before any
-    // band writes it
-    rotate_banded<NT, true, PAIRED>(B, A, B, s, carry, rq, N, P1, Pm1, H0, nb, nsg, zlast);
-    rotate_banded<NT, false, PAIRED>(B, A, img_out + img * NN, s, carry, rq + 1, N, P1, Pm1, H0,
-                                     nb, nsg, zlast);
+    // 2. layout rows, complete lines, in place (lanes on consecutive rows: the row stride is +-1
+    // mod 32, so a warp's accesses fall in 32 banks)
+    {
+        const int lpr = 32 * (kBandThreads / (32 * B.rseg));
+        const int lw = t % lpr, g = t / lpr;
+        const int k0 = g * kBandSeg, len = min(kBandSeg, N - k0);
+        const bool full = len == kBandSeg;                     // the same in a whole warp
+        const int g1 = g == 0 ? B.rseg - 1 : g - 1, g2 = g1 == 0 ? B.rseg - 1 : g1 - 1;
+        const int h1 = g == B.rseg - 1 ? 0 : g + 1, h2 = h1 == B.rseg - 1 ? 0 : h1 + 1;
+        const float zg1 = g1 == B.rseg - 1 ? B.zrlast : zseg;
+        const float zh1 = h1 == B.rseg - 1 ? B.zrlast : zseg;
+        for (int l0 = 0; l0 < rows; l0 += lpr) {
+            const int line = l0 + lw;
+            const bool on = g < B.rseg && line < rows;
+            float* x = s + line * P + k0;
+            float v[kBandSeg];
+            if (on) {
+#pragma unroll
+                for (int k = 0; k < kBandSeg; ++k)
+                    if (full || k < len) v[k] = x[k];
+                carry_c[g * lpr + lw] = full ? seg_end<true>(v, len) : seg_end<false>(v, len);
+            }
+            __syncthreads();
+            if (on) {
+                const float c = fmaf(zg1, carry_c[g2 * lpr + lw], carry_c[g1 * lpr + lw]);
+                carry_a[g * lpr + lw] =
+                        full ? seg_causal<true>(v, len, c) : seg_causal<false>(v, len, c);
+            }
+            __syncthreads();
+            if (on) {
+                const float c = fmaf(zh1, carry_a[h2 * lpr + lw], carry_a[h1 * lpr + lw]);
+                if (full)
+                    seg_anticausal<true>(v, len, c, x);
+                else
+                    seg_anticausal<false>(v, len, c, x);
+            }
+        }
+        __syncthreads();
+        for (int p = t; p < rows * 3; p += kBandThreads) {
+            const int rho = p / 3, j = p - rho * 3;
+            s[rho * P + N + j] = s[rho * P + j];
+        }
+        __syncthreads();
+    }
+    // 3. the samples.  Lane l finds the column intervals of output row warp + 16 l
+    constexpr int64_t kOne = 1ll << 32;
+    float* dst = out + img * out_stride;
+    const int warp = t >> 5, lane = t & 31;
+    const int64_t dXr = Q.rc, dYr = -Q.rs, dXc = Q.rs, dYc = Q.rc;     // steps per row, column
+    const int64_t dUr = TRANS ? dYr : dXr, dUc = TRANS ? dYc : dXc;
+    const int64_t dVr = TRANS ? dXr : dYr, dVc = TRANS ? dXc : dYc;
+    const int64_t U00 = (TRANS ? Q.by : Q.bx) - kOne, V00 = (TRANS ? Q.bx : Q.by) - kOne;
+    int lo[3], hi[3];
+    {
+        const int r = warp + kBandWarps * lane;
+        const int64_t Ur = U00 + (int64_t)r * dUr;
+        const float u0 = (float)Ur * 2.3283064365386963e-10f;
+        const float inv = 4294967296.0f / (float)dUc;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int base = b0 + (k - 1) * N;
+            lo[k] = 0;
+            hi[k] = N;
+            if (dUc != 0) {
+                // in layout rows; widened by a column each way (every sample checks its row)
+                const float ea = ((float)base - u0) * inv, eb = ((float)(base + h) - u0) * inv;
+                const float a = fminf(fmaxf(fminf(ea, eb), -2.f), (float)N + 2.f);
+                const float b = fminf(fmaxf(fmaxf(ea, eb), -2.f), (float)N + 2.f);
+                lo[k] = max(0, (int)floorf(a) - 1);
+                hi[k] = min(N, (int)ceilf(b) + 1);
+            } else {
+                const int f = (int)(Ur >> 32) - base;                  // a constant row
+                if (f < 0 || f >= h) hi[k] = 0;
+            }
+            if (r >= N) hi[k] = 0;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int base = b0 + (k - 1) * N;
+        unsigned todo = __ballot_sync(0xffffffffu, lo[k] < hi[k]);
+        while (todo) {                         // two rows with such an interval at a time
+            const int qa = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int qb = todo ? __ffs(todo) - 1 : qa;
+            const bool two = todo != 0;
+            todo &= todo - 1;
+            int ca = __shfl_sync(0xffffffffu, lo[k], qa), cb = __shfl_sync(0xffffffffu, lo[k], qb);
+            const int ea = __shfl_sync(0xffffffffu, hi[k], qa) - lane;
+            const int eb = two ? __shfl_sync(0xffffffffu, hi[k], qb) - lane : -1;
+            const int r = warp + kBandWarps * qa, r2 = warp + kBandWarps * qb;
+            int64_t Ua = U00 + (int64_t)r * dUr + (int64_t)(ca + lane) * dUc;
+            int64_t Va = V00 + (int64_t)r * dVr + (int64_t)(ca + lane) * dVc;
+            int64_t Ub = U00 + (int64_t)r2 * dUr + (int64_t)(cb + lane) * dUc;
+            int64_t Vb = V00 + (int64_t)r2 * dVr + (int64_t)(cb + lane) * dVc;
+            float* da = dst + r * N + ca + lane;
+            float* db = dst + r2 * N + cb + lane;
+            int left = max(ea - ca, eb - cb) + lane;           // the same in every lane
+#pragma unroll 1
+            for (; left > 0; left -= 32, ca += 32, cb += 32, da += 32, db += 32) {
+                int ra = (int)(Ua >> 32) - base, rb = (int)(Ub >> 32) - base;
+                const bool in_a = ca < ea && (unsigned)ra < (unsigned)h;
+                const bool in_b = cb < eb && (unsigned)rb < (unsigned)h;
+                ra = in_a ? ra : 0;            // a valid address for an unused half
+                rb = in_b ? rb : 0;
+                const int ia = in_a ? wrap_n((int)(Va >> 32), N) : 0;
+                const int ib = in_b ? wrap_n((int)(Vb >> 32), N) : 0;
+                const float2 v = sample_band2(s, P, ra, ia, Ua, Va, rb, ib, Ub, Vb);
+                if (in_a) *da = v.x;
+                if (in_b) *db = v.y;
+                Ua += 32 * dUc;
+                Va += 32 * dVc;
+                Ub += 32 * dUc;
+                Vb += 32 * dVc;
+            }
+        }
+    }
 }
 
 }  // namespace
@@ -341,38 +332,36 @@ int rotate_band(const mem_plan& P, float* xbuf, float2* spec, float* img_out, co
     if (P.n_images == 0) return MEM_OK;
     const int N = P.N;
     if (!rotate_band_supported(N) || P.Kc * 2 < (int64_t)N * N) return MEM_ERR_UNSUPPORTED;
-    // row strides >= N + 3 (the 3-column halo), one = 1 mod 32 and one = -1 mod 32 (the
-    // rotation picks one by its angle, see rotate_banded)
-    const int P1 = ((N + 3 + 30) / 32) * 32 + 1;
-    const int Pm1 = ((N + 3 + 32) / 32) * 32 - 1;
-    const int Pst = std::max(P1, Pm1);
-    // variant 0: one sample per step, 512 threads, two CTAs per SM; 1: two samples per step
-    // (paired FP32), 512 threads, two CTAs per SM; 2: two samples per step, 512 threads, one CTA
-    // per SM with the larger register file and bands up to 200 KB; 3: two samples per step,
-    // 1024 threads, one CTA per SM, bands up to 200 KB.  Bands: the fewest within the
-    // shared-memory budget (MEM_ROT_BANDS asks for more).
-    const int variant = P.rot_band_variant;
-    const int NT = variant == 3 ? 1024 : kBandThreads;
-    const size_t budget = (variant >= 2 ? 200 * 1024 : 100 * 1024) - 2 * NT * sizeof(float);
-    int nb = 1;
-    while ((size_t)((N + nb - 1) / nb + 3) * Pst * sizeof(float) > budget) ++nb;
-    if (const char* e = std::getenv("MEM_ROT_BANDS")) nb = std::max(nb, std::atoi(e));
-    const int H0 = (N + nb - 1) / nb;
-    nb = (N + H0 - 1) / H0;
-    const int nsg = (N + kBandSeg - 1) / kBandSeg;
-    const int last = N - kBandSeg * (nsg - 1);
-    const float zlast = (float)std::pow((double)kZ1, (double)last);
-    const size_t smem = (2 * NT + (size_t)(H0 + 3) * Pst) * sizeof(float);
-    if (smem > 227 * 1024) return MEM_ERR_UNSUPPORTED;
-    auto kfn = variant == 3   ? rotate_band_kernel<1024, 1, true>
-               : variant == 2 ? rotate_band_kernel<kBandThreads, 1, true>
-               : variant == 1 ? rotate_band_kernel<kBandThreads, 2, true>
-                              : rotate_band_kernel<kBandThreads, 2, false>;
-    MEM_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-    kfn<<<(unsigned)P.n_images, NT, smem, s>>>(
-            xbuf, spec, P.Kc, img_out, static_cast<const RotConst*>(rotc), N, P1, Pm1, H0, nb,
-            nsg, zlast);
+    BandShape B;
+    B.N = N;
+    // row strides >= N + 3 (the 3-column halo)
+    B.P1 = ((N + 3 + 30) / 32) * 32 + 1;
+    B.Pm1 = ((N + 3 + 32) / 32) * 32 - 1;
+    const int Pst = std::max(B.P1, B.Pm1);
+    // the fewest bands with two CTAs per SM (MEM_ROT_BANDS asks for more)
+    const size_t budget = 110 * 1024 - 2 * kBandThreads * sizeof(float);
+    B.nb = 1;
+    while ((size_t)((N + B.nb - 1) / B.nb + 3) * Pst * sizeof(float) > budget) ++B.nb;
+    if (const char* e = std::getenv("MEM_ROT_BANDS")) B.nb = std::max(B.nb, std::atoi(e));
+    B.H0 = (N + B.nb - 1) / B.nb;
+    B.nb = (N + B.H0 - 1) / B.H0;
+    B.cseg = (B.H0 + 3 + 2 * kWarm + kBandSeg - 1) / kBandSeg;
+    B.rseg = (N + kBandSeg - 1) / kBandSeg;
+    B.zrlast = (float)std::pow((double)kZ1, (double)(N - kBandSeg * (B.rseg - 1)));
+    const size_t smem = (2 * kBandThreads + (size_t)(B.H0 + 3) * Pst) * sizeof(float);
+    if (smem > 227 * 1024 || B.cseg > kBandWarps || B.rseg > kBandWarps)
+        return MEM_ERR_UNSUPPORTED;
+    const RotConst* rc = static_cast<const RotConst*>(rotc);
+    float* first = reinterpret_cast<float*>(spec);         // the first rotation's results
+    const int64_t NN = (int64_t)N * N;
+    const unsigned grid = (unsigned)(P.n_images * B.nb);
+    MEM_CUDA_TRY(cudaFuncSetAttribute(rotate_band_kernel<true>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    MEM_CUDA_TRY(cudaFuncSetAttribute(rotate_band_kernel<false>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    rotate_band_kernel<true><<<grid, kBandThreads, smem, s>>>(xbuf, NN, first, 2 * P.Kc, rc, B);
+    MEM_LAUNCH_CHECK();
+    rotate_band_kernel<false><<<grid, kBandThreads, smem, s>>>(first, 2 * P.Kc, img_out, NN, rc, B);
     MEM_LAUNCH_CHECK();
     return MEM_OK;
 }
