@@ -2,7 +2,7 @@
 // memory: the arithmetic and index maps of image_fft_mixed.cu.  Host-compilable, so that the
 // passes can be checked against numpy without a GPU.
 //
-// dft_any<R, DIR>: an in-register DFT of any length with prime factors 2, 3, 5, 7, 11, 13 (powers of
+// dft_any<R, DIR>: an in-register DFT of any length with prime factors up to 23 (powers of
 // two up to 16 are those of fft_radix.cuh; odd primes sum the half-length cosine and sine
 // products; composite lengths are Cooley-Tukey with constant twiddles).
 //

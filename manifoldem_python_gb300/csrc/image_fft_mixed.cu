@@ -1,7 +1,7 @@
 // Box sizes of the mixed-radix image transforms (fft_mixed_kernels.cuh) and their launches.
 //
-// The table holds even sizes from 36 to 512 px that factor as R1 R2 with R1 up to 16 (or 18,
-// 20, 25), R2 even and up to 32, and prime factors up to 13: about half of the even sizes and all
+// The table holds even sizes from 36 to 512 px that factor as R1 R2 with R1 up to 20, 23 or 25, R2
+// even and up to 32, and prime factors up to 23: two thirds of the even sizes up to 300 and all
 // the customary ones.  Other sizes keep cuFFT; 32, 64 and 128 px keep the kernels of image_fft.cu,
 // whose warps own their rows and columns (a spectrum of 128 px: 32 us per 1000 images).
 #include <algorithm>
@@ -15,15 +15,18 @@ namespace mixed {
     extern const Kernels kPart##i[]; \
     extern const int kPart##i##Count;
 MEM_PART(0) MEM_PART(1) MEM_PART(2) MEM_PART(3) MEM_PART(4) MEM_PART(5) MEM_PART(6) MEM_PART(7)
+MEM_PART(8) MEM_PART(9)
 #undef MEM_PART
 
 namespace {
 
 const Kernels* find(int N) {
-    const Kernels* parts[] = {kPart0, kPart1, kPart2, kPart3, kPart4, kPart5, kPart6, kPart7};
+    const Kernels* parts[] = {kPart0, kPart1, kPart2, kPart3, kPart4,
+                              kPart5, kPart6, kPart7, kPart8, kPart9};
     const int counts[] = {kPart0Count, kPart1Count, kPart2Count, kPart3Count,
-                          kPart4Count, kPart5Count, kPart6Count, kPart7Count};
-    for (int i = 0; i < 8; ++i)
+                          kPart4Count, kPart5Count, kPart6Count, kPart7Count,
+                          kPart8Count, kPart9Count};
+    for (int i = 0; i < 10; ++i)
         for (int j = 0; j < counts[i]; ++j)
             if (parts[i][j].N == N) return &parts[i][j];
     return nullptr;

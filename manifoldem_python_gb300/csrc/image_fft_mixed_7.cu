@@ -1,14 +1,14 @@
-// Image transforms and whole-image rotations of every eighth box size of the mixed-radix table
+// Image transforms and whole-image rotations of every tenth box size of the mixed-radix table
 // (see image_fft_mixed.cu); split over translation units to compile in parallel.
 #include "fft_mixed_kernels.cuh"
 
 namespace mem {
 namespace mixed {
 extern const Kernels kPart7[] = {
-    make_kernels<54, 9, 27, 54>(), make_kernels<84, 7, 28, 84>(), make_kernels<110, 11, 22, 55>(),
-    make_kernels<150, 15, 25, 150>(), make_kernels<182, 13, 26, 91>(),
-    make_kernels<220, 10, 10, 44>(), make_kernels<260, 13>(), make_kernels<312, 12>(),
-    make_kernels<360, 15>(), make_kernels<480, 20>(),
+    make_kernels<54, 9, 27, 54>(), make_kernels<90, 9, 18, 90>(), make_kernels<130, 13, 10, 65>(),
+    make_kernels<176, 11, 16, 88>(), make_kernels<220, 10, 10, 44>(), make_kernels<270, 15>(),
+    make_kernels<336, 14>(), make_kernels<432, 18>(), make_kernels<138, 23, 23, 138>(),
+    make_kernels<272, 17>(),
 };
 extern const int kPart7Count = sizeof(kPart7) / sizeof(kPart7[0]);
 }  // namespace mixed

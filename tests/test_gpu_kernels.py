@@ -201,8 +201,8 @@ def test_sums_of_many_and_of_few_items(cuda_ready, N, n_pd):
         d += counts[k] ** 2
 
 
-@pytest.mark.parametrize('N', [36, 42, 54, 66, 78, 100, 130, 150, 160, 200, 224, 234, 250, 256,
-                               324, 350, 400, 512])
+@pytest.mark.parametrize('N', [36, 42, 54, 66, 68, 78, 100, 130, 138, 150, 160, 190, 200, 224, 228,
+                               230, 234, 250, 256, 324, 350, 400, 512])
 def test_mixed_radix_transforms_match_cufft(cuda_ready, monkeypatch, N):
     """The shared-memory transforms of every radix family and both forms (whole image per CTA;
     rows and columns in tiles) against the cuFFT path of the same plan: SPIDER images with
@@ -253,8 +253,8 @@ def test_mixed_radix_transforms_match_cufft(cuda_ready, monkeypatch, N):
     assert bool(torch.isfinite(out['img_all'][[0, 2, 3, 4]]).all())
 
 
-@pytest.mark.parametrize('N', [36, 42, 50, 54, 70, 88, 96, 100, 144, 150, 162, 182, 192, 200, 220,
-                               224])
+@pytest.mark.parametrize('N', [36, 42, 50, 54, 70, 76, 88, 92, 96, 100, 144, 150, 162, 182, 190,
+                               192, 200, 204, 220, 224])
 def test_whole_image_rotation_matches_runtime_kernel(cuda_ready, monkeypatch, N):
     """The compile-time rotation of the mixed-radix sizes (segments of every length, several
     rounds, odd segments, the odd row stride of 224 px) against the runtime-size kernel, at angles
