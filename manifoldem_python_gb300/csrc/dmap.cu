@@ -18,6 +18,7 @@
 // block; everything else is float64.
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "mem_internal.cuh"
 
@@ -99,6 +100,17 @@ constexpr int kPer = 8, kMaxEps = 2048;
 constexpr int kSweepList = 256;                   // listed scales evaluated between two barriers
 constexpr float kExpOne = 1.4901161193847656e-8f; // 2^-26: exp2f(-d) = 1 for 0 <= d <= 2^-26
 
+// exp2(-d); PLAIN, for 0 <= d < 126 (normal results): the ex2.approx instruction alone.  With one
+// comparison per term and non-edges folded into +inf this takes the sweep's inner loop, which the
+// issue slots bound, from 600 to 296 us at n = 3000 and from 45 to 28 us at n = 300.
+template <bool PLAIN>
+__device__ __forceinline__ float exp2_neg(float d) {
+    if (!PLAIN) return exp2f(-d);
+    float v;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(v) : "f"(-d));
+    return v;
+}
+
 template <int NT>
 __global__ void __launch_bounds__(NT) dm_sweep_kernel(
         const double* __restrict__ Y, int64_t total, const float* __restrict__ scale,
@@ -108,7 +120,7 @@ __global__ void __launch_bounds__(NT) dm_sweep_kernel(
     __shared__ uint16_t list[kMaxEps];
     __shared__ float wsum[kSweepList][NW];
     __shared__ float wmin[NW], wmax[NW];
-    __shared__ int wzero[NW], wedge[NW], n_list;
+    __shared__ int wzero[NW], wedge[NW], n_list, n_odd;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (int e = t; e < n_eps; e += NT) part[e] = 0.0;
     const float tl = thr * 1.4426950408889634f;   // the threshold on d = Y/(2 eps), base 2
@@ -154,7 +166,10 @@ __global__ void __launch_bounds__(NT) dm_sweep_kernel(
             wzero[warp] = zero;
             wedge[warp] = edge;
         }
-        if (t == 0) n_list = 0;
+        if (t == 0) n_list = n_odd = 0;
+#pragma unroll
+        for (int u = 0; u < kPer; ++u)
+            if (!(y[u] >= 0.f)) y[u] = __int_as_float(0x7f800000);
         __syncthreads();
         for (int e = t; e < n_eps; e += NT) {
             const float c = scale[e];             // log2(e) / (2 eps)
@@ -171,30 +186,41 @@ __global__ void __launch_bounds__(NT) dm_sweep_kernel(
                 else
                     todo = true;
             }
-            if (todo)
+            if (todo) {
                 list[atomicAdd(&n_list, 1)] = (uint16_t)e;
-            else if (ones)
-                part[e] += (double)ones;
+                if (!(c > 0.f && c < __int_as_float(0x7f800000))) n_odd = 1;
+            }
+            if (!todo && ones) part[e] += (double)ones;
         }
         __syncthreads();
         const int nl = n_list;
+        const bool finite = n_odd == 0;
         for (int l0 = 0; l0 < nl; l0 += kSweepList) {
             const int l1 = min(nl, l0 + kSweepList);
+            // A term is exp2(-d log2(e)); beyond the threshold, and for a non-edge (kept as +inf
+            // here), 0.  scale is +inf for the smallest eps (beyond float range): zero-distance
+            // edges still give exp(0) = 1 there, all others are beyond the threshold.
+            auto evaluate = [&](auto plain) {
 #pragma unroll 2
-            for (int l = l0; l < l1; ++l) {
-                const float c = scale[list[l]];
-                float acc = 0.f;
+                for (int l = l0; l < l1; ++l) {
+                    const float c = scale[list[l]];
+                    float acc = 0.f;
 #pragma unroll
-                for (int u = 0; u < kPer; ++u) {
-                    // d log2(e); scale is +inf for the smallest eps (beyond float range):
-                    // zero-distance edges still give exp(0) = 1 there, all others are beyond
-                    // the threshold
-                    const float d2 = y[u] == 0.f ? 0.f : y[u] * c;
-                    acc += (y[u] >= 0.f && d2 < tl) ? exp2f(-d2) : 0.f;
+                    for (int u = 0; u < kPer; ++u) {
+                        const float d2 = decltype(plain)::value || y[u] != 0.f ? y[u] * c : 0.f;
+                        acc += d2 < tl ? exp2_neg<decltype(plain)::value>(d2) : 0.f;
+                    }
+                    for (int o = 16; o > 0; o >>= 1)
+                        acc += __shfl_xor_sync(0xffffffffu, acc, o);
+                    if (lane == 0) wsum[l - l0][warp] = acc;
                 }
-                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                if (lane == 0) wsum[l - l0][warp] = acc;
-            }
+            };
+            // the short form needs a finite scale in the whole list and a threshold that keeps
+            // the exponent out of the denormals
+            if (finite && tl <= 120.f)
+                evaluate(std::true_type{});
+            else
+                evaluate(std::false_type{});
             __syncthreads();
             for (int i = t; i < l1 - l0; i += NT) {
                 double s = 0.0;
@@ -219,7 +245,7 @@ __global__ void __launch_bounds__(NT) dm_sweep_kernel(
 // A column sum is split over the rows of a 16-column slice (64 row threads, added in a fixed
 // order), so that n = 300 already fills 19 SMs and n = 3000 all of them; one thread per column
 // walking all rows took 2498 + 1564 us at n = 3000 (now 162 + 34 + 30) and 249 + 148 us at
-// n = 300 (the whole embedding work there: 85 us now, 918 us before).
+// n = 300 (the whole embedding work there: 69 us now, 918 us before).
 __global__ void __launch_bounds__(256) dm_weights_kernel(double* __restrict__ W, int64_t n,
                                                          double inv_s2) {
     __shared__ double tb[kTile][kTile + 1];
