@@ -653,7 +653,7 @@ int image_stage(const mem_plan& P, const mem_inputs& in, const float* gtab, cons
 #define MEM_CALL(NV)                                                                           \
     do {                                                                                       \
         const size_t smem = std::max((size_t)(NV / 2) * NV * sizeof(float2),                   \
-                                     (size_t)(NV + 3) * rot::rot_stride<NV>() * sizeof(float)); \
+                                     (size_t)(NV + rot::kHalo) * rot::rot_stride<NV>() * sizeof(float)); \
         if (prepare(image_stage_kernel<NV>, smem) != MEM_OK) return MEM_ERR_CUDA;              \
         image_stage_kernel<NV><<<(unsigned)P.n_images, 2 * NV, smem, s>>>(                     \
                 in.stack, in.num_stack, in.stack_index, in.flip, gtab, twid, xbuf, img_out,    \

@@ -1271,7 +1271,7 @@ int rotate(const mem_plan& P, const mem_inputs& in, float* xbuf, float* img_out,
     constexpr int NT = 512;
     if (N == 128 || N == 64) {
         auto kfn = N == 128 ? rotate_fixed_kernel<NT, 128> : rotate_fixed_kernel<NT, 64>;
-        const size_t smem_f = (size_t)(N + 3) *
+        const size_t smem_f = (size_t)(N + rot::kHalo) *
                               (N == 128 ? rot_stride<128>() : rot_stride<64>()) * sizeof(float);
         MEM_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem_f));

@@ -34,30 +34,33 @@ __device__ __forceinline__ RotConst make_rot(double cs, double sn, int N) {
 }
 
 
-// The coefficient image sits in smem with a 3-pixel periodic halo: rows/columns N..N+2 repeat
-// 0..2, so the 4x4 taps at (r0..r0+3, c0..c0+3), r0, c0 in [0, N), need no further wrapping.
-template <int NT>
+// The coefficient image sits in smem with a periodic halo: rows/columns N..N+H-1 repeat 0..H-1, so
+// the 4x4 taps at (r0..r0+3, c0..c0+3), r0, c0 in [0, N), need no further wrapping (H = 3), nor
+// the 5x5 union of two samples' taps (H = kHalo).
+constexpr int kHalo = 4;
+
+template <int NT, int H = 3>
 __device__ __forceinline__ void fill_halo(float* s, int N, int P) {
     __syncthreads();
-    for (int p = threadIdx.x; p < 3 * N; p += NT) {
+    for (int p = threadIdx.x; p < H * N; p += NT) {
         const int r = p / N, c = p - r * N;
         s[(N + r) * P + c] = s[r * P + c];
     }
     __syncthreads();
-    for (int p = threadIdx.x; p < 3 * (N + 3); p += NT) {
-        const int r = p / 3, c = p - r * 3;
+    for (int p = threadIdx.x; p < H * (N + H); p += NT) {
+        const int r = p / H, c = p - r * H;
         s[r * P + N + c] = s[r * P + c];
     }
     __syncthreads();
 }
 
 
-// Row stride of the coefficient image in the compile-time kernels: >= N + 3 (halo) and = 1 mod 32,
+// Row stride of the coefficient image in the compile-time kernels: >= N + kHalo and = 1 mod 32,
 // so that the bank of tap (ix, iy) is (ix + iy) mod 32; a warp's 32 samples along a line whose
 // direction has components of one sign then meet at most about two to a bank.
 template <int N>
 __host__ __device__ constexpr int rot_stride() {
-    return ((N + 3 + 30) / 32) * 32 + 1;
+    return ((N + kHalo + 30) / 32) * 32 + 1;
 }
 
 template <int NT, int N>
@@ -149,7 +152,7 @@ __device__ __forceinline__ void bspline_w(float t, float w[4]) {
 }
 
 // Two output samples a, b at once with paired FP32 instructions (fma.rn.f32x2 and friends);
-// per sample the same operations in the same order as bspline_w / sample_fixed.
+// per sample the same operations in the same order as bspline_w.
 __device__ __forceinline__ void bspline_w2(float2 t, float2 w[4]) {
     const float2 one = make_float2(1.f, 1.f), sixth = make_float2(1.f / 6.f, 1.f / 6.f);
     const float2 two3 = make_float2(2.f / 3.f, 2.f / 3.f), half = make_float2(0.5f, 0.5f);
@@ -163,28 +166,44 @@ __device__ __forceinline__ void bspline_w2(float2 t, float2 w[4]) {
     w[2] = __ffma2_rn(u2, __ffma2_rn(half, u, mone), two3);
 }
 
-template <int N>
-__device__ __forceinline__ float2 sample_fixed2(const float* s, int64_t XA, int64_t YA, int64_t XB,
-                                                int64_t YB) {
-    constexpr int P = rot_stride<N>();
+// w[0..3] at offset `shift` (0 or 1) of a 5-tap window, 0 elsewhere: tap i
+__device__ __forceinline__ float2 shifted_w(const float2 w[4], int i, bool sa, bool sb) {
+    const float2 lo = i < 4 ? w[i] : make_float2(0.f, 0.f);
+    const float2 hi = i > 0 ? w[i - 1] : make_float2(0.f, 0.f);
+    return make_float2(sa ? hi.x : lo.x, sb ? hi.y : lo.y);
+}
+
+// Samples a and b one output pixel apart: a rotation keeps their distance, so their windows' first
+// rows and columns differ by at most one, and one set of 5x5 coefficients (origin at the smaller
+// row and column, wrapped by the caller's `at`) holds both 4x4 windows: 25 shared-memory loads for
+// two samples instead of 32.  A window's fifth row and column have weight 0, which leaves every
+// partial sum as it is, so the bits are those of two separate samples.
+template <int P, class At>
+__device__ __forceinline__ float2 sample_pair(int64_t XA, int64_t YA, int64_t XB, int64_t YB,
+                                              At at) {
     const float2 k32 = make_float2(2.3283064365386963e-10f, 2.3283064365386963e-10f);
     const float2 tx = __fmul2_rn(make_float2((float)(uint32_t)(XA & 0xffffffffll),
                                              (float)(uint32_t)(XB & 0xffffffffll)), k32);
     const float2 ty = __fmul2_rn(make_float2((float)(uint32_t)(YA & 0xffffffffll),
                                              (float)(uint32_t)(YB & 0xffffffffll)), k32);
-    float2 wx[4], wy[4];
+    float2 wx[4], wy[4], w5[5];
     bspline_w2(tx, wx);
     bspline_w2(ty, wy);
-    const float* a = s + ((int)(XA >> 32) & (N - 1)) * P + ((int)(YA >> 32) & (N - 1));
-    const float* b = s + ((int)(XB >> 32) & (N - 1)) * P + ((int)(YB >> 32) & (N - 1));
+    const int xa = (int)(XA >> 32), xb = (int)(XB >> 32);
+    const int ya = (int)(YA >> 32), yb = (int)(YB >> 32);
+    const float* a = at(min(xa, xb), min(ya, yb));
+#pragma unroll
+    for (int j = 0; j < 5; ++j) w5[j] = shifted_w(wy, j, ya > yb, yb > ya);
     float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float2 v = __fmul2_rn(wy[0], make_float2(a[i * P], b[i * P]));
-        v = __ffma2_rn(wy[1], make_float2(a[i * P + 1], b[i * P + 1]), v);
-        v = __ffma2_rn(wy[2], make_float2(a[i * P + 2], b[i * P + 2]), v);
-        v = __ffma2_rn(wy[3], make_float2(a[i * P + 3], b[i * P + 3]), v);
-        acc = __ffma2_rn(wx[i], v, acc);
+    for (int i = 0; i < 5; ++i) {
+        float c[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) c[j] = a[i * P + j];
+        float2 v = __fmul2_rn(w5[0], make_float2(c[0], c[0]));
+#pragma unroll
+        for (int j = 1; j < 5; ++j) v = __ffma2_rn(w5[j], make_float2(c[j], c[j]), v);
+        acc = __ffma2_rn(shifted_w(wx, i, xa > xb, xb > xa), v, acc);
     }
     return acc;
 }
@@ -197,7 +216,7 @@ __device__ __forceinline__ float2 sample_fixed2(const float* s, int64_t XA, int6
 // along axis 1 or 0.  Returns whether the lanes run along columns.
 template <int NT, int N>
 __device__ __forceinline__ bool rotate_once(const float* s, const RotConst& Q, float* keep) {
-    constexpr int R = NT / N, MAXV = N / R;
+    constexpr int P = rot_stride<N>(), R = NT / N, MAXV = N / R;
     constexpr int64_t kOne = 1ll << 32;
     const int u = threadIdx.x % N, v0 = (threadIdx.x / N) * MAXV;
     const bool along_cols = (Q.rc > 0) != (Q.rs > 0);
@@ -208,7 +227,9 @@ __device__ __forceinline__ bool rotate_once(const float* s, const RotConst& Q, f
     const int64_t dY = along_cols ? Q.rc : -Q.rs;
 #pragma unroll
     for (int k = 0; k < MAXV; k += 2) {
-        const float2 v = sample_fixed2<N>(s, X, Y, X + dX, Y + dY);
+        const float2 v = sample_pair<P>(X, Y, X + dX, Y + dY, [s](int x, int y) {
+            return s + (x & (N - 1)) * P + (y & (N - 1));
+        });
         keep[k] = v.x;
         keep[k + 1] = v.y;
         X += 2 * dX;
@@ -240,7 +261,7 @@ __device__ __forceinline__ void rotate_image(const float* __restrict__ xi, float
     }
     prefilter_fixed<NT, N, 0, true>(s, carry, keep);
     prefilter_fixed<NT, N, 1>(s, carry);
-    fill_halo<NT>(s, N, P);
+    fill_halo<NT, kHalo>(s, N, P);
     // the second prefilter starts on the axis of the first rotation's samples, from registers
     // (the prefilter's barriers precede its stores, so every thread has finished sampling)
     if (rotate_once<NT, N>(s, rot[0], keep)) {
@@ -250,7 +271,7 @@ __device__ __forceinline__ void rotate_image(const float* __restrict__ xi, float
         prefilter_fixed<NT, N, 1, true>(s, carry, keep);
         prefilter_fixed<NT, N, 0>(s, carry);
     }
-    fill_halo<NT>(s, N, P);
+    fill_halo<NT, kHalo>(s, N, P);
     const bool along_cols = rotate_once<NT, N>(s, rot[1], keep);
     const int u = threadIdx.x % N, v0 = (threadIdx.x / N) * MAXV;
     if (!along_cols) {

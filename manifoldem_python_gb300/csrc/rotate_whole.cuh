@@ -25,8 +25,8 @@ namespace rot {
 constexpr size_t kWholeSmem = 225 * 1024;
 template <int N, int CARRY>
 constexpr int whole_stride() {
-    constexpr int p = ((N + 3 + 30) / 32) * 32 + 1;
-    return ((size_t)(N + 3) * p + CARRY) * sizeof(float) <= kWholeSmem ? p : ((N + 3) | 1);
+    constexpr int p = ((N + kHalo + 30) / 32) * 32 + 1;
+    return ((size_t)(N + kHalo) * p + CARRY) * sizeof(float) <= kWholeSmem ? p : ((N + kHalo) | 1);
 }
 
 template <int N_, int SEG_, int LPR_>
@@ -36,7 +36,7 @@ struct WholeShape {
     static constexpr int TASKS = LPR * G, NT = (TASKS + 31) / 32 * 32;
     static constexpr int CARRY = 2 * TASKS;                    // floats
     static constexpr int P = whole_stride<N, CARRY>();
-    static constexpr size_t SMEM = ((size_t)(N + 3) * P + CARRY) * sizeof(float);
+    static constexpr size_t SMEM = ((size_t)(N + kHalo) * P + CARRY) * sizeof(float);
     static constexpr int BY_SMEM = (int)(kWholeSmem / SMEM), BY_REGS = 65536 / (NT * 64);
     static constexpr int MINB = BY_SMEM < 1 ? 1 : BY_SMEM < BY_REGS ? BY_SMEM
                                                   : BY_REGS < 1     ? 1
@@ -117,32 +117,6 @@ __device__ __forceinline__ int wrap_any(int i) {               // [-N, 2N) -> [0
     return i - ((i >= N) ? N : 0);
 }
 
-template <class Sh>
-__device__ __forceinline__ float2 sample_whole2(const float* s, int64_t XA, int64_t YA,
-                                                int64_t XB, int64_t YB) {
-    constexpr int P = Sh::P, N = Sh::N;
-    const float2 k32 = make_float2(2.3283064365386963e-10f, 2.3283064365386963e-10f);
-    const float2 tx = __fmul2_rn(make_float2((float)(uint32_t)(XA & 0xffffffffll),
-                                             (float)(uint32_t)(XB & 0xffffffffll)), k32);
-    const float2 ty = __fmul2_rn(make_float2((float)(uint32_t)(YA & 0xffffffffll),
-                                             (float)(uint32_t)(YB & 0xffffffffll)), k32);
-    float2 wx[4], wy[4];
-    bspline_w2(tx, wx);
-    bspline_w2(ty, wy);
-    const float* a = s + wrap_any<N>((int)(XA >> 32)) * P + wrap_any<N>((int)(YA >> 32));
-    const float* b = s + wrap_any<N>((int)(XB >> 32)) * P + wrap_any<N>((int)(YB >> 32));
-    float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float2 v = __fmul2_rn(wy[0], make_float2(a[i * P], b[i * P]));
-        v = __ffma2_rn(wy[1], make_float2(a[i * P + 1], b[i * P + 1]), v);
-        v = __ffma2_rn(wy[2], make_float2(a[i * P + 2], b[i * P + 2]), v);
-        v = __ffma2_rn(wy[3], make_float2(a[i * P + 3], b[i * P + 3]), v);
-        acc = __ffma2_rn(wx[i], v, acc);
-    }
-    return acc;
-}
-
 // One rotation of the coefficient image in s: the thread of (u, g) samples the outputs (g SEG + k,
 // u) when the lanes run along output rows, (u, g SEG + k) when they run along columns
 // (whichever lane step has components of one sign), into dst[(g SEG + k) N + u].
@@ -165,7 +139,10 @@ __device__ __forceinline__ bool rotate_whole_once(const float* s, const RotConst
             for (int k = 0; k < SEG; k += 2, X += 2 * dX, Y += 2 * dY, d += 2 * N) {
                 // an odd SEG's last sample alone: its partner repeats it
                 const bool two = SEG % 2 == 0 || k + 1 < SEG;
-                const float2 v = sample_whole2<Sh>(s, X, Y, two ? X + dX : X, two ? Y + dY : Y);
+                const float2 v = sample_pair<Sh::P>(
+                    X, Y, two ? X + dX : X, two ? Y + dY : Y, [s](int x, int y) {
+                        return s + wrap_any<N>(x) * Sh::P + wrap_any<N>(y);
+                    });
                 d[0] = v.x;
                 if (two) d[N] = v.y;
             }
@@ -193,7 +170,7 @@ __global__ void __launch_bounds__(Sh::NT, Sh::MINB) rotate_whole_kernel(
     const RotConst q0 = rotc[2 * img];
     prefilter_whole<Sh, 0, 1>(s, carry, xi);
     prefilter_whole<Sh, 1, 0>(s, carry, nullptr);
-    fill_halo<NT>(s, N, P);
+    fill_halo<NT, kHalo>(s, N, P);
     // every read of xi is behind a barrier: it takes the first rotation's samples; a thread's
     // samples are the prefilter segment it reads back, and the prefilter's barriers separate the
     // sampling from the stores into s
@@ -204,7 +181,7 @@ __global__ void __launch_bounds__(Sh::NT, Sh::MINB) rotate_whole_kernel(
         prefilter_whole<Sh, 1, 2>(s, carry, xi);
         prefilter_whole<Sh, 0, 0>(s, carry, nullptr);
     }
-    fill_halo<NT>(s, N, P);
+    fill_halo<NT, kHalo>(s, N, P);
     const RotConst q1 = rotc[2 * img + 1];
     const bool turned = (q1.rc > 0) != (q1.rs > 0);
     rotate_whole_once<Sh>(s, q1, turned ? xi : out);
