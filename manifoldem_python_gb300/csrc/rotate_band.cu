@@ -11,19 +11,21 @@
 //   2. the prefilter along each of the band's rows in shared memory, and the 3-column halo;
 //   3. every output sample whose window starts in the band: along an output row the window's
 //      first layout row is linear in the column, so the samples in the band are up to three
-//      intervals of columns (the band and its periodic copies).  A warp owns every 16th output
-//      row; its lanes find the intervals of one row each, then walk those of two rows at a time
-//      together, 32 columns of each (paired FP32): stores are coalesced and few lanes idle.
+//      intervals of columns (the band and its periodic copies).  A warp owns every 16th pair of
+//      output rows; its lanes find the intervals of one row each, then walk the pairs' intervals
+//      together, 32 columns of both rows (paired FP32): stores are coalesced and few lanes idle.
 // The first rotation reads the low-passed image in its storage orientation (transposed), so its
 // layout rows are reference columns: it samples at (Y, X) and filters the reference rows first,
 // as the other rotation kernels do; its result goes to the image's spectrum slot (free at this
 // point) in the reference orientation, where the second rotation reads it.
 //
-// Bound by shared-memory wavefronts (16 tap loads per sample, about two-way conflicts).  Three
-// bands of 84 rows at 250 px, two CTAs of 512 threads per SM.  1160 images of 250 px: 1032 us;
-// 1453 with one CTA per image working through the bands of both rotations, which was bound
-// by its barriers (one CTA per SM, the column coefficients through global scratch) and by the
-// sampling loops' idle lanes (611 K warp instructions per image).
+// Bound by issue slots, then shared-memory wavefronts (16 tap loads per sample, about two-way
+// conflicts; one 5x5 window for two samples, rot::sample_pair, has fewer loads but more
+// instructions and took 1016 us).  Three bands of 84 rows at 250 px, two CTAs of 512 threads per
+// SM.  1160 images of 250 px: 956 us; 1032 with the paired rows 16 apart (coordinates, column
+// counters and bounds of their own); 1453 with one CTA per image working through the bands of
+// both rotations, which was bound by its barriers (one CTA per SM, the column coefficients
+// through global scratch) and by the sampling loops' idle lanes.
 #include <algorithm>
 #include <cmath>
 
@@ -91,12 +93,10 @@ __device__ __forceinline__ void seg_anticausal(const float* v, int len, float c,
         }
 }
 
-// Two output samples a, b from the band with paired FP32 instructions: layout coordinates (U, V)
-// in 32.32 fixed point with the window's -1 folded in, band row rho = the window's first layout
-// row - b0, iv its first layout column.
-__device__ __forceinline__ float2 sample_band2(const float* s, int P, int rho_a, int iv_a,
-                                               int64_t Ua, int64_t Va, int rho_b, int iv_b,
-                                               int64_t Ub, int64_t Vb) {
+// Two output samples a, b from the band with paired FP32 instructions: fixed-point layout
+// coordinates (U, V) and the first coefficient of each window
+__device__ __forceinline__ float2 sample_band2(const float* a, const float* b, int P, int64_t Ua,
+                                               int64_t Va, int64_t Ub, int64_t Vb) {
     const float2 k32 = make_float2(2.3283064365386963e-10f, 2.3283064365386963e-10f);
     const float2 tu = __fmul2_rn(make_float2((float)(uint32_t)(Ua & 0xffffffffll),
                                              (float)(uint32_t)(Ub & 0xffffffffll)), k32);
@@ -105,8 +105,6 @@ __device__ __forceinline__ float2 sample_band2(const float* s, int P, int rho_a,
     float2 wu[4], wv[4];
     rot::bspline_w2(tu, wu);
     rot::bspline_w2(tv, wv);
-    const float* a = s + rho_a * P + iv_a;
-    const float* b = s + rho_b * P + iv_b;
     float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -246,7 +244,7 @@ __global__ void __launch_bounds__(kBandThreads, 2) rotate_band_kernel(
         }
         __syncthreads();
     }
-    // 3. the samples.  Lane l finds the column intervals of output row warp + 16 l
+    // 3. the samples.  Lane l finds the column intervals of row l % 2 of the warp's pair l / 2
     constexpr int64_t kOne = 1ll << 32;
     float* dst = out + img * out_stride;
     const int warp = t >> 5, lane = t & 31;
@@ -256,7 +254,7 @@ __global__ void __launch_bounds__(kBandThreads, 2) rotate_band_kernel(
     const int64_t U00 = (TRANS ? Q.by : Q.bx) - kOne, V00 = (TRANS ? Q.bx : Q.by) - kOne;
     int lo[3], hi[3];
     {
-        const int r = warp + kBandWarps * lane;
+        const int r = 2 * warp + 2 * kBandWarps * (lane >> 1) + (lane & 1);
         const int64_t Ur = U00 + (int64_t)r * dUr;
         const float u0 = (float)Ur * 2.3283064365386963e-10f;
         const float inv = 4294967296.0f / (float)dUc;
@@ -277,45 +275,42 @@ __global__ void __launch_bounds__(kBandThreads, 2) rotate_band_kernel(
                 if (f < 0 || f >= h) hi[k] = 0;
             }
             if (r >= N) hi[k] = 0;
+            // both rows of the pair: the even lane's interval covers the two
+            if (lo[k] >= hi[k]) {
+                lo[k] = N;
+                hi[k] = 0;
+            }
+            lo[k] = min(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], 1));
+            hi[k] = max(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], 1));
         }
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const int base = b0 + (k - 1) * N;
-        unsigned todo = __ballot_sync(0xffffffffu, lo[k] < hi[k]);
-        while (todo) {                         // two rows with such an interval at a time
-            const int qa = __ffs(todo) - 1;
+        unsigned todo = __ballot_sync(0xffffffffu, lo[k] < hi[k]) & 0x55555555u;
+        while (todo) {                         // two rows r, r + 1 at a time
+            const int q = __ffs(todo) - 1;
             todo &= todo - 1;
-            const int qb = todo ? __ffs(todo) - 1 : qa;
-            const bool two = todo != 0;
-            todo &= todo - 1;
-            int ca = __shfl_sync(0xffffffffu, lo[k], qa), cb = __shfl_sync(0xffffffffu, lo[k], qb);
-            const int ea = __shfl_sync(0xffffffffu, hi[k], qa) - lane;
-            const int eb = two ? __shfl_sync(0xffffffffu, hi[k], qb) - lane : -1;
-            const int r = warp + kBandWarps * qa, r2 = warp + kBandWarps * qb;
-            int64_t Ua = U00 + (int64_t)r * dUr + (int64_t)(ca + lane) * dUc;
-            int64_t Va = V00 + (int64_t)r * dVr + (int64_t)(ca + lane) * dVc;
-            int64_t Ub = U00 + (int64_t)r2 * dUr + (int64_t)(cb + lane) * dUc;
-            int64_t Vb = V00 + (int64_t)r2 * dVr + (int64_t)(cb + lane) * dVc;
-            float* da = dst + r * N + ca + lane;
-            float* db = dst + r2 * N + cb + lane;
-            int left = max(ea - ca, eb - cb) + lane;           // the same in every lane
+            int c = __shfl_sync(0xffffffffu, lo[k], q);
+            int left = __shfl_sync(0xffffffffu, hi[k], q) - c;     // the same in every lane
+            const int r = 2 * warp + kBandWarps * q;
+            const bool two = r + 1 < N;
+            int64_t U = U00 + (int64_t)r * dUr + (int64_t)(c + lane) * dUc;
+            int64_t V = V00 + (int64_t)r * dVr + (int64_t)(c + lane) * dVc;
+            float* d = dst + r * N + c + lane;
 #pragma unroll 1
-            for (; left > 0; left -= 32, ca += 32, cb += 32, da += 32, db += 32) {
-                int ra = (int)(Ua >> 32) - base, rb = (int)(Ub >> 32) - base;
-                const bool in_a = ca < ea && (unsigned)ra < (unsigned)h;
-                const bool in_b = cb < eb && (unsigned)rb < (unsigned)h;
-                ra = in_a ? ra : 0;            // a valid address for an unused half
-                rb = in_b ? rb : 0;
-                const int ia = in_a ? wrap_n((int)(Va >> 32), N) : 0;
-                const int ib = in_b ? wrap_n((int)(Vb >> 32), N) : 0;
-                const float2 v = sample_band2(s, P, ra, ia, Ua, Va, rb, ib, Ub, Vb);
-                if (in_a) *da = v.x;
-                if (in_b) *db = v.y;
-                Ua += 32 * dUc;
-                Va += 32 * dVc;
-                Ub += 32 * dUc;
-                Vb += 32 * dVc;
+            for (; left > 0; left -= 32, d += 32, U += 32 * dUc, V += 32 * dVc) {
+                const int64_t Ub = U + dUr, Vb = V + dVr;
+                const bool in_a = lane < left && (unsigned)((int)(U >> 32) - base) < (unsigned)h;
+                const bool in_b = two && lane < left &&
+                                  (unsigned)((int)(Ub >> 32) - base) < (unsigned)h;
+                // a valid address for an unused half
+                const float* a = s, *b = s;
+                if (in_a) a += ((int)(U >> 32) - base) * P + wrap_n((int)(V >> 32), N);
+                if (in_b) b += ((int)(Ub >> 32) - base) * P + wrap_n((int)(Vb >> 32), N);
+                const float2 v = sample_band2(a, b, P, U, V, Ub, Vb);
+                if (in_a) d[0] = v.x;
+                if (in_b) d[N] = v.y;
             }
         }
     }
