@@ -178,9 +178,10 @@ __device__ __forceinline__ float2 shifted_w(const float2 w[4], int i, bool sa, b
 // row and column, wrapped by the caller's `at`) holds both 4x4 windows: 25 shared-memory loads for
 // two samples instead of 32.  A window's fifth row and column have weight 0, which leaves every
 // partial sum as it is, so the bits are those of two separate samples.  Shared-memory wavefronts
-// bound the rotations; both of 10,000 images of 128 px: 1344 us with two separate windows, 1127 so.
-template <int P, class At>
-__device__ __forceinline__ float2 sample_pair(int64_t XA, int64_t YA, int64_t XB, int64_t YB,
+// bound the rotations; both of 10,000 images of 128 px: 1344 us with two separate windows, 1127 with
+// 25 loads, 1102 with the fifth row and column loaded only where the windows differ.
+template <class At>
+__device__ __forceinline__ float2 sample_pair(int64_t XA, int64_t YA, int64_t XB, int64_t YB, int P,
                                               At at) {
     const float2 k32 = make_float2(2.3283064365386963e-10f, 2.3283064365386963e-10f);
     const float2 tx = __fmul2_rn(make_float2((float)(uint32_t)(XA & 0xffffffffll),
@@ -200,7 +201,8 @@ __device__ __forceinline__ float2 sample_pair(int64_t XA, int64_t YA, int64_t XB
     for (int i = 0; i < 5; ++i) {
         float c[5];
 #pragma unroll
-        for (int j = 0; j < 5; ++j) c[j] = a[i * P + j];
+        for (int j = 0; j < 5; ++j)
+            c[j] = (i < 4 || xa != xb) && (j < 4 || ya != yb) ? a[i * P + j] : 0.f;
         float2 v = __fmul2_rn(w5[0], make_float2(c[0], c[0]));
 #pragma unroll
         for (int j = 1; j < 5; ++j) v = __ffma2_rn(w5[j], make_float2(c[j], c[j]), v);
@@ -228,7 +230,7 @@ __device__ __forceinline__ bool rotate_once(const float* s, const RotConst& Q, f
     const int64_t dY = along_cols ? Q.rc : -Q.rs;
 #pragma unroll
     for (int k = 0; k < MAXV; k += 2) {
-        const float2 v = sample_pair<P>(X, Y, X + dX, Y + dY, [s](int x, int y) {
+        const float2 v = sample_pair(X, Y, X + dX, Y + dY, P, [s](int x, int y) {
             return s + (x & (N - 1)) * P + (y & (N - 1));
         });
         keep[k] = v.x;

@@ -139,8 +139,8 @@ __device__ __forceinline__ bool rotate_whole_once(const float* s, const RotConst
             for (int k = 0; k < SEG; k += 2, X += 2 * dX, Y += 2 * dY, d += 2 * N) {
                 // an odd SEG's last sample alone: its partner repeats it
                 const bool two = SEG % 2 == 0 || k + 1 < SEG;
-                const float2 v = sample_pair<Sh::P>(
-                    X, Y, two ? X + dX : X, two ? Y + dY : Y, [s](int x, int y) {
+                const float2 v = sample_pair(
+                    X, Y, two ? X + dX : X, two ? Y + dY : Y, Sh::P, [s](int x, int y) {
                         return s + wrap_any<N>(x) * Sh::P + wrap_any<N>(y);
                     });
                 d[0] = v.x;
