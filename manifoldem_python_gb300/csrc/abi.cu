@@ -169,8 +169,11 @@ void feature_layout(mem_plan* P) {
                 ring_start.push_back((int32_t)i);
                 ring_m.push_back((int32_t)mk[order[i]]);
             }
-            pos_of[order[i]] = (int32_t)i;
-            ring_of[order[i]] = (int32_t)ring_m.size() - 1;
+            const int32_t R = (int32_t)ring_m.size() - 1;
+            const int kb = order[i] % Nh;
+            const bool w1 = kb == 0 || (N % 2 == 0 && kb == N / 2);
+            pos_of[order[i]] = (int32_t)((uint32_t)i | (uint32_t)R << 16 | (w1 ? 1u << 31 : 0u));
+            ring_of[order[i]] = R;
         }
         ring_start.push_back((int32_t)Kc);
         P->Kr = (int64_t)ring_m.size();

@@ -71,7 +71,8 @@ __device__ __forceinline__ int ctf_sign(int m, uint64_t qf, const CtfConst& cc) 
 // device tables of the feature layout (feature_layout): colmap [Kc_pad] = column of frequency
 // slot k within the r' / s' blocks; ring features: ring R = frequencies of |k|^2 = ring_m[R],
 // stored at positions ring_start[R] .. ring_start[R+1] of the ring order, pos_of[k] = position of
-// frequency k, ring_of[k] = its ring; chunks [n_chunks] = (A column, B column, negate B, add the
+// frequency k (16 bits), its ring (15 bits) and, in bit 31, whether its half-plane weight is 1;
+// ring_of[k] = its ring; chunks [n_chunks] = (A column, B column, negate B, add the
 // lo.lo product) of each 64-wide K chunk of the contraction
 struct FeatTables {
     const int32_t* colmap;
@@ -282,6 +283,7 @@ int apply_contraction(mem_plan* P, int n_classes, const mem_contraction_config* 
 // largest half-plane size for ring features (the features kernel keeps one float per frequency
 // in shared memory); larger boxes use per-frequency U', V' blocks
 constexpr int64_t kRingMaxKc = 40960;
+static_assert(kRingMaxKc <= 65536, "FeatTables::pos_of keeps a position in 16 bits");
 
 // sets Kc_pad, colmap, the ring tables, Kr, Kr_pad, Kf and the chunk schedule of a plan whose N,
 // Nh, Kc and ring_features are set
