@@ -907,7 +907,7 @@ __global__ void __launch_bounds__(256) pd_finalize_kernel(
 //     a frequency's ring, weight and position come from one table word: 10.6 K images of 128 px
 //     took 748 us with an evaluation and two divisions per frequency, 488 so.
 template <int MODE, bool RINGS, int NT>
-__global__ void __launch_bounds__(NT) features_kernel(
+__global__ void __launch_bounds__(NT, 1024 / NT) features_kernel(
         float2* __restrict__ spec, const uint64_t* __restrict__ qfix,
         const PdDev* __restrict__ pds, const int32_t* __restrict__ img_pd,
         const int32_t* __restrict__ img_row, const FeatTables ft,
@@ -932,9 +932,8 @@ __global__ void __launch_bounds__(NT) features_kernel(
     KSum acc;
     // C of frequency slot k (RINGS: its ring's), whether its half-plane weight is 1, and its place
     // in ring order
-    auto locate = [&](int64_t k, float* C, bool* w1, int* pos, int* sg) {
+    auto locate = [&](int64_t k, uint32_t o, float* C, bool* w1, int* pos, int* sg) {
         if (RINGS) {
-            const uint32_t o = (uint32_t)ft.pos_of[k];
             *pos = (int)(o & 0xffffu);
             *w1 = (o >> 31) != 0;
             const int R = (int)((o >> 16) & 0x7fffu);
@@ -962,7 +961,7 @@ __global__ void __launch_bounds__(NT) features_kernel(
         float C;
         bool w1;
         int pos, sg;
-        locate(k, &C, &w1, &pos, &sg);
+        locate(k, RINGS ? (uint32_t)ft.pos_of[k] : 0u, &C, &w1, &pos, &sg);
         const float sw = w1 ? 1.0f : 1.41421356237309505f;
         const float s2w = w1 ? 1.41421356237309505f : 2.0f;
         const float2 F = sp[k];
@@ -989,29 +988,44 @@ __global__ void __launch_bounds__(NT) features_kernel(
     // 8-byte centring-vector loads (pair_loads: Kc even, so both are aligned); the same
     // operations per element as feature(), the a_i terms summed in a second compensated pair
     KSum2 acc2;
-    auto feature_pair = [&](int64_t k, float (&f0)[4], float (&f1)[4]) {
+    // Loads of the next pair are issued before the current one is worked on
+    struct Loaded {
+        float4 F;
+        float2 mu[4];
+        uint32_t o0, o1;
+        int col;
+    };
+    auto load_pair = [&](int64_t k) {
+        Loaded d;
+        d.F = *reinterpret_cast<const float4*>(sp + k);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            d.mu[j] = *reinterpret_cast<const float2*>(mu + j * Kc_pad + k);
+        d.o0 = RINGS ? (uint32_t)ft.pos_of[k] : 0u;
+        d.o1 = RINGS ? (uint32_t)ft.pos_of[k + 1] : 0u;
+        d.col = ft.colmap[k];
+        return d;
+    };
+    auto feature_pair = [&](int64_t k, const Loaded& d, float (&f0)[4], float (&f1)[4]) {
         const float2 m1 = make_float2(-1.f, -1.f);
         auto sub2 = [&](float2 a, float2 b) { return __ffma2_rn(b, m1, a); };     // a - b
         float2 C;
         bool w0, wb;
         int pos0, posb, sg0, sg1;
-        locate(k, &C.x, &w0, &pos0, &sg0);
-        locate(k + 1, &C.y, &wb, &posb, &sg1);
+        locate(k, d.o0, &C.x, &w0, &pos0, &sg0);
+        locate(k + 1, d.o1, &C.y, &wb, &posb, &sg1);
         const float2 sw = make_float2(w0 ? 1.0f : 1.41421356237309505f,
                                       wb ? 1.0f : 1.41421356237309505f);
         const float2 s2w = make_float2(w0 ? 1.41421356237309505f : 2.0f,
                                        wb ? 1.41421356237309505f : 2.0f);
-        const float4 FF = *reinterpret_cast<const float4*>(sp + k);
+        const float4 FF = d.F;
         if (spectrum_out) *reinterpret_cast<float4*>(spectrum_out + img * Kc + k) = FF;
         const float2 Fx = make_float2(FF.x, FF.z), Fy = make_float2(FF.y, FF.w);
         const float2 u = __fmul2_rn(sw, __ffma2_rn(Fx, Fx, __fmul2_rn(Fy, Fy)));
         const float2 v = __fmul2_rn(sw, __fmul2_rn(C, C));
         const float2 q = __fmul2_rn(s2w, C);
         const float2 r = __fmul2_rn(q, Fx), sv = __fmul2_rn(q, Fy);
-        const float2 mu_u = *reinterpret_cast<const float2*>(mu + k);
-        const float2 mu_v = *reinterpret_cast<const float2*>(mu + Kc_pad + k);
-        const float2 mu_r = *reinterpret_cast<const float2*>(mu + 2 * Kc_pad + k);
-        const float2 mu_s = *reinterpret_cast<const float2*>(mu + 3 * Kc_pad + k);
+        const float2 mu_u = d.mu[0], mu_v = d.mu[1], mu_r = d.mu[2], mu_s = d.mu[3];
         const float2 half = make_float2(0.5f, 0.5f);
         // mu_u (v - mu_v) + mu_v u + mu_r (mu_r / 2 - r) + mu_s (mu_s / 2 - s)
         float2 a = __fmul2_rn(mu_u, sub2(v, mu_v));
@@ -1049,15 +1063,21 @@ __global__ void __launch_bounds__(NT) features_kernel(
     };
     // two consecutive slots per thread: they share a 64-wide chunk, so their feature columns
     // are adjacent (col even) and each block gets one paired store
+    Loaded next = {};
+    if (pair_loads && 2 * (int64_t)threadIdx.x < Kc) next = load_pair(2 * (int64_t)threadIdx.x);
     for (int64_t k = 2 * (int64_t)threadIdx.x; k < Kc_pad; k += 2 * NT) {
         float f0[4], f1[4];
+        int64_t col;
         if (pair_loads && k < Kc) {
-            feature_pair(k, f0, f1);
+            const Loaded d = next;
+            if (k + 2 * NT < Kc) next = load_pair(k + 2 * NT);
+            feature_pair(k, d, f0, f1);
+            col = d.col;
         } else {
             feature(k, f0);
             feature(k + 1, f1);
+            col = ft.colmap[k];
         }
-        const int64_t col = ft.colmap[k];
         if (!RINGS) {
             store2(col, f0[0], f1[0]);
             store2(Kr_pad + col, f0[1], f1[1]);
