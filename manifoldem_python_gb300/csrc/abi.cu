@@ -288,6 +288,26 @@ mem_contraction_config default_contraction() {
     return c;
 }
 
+// The default tile width of a plan's split-BF16 contraction.  A 128 x 128 tile is bound by the
+// shared-memory bytes of its operands (213 a clock wanted, 128 there), a 128 x 256 tile reads and
+// stages a quarter fewer of them per MMA, but pads small PDs more and takes 1.37 to 1.47 times as
+// long as a 128 x 128 tile; one tile runs per SM at a time, so that a launch takes whole waves of
+// tiles.  So the wide tile is taken where its waves, counted 1.5 fold, are fewer.  PDs of 1909 and
+// 3274 images of 128 px: 4 waves of narrow tiles 1096 us, 2 of wide ones 796; 24 PDs of 400: 2 and 2,
+// 551 and 759; 6 PDs of 1500 at 64 px: 4 and 3, 370 and 408.  The same bits in every schedule.
+static int32_t default_tile_width(const mem_plan& P, const mem_contraction_config& dc) {
+    if (dc.accumulators != 2 || P.tc_kahan) return dc.tile_n;
+    int64_t narrow = 0, wide = 0;
+    for (const auto& pd : P.pd) {
+        const int64_t nb = (pd.n + 127) / 128, nj = (pd.n + 255) / 256;
+        narrow += nb * (nb + 1) / 2;
+        for (int64_t I = 0; I < nb; ++I) wide += nj - I / 2;
+    }
+    const int64_t sms = std::max(P.num_sms, 1);
+    const int64_t wn = (narrow + sms - 1) / sms, ww = (wide + sms - 1) / sms;
+    return 3 * ww < 2 * wn ? 256 : 128;
+}
+
 int apply_contraction(mem_plan* P, int n_classes, const mem_contraction_config* classes) {
     if (n_classes < 1 || !classes) return MEM_ERR_INVALID;
     for (int k = 0; k < n_classes; ++k) {
@@ -438,10 +458,6 @@ int mem_plan_create(const mem_params* params, int32_t n_pd, const int32_t* pd_co
     if (const char* e = std::getenv("MEM_TC_GROUP_CHUNKS")) P->tc_group_chunks = std::atoi(e);
     if (const char* e = std::getenv("MEM_TC_KAHAN")) P->tc_kahan = std::atoi(e) != 0;
     if (const char* e = std::getenv("MEM_TC_TERMS")) P->tc_lolo = std::atoi(e) >= 4;
-    {
-        const mem_contraction_config dc = default_contraction();
-        apply_contraction(P, 1, &dc);
-    }
     // image transforms: the shared-memory FFT kernels where they exist (MEM_SMEM_FFT=0 selects
     // cuFFT, for comparison)
     if (const char* e = std::getenv("MEM_SMEM_FFT")) P->smem_fft = std::atoi(e) != 0;
@@ -465,6 +481,12 @@ int mem_plan_create(const mem_params* params, int32_t n_pd, const int32_t* pd_co
     if (!have_dev) {
         P->device = -1;
         P->num_sms = 152;
+    }
+    {
+        mem_contraction_config dc = default_contraction();
+        if (!std::getenv("MEM_TC_TILE_N") && !std::getenv("MEM_TC_TILE_M"))
+            dc.tile_n = default_tile_width(*P, dc);
+        apply_contraction(P, 1, &dc);
     }
     size_t work = 0;
     if (P->smem_fft) img_batches.clear();      // no cuFFT plan is used

@@ -383,3 +383,37 @@ def test_contraction_split_by_chunks(cuda_ready, N, counts):
         got.append(out['D'])
     assert bool(torch.isfinite(got[0]).all())
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize('counts,width', [([1900], 128), ([2300], 256), ([2305, 100], 256),
+                                          ([128 * 17 + 1], 256), ([700] * 8, 256)])
+def test_default_tile_width(cuda_ready, counts, width):
+    """The width chosen from a plan's PD sizes: the same D, bit for bit, as 128 x 128 tiles."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip('the expected widths are those of 152 SMs')
+
+    def tiles(cols):
+        return sum(sum(-(-n // cols) - 128 * i // cols for i in range(-(-n // 128)))
+                   for n in counts)
+    waves = [-(-tiles(c) // 152) for c in (128, 256)]
+    assert (256 if 3 * waves[1] < 2 * waves[0] else 128) == width
+    N, n = 32, sum(counts)
+    rng = np.random.default_rng(n)
+    stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
+    idx = torch.arange(n, device='cuda')
+    flip = torch.zeros(n, dtype=torch.uint8, device='cuda')
+    psi = torch.from_numpy(rng.uniform(-3, 3, n)).cuda()
+    df = torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda()
+    params = StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1,
+                         precision='bf16x3')
+    narrow = [dict(max_n=2 ** 31 - 1, persistent=0, accumulators=2)]
+    D = []
+    for c in (None, narrow):
+        plan = Plan(params, counts, [0.3] * len(counts), contraction=c)
+        out = plan.allocate_outputs(('D',))
+        plan.execute(stack, idx, flip, psi, df, out)
+        torch.cuda.synchronize()
+        D.append(out['D'].clone())
+    assert torch.equal(D[0], D[1]) and bool(torch.isfinite(D[0]).all())
