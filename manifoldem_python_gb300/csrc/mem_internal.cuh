@@ -85,7 +85,7 @@ struct FeatTables {
 
 struct Layout {
     size_t status, pd_table, sum_items, img_pd, img_row, tiles, tc_tiles;
-    size_t item_off, qfix, rotc, gtab, pd_max, colmap, twid, ident;
+    size_t item_off, qfix, rotc, gtab, pd_max, colmap, twid, ident, tables_end;
     size_t xbuf, spec, feat_a, feat_b, pair_norm, partial, means, avg_spec, avg_real, cufft_work;
     size_t tc_part, total;
 };

@@ -23,6 +23,11 @@ OUTPUT_NAMES = ('D', 'img_avg', 'img_avg_flip', 'img_all_intensity', 'img_all', 
                 'ctf', 'spectrum', 'pair_norm')
 DEFAULT_OUTPUTS = ('D', 'img_avg', 'img_avg_flip', 'img_all_intensity', 'img_all',
                    'img_all_flip', 'ctf')
+# Host results of up to this size in all are read back in one copy, larger ones array by array: a
+# copy costs about 20 us on the host (seven of them 150 us, one 55; one call of 100 images of 64 px
+# 672 us with torch views of one block, 472 with spans), and large arrays stay apart so that each
+# can be freed by itself.
+ONE_BLOCK_BYTES = 32 << 20
 
 
 @dataclasses.dataclass
@@ -103,6 +108,11 @@ class Plan:
 
     def allocate_outputs(self, names: Iterable[str] = DEFAULT_OUTPUTS) -> Dict[str, object]:
         import torch
+        return {k: torch.empty(shp, dtype=dt, device=self.device)
+                for k, (shp, dt) in self._output_shapes(names).items()}
+
+    def _output_shapes(self, names: Iterable[str]) -> Dict[str, tuple]:
+        import torch
         N = self.params.N
         n_pd, n_img = len(self.counts), self.n_images
         shapes = {
@@ -116,13 +126,24 @@ class Plan:
             'spectrum': ((n_img, N, N // 2 + 1, 2), torch.float32),
             'pair_norm': ((n_img,), torch.float64),
         }
-        out = {}
-        for name in names:
-            if name == 'D' and self.params.avg_only:
-                continue
-            shp, dt = shapes[name]
-            out[name] = torch.empty(shp, dtype=dt, device=self.device)
-        return out
+        return {k: shapes[k] for k in names if not (k == 'D' and self.params.avg_only)}
+
+    def _allocate_block(self, names: Iterable[str]):
+        """(outputs, block): outputs of up to ONE_BLOCK_BYTES in all as spans of one allocation,
+        which is read back in one copy; larger ones as ``allocate_outputs``, block None."""
+        import torch
+        spans, o = {}, 0
+        for k, (shape, dt) in self._output_shapes(names).items():
+            dt = np.float64 if dt == torch.float64 else np.float32
+            n = math.prod(shape) * np.dtype(dt).itemsize
+            spans[k] = Span(o, n, dt, shape)
+            o += _aligned(n)
+        if not 0 < o <= ONE_BLOCK_BYTES:
+            return self.allocate_outputs(names), None
+        block = torch.empty(o, dtype=torch.uint8, device=self.device)
+        for v in spans.values():
+            v.base = block.data_ptr()
+        return spans, block
 
     def execute(self, stack, stack_index, flip, psi_rad, df, outputs: Dict[str, object],
                 stream=None, shift_yx=None, pd_mask=None) -> None:
@@ -271,21 +292,21 @@ class DistanceStage:
         counts = [int(np.asarray(j.ind).shape[0]) for j in jobs]
         plan = Plan(self.params, counts, [g.psi_p for g in geoms], self.device)
         dev = self.device
-        sidx = torch.from_numpy(np.concatenate([g.stack_index for g in geoms])).to(dev)
-        flip = torch.from_numpy(np.concatenate([g.flip for g in geoms])).to(dev)
-        psi = torch.from_numpy(np.concatenate([g.psi_rad for g in geoms])).to(dev)
-        df = torch.from_numpy(np.concatenate([np.asarray(j.df, dtype=np.float64).reshape(-1)
-                                              for j in jobs])).to(dev)
-        outs = plan.allocate_outputs(outputs)
-        shifts = None
+        index = np.concatenate([g.stack_index for g in geoms])
+        arrays = [index, np.concatenate([g.psi_rad for g in geoms]),
+                  np.concatenate([np.asarray(j.df, dtype=np.float64).reshape(-1) for j in jobs]),
+                  np.concatenate([g.flip for g in geoms])]
         if sh is not None:
-            shifts = torch.from_numpy(relion_shifts(
-                np.concatenate([g.stack_index for g in geoms]), sh)).to(dev)
+            arrays.append(np.asarray(relion_shifts(index, sh)))
+        inputs, (sidx, psi, df, flip, *shifts) = to_device(arrays, dev)
+        shifts = shifts[0] if shifts else None
+        outs, block = (plan._allocate_block(outputs) if to_host
+                       else (plan.allocate_outputs(outputs), None))
         masks = mask.project(geoms) if mask is not None else None
         plan.execute(stack, sidx, flip, psi, df, outs, shift_yx=shifts, pd_mask=masks)
         torch.cuda.synchronize(dev)
         plan.device_status()
-        res = split_outputs(plan, counts, outs, to_host)
+        res = split_outputs(plan, counts, outs, to_host, block)
         if masks is not None:
             for r, m in zip(res, masks.bool()):
                 r['msk2'] = m.cpu().numpy() if to_host else m
@@ -537,13 +558,55 @@ class StreamedStage:
             p.device_status()
 
 
-def split_outputs(plan: Plan, counts: Sequence[int], outs: Dict[str, object], to_host: bool):
-    """Per-PD views of the batched outputs."""
+def _aligned(nbytes: int) -> int:
+    return -(-nbytes // 512) * 512
+
+
+class Span:
+    """An array inside a device block: what ``Plan.execute`` needs of a tensor (a torch view of
+    the block costs 5 us on the host, as much as a launch)."""
+    __slots__ = ('offset', 'nbytes', 'dtype', 'shape', 'base')
+
+    def __init__(self, offset, nbytes, dtype, shape):
+        self.offset, self.nbytes, self.dtype, self.shape = offset, nbytes, dtype, shape
+
+    def data_ptr(self) -> int:
+        return self.base + self.offset
+
+    def of(self, host: np.ndarray) -> np.ndarray:
+        """The array in a host copy of the block."""
+        return host[self.offset:self.offset + self.nbytes].view(self.dtype).reshape(self.shape)
+
+
+def to_device(arrays: Sequence[np.ndarray], device):
+    """(block, spans): host arrays copied to the device as one block (a copy of each would cost
+    about 15 us on the host, more than the per-entry tables of a small batch take to transfer)."""
+    import torch
+    spans, o = [], 0
+    for a in arrays:
+        spans.append(Span(o, a.nbytes, a.dtype, a.shape))
+        o += _aligned(a.nbytes)
+    host = np.empty(o, dtype=np.uint8)
+    for a, v in zip(arrays, spans):
+        v.of(host)[...] = a
+    block = torch.from_numpy(host).to(device)
+    for v in spans:
+        v.base = block.data_ptr()
+    return block, spans
+
+
+def split_outputs(plan: Plan, counts: Sequence[int], outs: Dict[str, object], to_host: bool,
+                  block=None):
+    """Per-PD views of the batched outputs (``block``: the allocation they are spans of)."""
     N = plan.params.N
     res = []
     img_off = np.concatenate([[0], np.cumsum(counts)])
     d_off = np.concatenate([[0], np.cumsum(np.asarray(counts, dtype=np.int64) ** 2)])
-    host = {k: (v.cpu().numpy() if to_host else v) for k, v in outs.items()}
+    if to_host and block is not None:
+        data = block.cpu().numpy()
+        host = {k: v.of(data) for k, v in outs.items()}
+    else:
+        host = {k: (v.cpu().numpy() if to_host else v) for k, v in outs.items()}
     for p, n in enumerate(counts):
         r = {}
         for k, v in host.items():

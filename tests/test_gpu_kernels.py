@@ -417,3 +417,32 @@ def test_default_tile_width(cuda_ready, counts, width):
         torch.cuda.synchronize()
         D.append(out['D'].clone())
     assert torch.equal(D[0], D[1]) and bool(torch.isfinite(D[0]).all())
+
+
+@pytest.mark.parametrize('N,relion', [(32, False), (36, True)])
+def test_outputs_read_back_in_one_block(cuda_ready, monkeypatch, N, relion):
+    """One copy each way for a small batch: the same arrays as with one copy per output."""
+    torch = cuda_ready
+    from manifoldem_python_gb300 import pipeline
+    from manifoldem_python_gb300.geometry import pd_geometry
+    rng = np.random.default_rng(N)
+    n = 41
+    q = rng.standard_normal((4, n))
+    q /= np.linalg.norm(q, axis=0)
+    df = rng.uniform(1e4, 3e4, n)
+    jobs = [pipeline.PdJob(ind=np.arange(a, b), q=q[:, a:b], df=df[a:b])
+            for a, b in ((0, 7), (7, 8), (8, n))]
+    geoms = [pd_geometry(j.ind, j.q, 2 * n) for j in jobs]
+    stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
+    sh = (rng.uniform(-3, 3, n), rng.uniform(-3, 3, n)) if relion else None
+    stage = pipeline.DistanceStage(pipeline.StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0,
+                                                        AmpContrast=0.1))
+    got = []
+    for limit in (pipeline.ONE_BLOCK_BYTES, 0):
+        monkeypatch.setattr(pipeline, 'ONE_BLOCK_BYTES', limit)
+        got.append(stage.run(jobs, stack, 2 * n, pipeline.OUTPUT_NAMES, geoms=geoms, sh=sh))
+    for a, b in zip(*got):
+        assert list(a) == list(b)
+        for k in a:
+            assert a[k].dtype == b[k].dtype and a[k].flags.writeable
+            np.testing.assert_array_equal(a[k], b[k])
