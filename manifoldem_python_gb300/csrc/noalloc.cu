@@ -61,7 +61,7 @@ size_t a256(size_t x) { return (x + 255) / 256 * 256; }
 // then the per-call tables and buffers.
 struct NoallocLayout {
     size_t status, colmap, pd_table, items, item_off, img_pd, img_row, tiles, qfix, partial, means,
-        avg_spec, pd_max, spec, feat_a, feat_b, pair_norm, total;   // the rest: scratch units
+        avg_spec, pd_max, feat_a, feat_b, pair_norm, spec, total;   // the rest: scratch units
 };
 
 NoallocLayout layout_for(const mem_plan& P) {
@@ -86,10 +86,10 @@ NoallocLayout layout_for(const mem_plan& P) {
     L.means = take(sizeof(float) * means_stride(P));
     L.avg_spec = take(sizeof(float) * 4 * P.Kc);
     L.pd_max = take(sizeof(uint32_t));
-    L.spec = take(sizeof(float) * 2 * P.Kc * P.n_images);
     L.feat_a = take(feat_elem * P.Kf * P.n_rows);
     L.feat_b = (feat_elem == 4) ? L.feat_a : take(feat_elem * P.Kf * P.n_rows);
     L.pair_norm = take(sizeof(double) * P.n_images);
+    L.spec = take(sizeof(float) * 2 * P.Kc * P.n_images);    // spectra off a 16-byte boundary only
     L.total = off;
     return L;
 }
@@ -106,12 +106,23 @@ long long ftab_hash(const std::vector<int32_t>& t) {
 
 // the per-call tables of a one-PD plan of n images, written on the device (no host copy):
 // the PD, the partial-sum items of kSumChunk images, image -> (PD, feature row), and the
-// upper-triangle tiles (I, J), I <= J < nb, in the host plan's order (I outer)
+// upper-triangle tiles (I, J), I <= J < nb, in the host plan's order (I outer); and zeros in the
+// status words and the padding rows of the feature matrices (the scratch keeps old contents).
+// One launch for all of it: three memsets and a copy of the spectra besides took 300 images of
+// 70 px 100 us, 76 so.
 __global__ void noalloc_tables_kernel(PdDev* __restrict__ pd, SumItem* __restrict__ items,
                                       int32_t* __restrict__ item_off, int32_t* __restrict__ img_pd,
                                       int32_t* __restrict__ img_row, Tile* __restrict__ tiles,
-                                      int n, int n_items, int nb, int n_tiles) {
+                                      int n, int n_items, int nb, int n_tiles,
+                                      uint32_t* __restrict__ status, uint4* __restrict__ pad_a,
+                                      uint4* __restrict__ pad_b, int64_t pad16) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    for (int64_t i = t; i < pad16; i += (int64_t)gridDim.x * blockDim.x) {
+        pad_a[i] = zero;
+        pad_b[i] = zero;
+    }
+    if (t < 4) status[t] = 0;
     if (t == 0) {
         *pd = PdDev{0, 0, 0, n, 0, 1.0, 0.0};
         item_off[0] = 0;
@@ -214,7 +225,6 @@ extern "C" int mem_pd_distances_noalloc(const mem_params* params, int32_t n, con
     void* ws = slot->ptr;
     cudaStream_t s = (cudaStream_t)stream;
 
-    MEM_CUDA_TRY(cudaMemsetAsync(at<char>(ws, L.status), 0, 16, s));
     {
         // the feature-layout tables: copied from the host only when the array holds another
         // box size's (first call on the device or a change of box size)
@@ -230,23 +240,26 @@ extern "C" int mem_pd_distances_noalloc(const mem_params* params, int32_t n, con
     const int nb = (n + kRowBlock - 1) / kRowBlock;
     const int n_items = (int)P.items.size(), n_tiles = (int)P.tiles.size();
     const int fill = std::max(n, std::max(n_items, n_tiles));
-    noalloc_tables_kernel<<<(fill + 255) / 256, 256, 0, s>>>(
+    const size_t feat_elem = (P.params.precision == MEM_PREC_FP32) ? 4 : 2;
+    const size_t row_bytes = feat_elem * P.Kf;               // whole 128-byte rows
+    const int64_t pad16 = (P.n_rows - n) * (int64_t)(row_bytes / 16);
+    const int64_t blocks = std::max<int64_t>((fill + 255) / 256,
+                                             std::min<int64_t>((pad16 + 255) / 256, 4 * P.num_sms));
+    noalloc_tables_kernel<<<(unsigned)blocks, 256, 0, s>>>(
         at<PdDev>(ws, L.pd_table), at<SumItem>(ws, L.items), at<int32_t>(ws, L.item_off),
         at<int32_t>(ws, L.img_pd), at<int32_t>(ws, L.img_row), at<Tile>(ws, L.tiles), n, n_items,
-        nb, n_tiles);
+        nb, n_tiles, at<uint32_t>(ws, L.status), at<uint4>(ws, L.feat_a + n * row_bytes),
+        at<uint4>(ws, L.feat_b + n * row_bytes), pad16);
     MEM_LAUNCH_CHECK();
-    // the feature kernel overwrites its spectrum with sign(C) F: work on a copy in the scratch
-    MEM_CUDA_TRY(cudaMemcpyAsync(at<char>(ws, L.spec), spectra, sizeof(float) * 2 * P.Kc * n,
-                                 cudaMemcpyDeviceToDevice, s));
-    // padding rows of the feature matrices must read as zero; the scratch keeps old contents
-    const size_t feat_elem = (P.params.precision == MEM_PREC_FP32) ? 4 : 2;
-    const size_t row_bytes = feat_elem * P.Kf;
-    const size_t pad_rows = (size_t)(P.n_rows - n);
-    if (pad_rows) {
-        MEM_CUDA_TRY(cudaMemsetAsync(at<char>(ws, L.feat_a) + n * row_bytes, 0, pad_rows * row_bytes, s));
-        if (L.feat_b != L.feat_a)
-            MEM_CUDA_TRY(cudaMemsetAsync(at<char>(ws, L.feat_b) + n * row_bytes, 0,
-                                         pad_rows * row_bytes, s));
+    // the kernels only read the spectra here, 16 bytes at a time: from the caller's array, or from
+    // a copy when it starts off a 16-byte boundary
+    const float2* spectra2 = reinterpret_cast<const float2*>(spectra);
+    size_t used = L.spec;
+    if ((reinterpret_cast<uintptr_t>(spectra) & 15) != 0) {
+        MEM_CUDA_TRY(cudaMemcpyAsync(at<char>(ws, L.spec), spectra, sizeof(float) * 2 * P.Kc * n,
+                                     cudaMemcpyDeviceToDevice, s));
+        spectra2 = at<float2>(ws, L.spec);
+        used = L.total;
     }
     mem_inputs in{};
     in.df = df;
@@ -256,7 +269,7 @@ extern "C" int mem_pd_distances_noalloc(const mem_params* params, int32_t n, con
         if (st != MEM_OK) return st; \
     } while (0)
     const PdDev* pds = at<PdDev>(ws, L.pd_table);
-    float2* spec = at<float2>(ws, L.spec);
+    float2* spec = const_cast<float2*>(spectra2);     // features: write_signed false, read only
     uint64_t* qf = at<uint64_t>(ws, L.qfix);
     uint32_t* pd_max = at<uint32_t>(ws, L.pd_max);
     const uint32_t* scale_bits = pd_max;
@@ -278,12 +291,12 @@ extern "C" int mem_pd_distances_noalloc(const mem_params* params, int32_t n, con
         // what the layout leaves of the array is scratch for the contraction of few tiles
         const int64_t T = (int64_t)P.tiles.size();
         const int64_t room =
-            (int64_t)(((size_t)MEM_NOALLOC_SCRATCH_BYTES - L.total) / kTcUnitBytes) - T;
+            (int64_t)(((size_t)MEM_NOALLOC_SCRATCH_BYTES - used) / kTcUnitBytes) - T;
         const int64_t units = room > 0 ? tc_split_units(T, P.n_chunks, room) : 0;
         NA_STEP(kern::gemm_split_bf16(P, at<char>(ws, L.feat_a), at<char>(ws, L.feat_b),
                                       pair_norm, scale_bits, at<Tile>(ws, L.tiles), pds,
                                       ft.chunks, D, at<uint32_t>(ws, L.status),
-                                      at<float>(ws, L.total), units, s));
+                                      at<float>(ws, used), units, s));
     }
 #undef NA_STEP
     return MEM_OK;

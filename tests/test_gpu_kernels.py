@@ -446,3 +446,29 @@ def test_outputs_read_back_in_one_block(cuda_ready, monkeypatch, N, relion):
         for k in a:
             assert a[k].dtype == b[k].dtype and a[k].flags.writeable
             np.testing.assert_array_equal(a[k], b[k])
+
+
+@pytest.mark.parametrize('N,n,precision', [(33, 5, 'fp32'), (64, 130, 'bf16x3'),
+                                           (70, 300, 'bf16x3')])
+def test_distances_from_spectra_at_any_address(cuda_ready, N, n, precision):
+    """Spectra on a 16-byte boundary are read in place, others through a copy: the same D, and the
+    caller's array is left as it was."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import StageParams
+    rng = np.random.default_rng(N + n)
+    host = rng.standard_normal((n, N, N // 2 + 1, 2)).astype(np.float32)
+    df = torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda()
+    params = StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1,
+                         precision=precision).to_c()
+    D = []
+    for lead in (0, 1, 2, 4):
+        buf = torch.empty(host.size + lead, dtype=torch.float32, device='cuda')
+        buf[lead:] = torch.from_numpy(host.reshape(-1)).cuda()
+        d = torch.full((n, n), float('nan'), dtype=torch.float64, device='cuda')
+        _call(torch, 'mem_pd_distances_noalloc', ctypes.byref(params), n,
+              buf[lead:].data_ptr(), df.data_ptr(), d.data_ptr())
+        torch.cuda.synchronize()
+        assert np.array_equal(buf[lead:].cpu().numpy(), host.reshape(-1))
+        D.append(d)
+    assert bool(torch.isfinite(D[0]).all())
+    assert all(torch.equal(D[0], d) for d in D[1:])
