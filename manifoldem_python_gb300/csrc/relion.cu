@@ -18,9 +18,11 @@
 // per segment holding it in registers; the states between segments go through shared memory.
 // Axis 0 comes first, its lines read from global memory (lanes on consecutive columns), and
 // axis 1 last, its results written to global memory (lanes on consecutive rows of the transposed
-// output): an image is read and written once, coalesced.  Bound by latency: 800 images of
-// 100 px take 111 us; with a whole line per thread (serial chains of 3 N) and the taps of every
-// output in FP64 it was 209 us.  Smaller boxes keep that form, whose start values are exact for
+// output): an image is read and written once, coalesced.  Bound by the latency of the
+// segments at a line's ends (their windows are mirrored or wrapped tap by tap, inner segments slide
+// theirs along the line): 800 images of 100 px take 98 us, 111 with mirrored taps everywhere and
+// two operations per anticausal step; 209 with a whole line per thread (serial chains of 3 N)
+// and the taps of every output in FP64.  512 threads: 98, a branch per output: 125.  Smaller boxes keep that form, whose start values are exact for
 // any length (relion_small_kernel).
 #include <algorithm>
 #include <cmath>
@@ -206,7 +208,7 @@ __device__ __forceinline__ void shift_axis(float* s, float* carry, const float* 
         const int line = l0 + lw;
         const bool on = g < ax.nseg && line < N;
         float* x = s + line * SL;
-        float v[kSeg];
+        float v[kSeg], line_end = 0.f;
         if (on) {
             float e = 0.f;
 #pragma unroll
@@ -237,38 +239,33 @@ __device__ __forceinline__ void shift_axis(float* s, float* carry, const float* 
             for (int k = 0; k < kSeg; ++k)
                 if (k < len) {
                     c = fmaf(z, c, v[k]);
-                    v[k] = c;
+                    v[k] = -z * c;                 // z (e - c) = fma(z, e, -z c): one step
                     before = last;
                     last = c;
                 }
+            const float end = (z / (z * z - 1.f)) * (last + z * before);
             float e = 0.f;
             if (g == ax.nseg - 1) {                    // the mirror's closed form at the end
-                e = (z / (z * z - 1.f)) * (last + z * before);
+                e = end;
 #pragma unroll
                 for (int k = kSeg - 1; k >= 0; --k)
-                    if (k < len - 1) e = z * (e - v[k]);
+                    if (k < len - 1) e = fmaf(z, e, v[k]);
             } else {
 #pragma unroll
                 for (int k = kSeg - 1; k >= 0; --k)
-                    if (k < len) e = z * (e - v[k]);
+                    if (k < len) e = fmaf(z, e, v[k]);
             }
             carry_a[g * ax.lpr + lw] = e;
+            line_end = end;
         }
         __syncthreads();
         if (on) {
             if (g == ax.nseg - 1) {
-                float last = 0.f, before = 0.f;
-#pragma unroll
-                for (int k = 0; k < kSeg; ++k)
-                    if (k < len) {
-                        before = last;
-                        last = v[k];
-                    }
-                float c = (z / (z * z - 1.f)) * (last + z * before);
+                float c = line_end;
 #pragma unroll
                 for (int k = kSeg - 1; k >= 0; --k)
                     if (k < len) {
-                        if (k < len - 1) c = z * (c - v[k]);
+                        if (k < len - 1) c = fmaf(z, c, v[k]);
                         x[(k0 + k) * SK] = 6.f * c;
                     }
             } else {
@@ -280,18 +277,34 @@ __device__ __forceinline__ void shift_axis(float* s, float* carry, const float* 
 #pragma unroll
                 for (int k = kSeg - 1; k >= 0; --k)
                     if (k < len) {
-                        c = z * (c - v[k]);
+                        c = fmaf(z, c, v[k]);
                         x[(k0 + k) * SK] = 6.f * c;
                     }
             }
         }
         __syncthreads();
-        if (on) {
+        const int f0 = k0 + i0;
+        if (on && f0 >= 1 && f0 + len <= N - 2) {
+            // every window inside the line: taps f - 1 .. f + 2 slide along it
+            const float* q = x + (f0 - 1) * SK;
+            float a = q[0], b = q[SK], c = q[2 * SK];
+            q += 3 * SK;
+#pragma unroll
+            for (int k = 0; k < kSeg; ++k)
+                if (k < len) {
+                    const float d = *q;
+                    q += SK;
+                    v[k] = fmaf(w[3], d, fmaf(w[2], c, fmaf(w[1], b, w[0] * a)));
+                    a = b;
+                    b = c;
+                    c = d;
+                }
+        } else if (on) {
 #pragma unroll
             for (int k = 0; k < kSeg; ++k)
                 if (k < len) {
                     // wrapped with period N - 1 where the sample point lies outside [0, N - 1]
-                    int f = k0 + k + i0;
+                    int f = f0 + k;
                     if (f < 0 || f > N - 1 || (f == N - 1 && t > 0.f)) {
                         const bool below = f < 0;
                         f %= N - 1;
