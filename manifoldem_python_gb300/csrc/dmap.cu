@@ -29,13 +29,29 @@ constexpr double kZeroDist = 1e-6;
 constexpr int kTile = 32;
 
 // 1. Y from D (row-major n x n); listed = nullptr: every entry is a listed neighbour (k = n).
+// s_ij^2 and s_ji^2 are D_ji and D_ij themselves, so square roots are left for the product of two
+// different entries; where they are equal, as in every D of the distance stage, Y_ij = D_ij.
 // One CTA per unordered pair of 32 x 32 tiles (bi, bj), bi <= bj: it reads both tiles once and
-// writes both, and a pair of entries shares its square roots -- one where D_ij and D_ji are
-// equal, as in every D of the distance stage -- because FP64 (2 FMA per clock and SM) bounds
-// this kernel: n = 3000 takes 152 us, 387 us with four square roots per pair.
-__device__ __forceinline__ double dm_pair_value(double sij, double sji, bool zero_edge) {
-    const double y = sij * sij + sji * sji - sij * sji;
-    return (y != 0.0 || zero_edge) ? y : -1.0;
+// writes both.  Bound by memory for a symmetric D: n = 3000 takes 36 us; 152 with a square root
+// per pair, where FP64 (2 FMA per clock and SM) bounded it, and 387 with four.
+// Comparisons are on the bit patterns (positive doubles sort as integers), off the FP64 unit.
+constexpr long long kInfBits = 0x7ff0000000000000ll;
+// kZeroDist <= d <= inf
+__device__ __forceinline__ bool dm_far(double d) {
+    const long long zero = __double_as_longlong(kZeroDist);
+    return (unsigned long long)(__double_as_longlong(d) - zero) <=
+           (unsigned long long)(kInfBits - zero);
+}
+__device__ __forceinline__ bool dm_nan(double d) {
+    return (__double_as_longlong(d) & 0x7fffffffffffffffll) > kInfBits;
+}
+// Y of a pair with at least one of u1 (s_ij = sqrt(D_ji) counts) and u2 (s_ji); NaN where an
+// infinite distance counts
+__device__ __forceinline__ double dm_pair_value(double dij, double dji, bool u1, bool u2) {
+    const long long a = __double_as_longlong(dij), b = __double_as_longlong(dji);
+    if (u1 && u2 && a != b) return dji + dij - sqrt(dji) * sqrt(dij);
+    const long long v = u1 ? b : a;
+    return __longlong_as_double(v == kInfBits ? 0x7ff8000000000000ll : v);
 }
 
 __global__ void __launch_bounds__(256) dm_sym_kernel(
@@ -68,14 +84,15 @@ __global__ void __launch_bounds__(256) dm_sym_kernel(
         if (i >= n || j >= n) continue;
         const double dji = tY[tx][r];                          // D_ji
         const bool l1 = lij[q] != 0, l2 = tL[tx][r] != 0;      // j listed for i, i listed for j
-        const bool u1 = l1 && i != j && dji >= kZeroDist;      // s_ij = sqrt(D_ji)
-        const bool u2 = l2 && i != j && dij[q] >= kZeroDist;   // s_ji = sqrt(D_ij)
-        const double rji = (u1 || u2) ? sqrt(dji) : 0.0;
-        const double sij = u1 ? rji : 0.0;
-        const double sji = u2 ? (dij[q] == dji ? rji : sqrt(dij[q])) : 0.0;
-        Y[i * n + j] = dm_pair_value(sij, sji, l1 && (i == j || dji < kZeroDist));
+        const bool far1 = i != j && dm_far(dji), far2 = i != j && dm_far(dij[q]);
+        const bool u1 = l1 && far1, u2 = l2 && far2;           // s_ij, s_ji are not 0
+        const double y = u1 || u2 ? dm_pair_value(dij[q], dji, u1, u2) : -1.0;
+        // a pair of s = 0 is an edge where a listed distance is below kZeroDist
+        const bool z1 = l1 && (i == j || !(far1 || dm_nan(dji)));
+        const bool z2 = l2 && (i == j || !(far2 || dm_nan(dij[q])));
+        Y[i * n + j] = u1 || u2 || !z1 ? y : 0.0;
         // this thread alone reads and writes element (tx, r) of the shared tile
-        tY[tx][r] = dm_pair_value(sji, sij, l2 && (i == j || dij[q] < kZeroDist));
+        tY[tx][r] = u1 || u2 || !z2 ? y : 0.0;
     }
     if (bi == bj) return;                          // the diagonal tile is complete
     __syncthreads();
@@ -244,8 +261,14 @@ __global__ void __launch_bounds__(NT) dm_sweep_kernel(
 //   d. L_ij = W_ij f_i f_j with f = 1 / (d e), L = |L + L^T| / 2, tile pairs.
 // A column sum is split over the rows of a 16-column slice (64 row threads, added in a fixed
 // order), so that n = 300 already fills 19 SMs and n = 3000 all of them; one thread per column
-// walking all rows took 2498 + 1564 us at n = 3000 (now 162 + 34 + 30) and 249 + 148 us at
-// n = 300 (the whole embedding work there: 69 us now, 918 us before).
+// walking all rows took 2498 + 1564 us at n = 3000 (now 153 + 34 + 30) and 249 + 148 us at
+// n = 300 (the whole embedding work there: 65 us now, 918 us before).
+// y >= 0 by the bit pattern (-0 included, a NaN not)
+__device__ __forceinline__ bool dm_edge(double y) {
+    const long long v = __double_as_longlong(y);
+    return v >= 0 ? v <= kInfBits : (v << 1) == 0;
+}
+
 __global__ void __launch_bounds__(256) dm_weights_kernel(double* __restrict__ W, int64_t n,
                                                          double inv_s2) {
     __shared__ double tb[kTile][kTile + 1];
@@ -264,8 +287,9 @@ __global__ void __launch_bounds__(256) dm_weights_kernel(double* __restrict__ W,
     for (int q = 0; q < kTile / 8; ++q) {
         const int r = ty + 8 * q;
         const double yij = a[q], yji = tb[tx][r];
-        const double wij = yij >= 0.0 ? exp(-yij * inv_s2) : 0.0;
-        const double wji = yji == yij ? wij : (yji >= 0.0 ? exp(-yji * inv_s2) : 0.0);
+        const bool same = __double_as_longlong(yij) == __double_as_longlong(yji);
+        const double wij = dm_edge(yij) ? exp(-yij * inv_s2) : 0.0;
+        const double wji = same ? wij : (dm_edge(yji) ? exp(-yji * inv_s2) : 0.0);
         if (bi + r < n && bj + tx < n) W[(bi + r) * n + bj + tx] = wij;
         tb[tx][r] = wji;
     }

@@ -472,3 +472,29 @@ def test_distances_from_spectra_at_any_address(cuda_ready, N, n, precision):
         D.append(d)
     assert bool(torch.isfinite(D[0]).all())
     assert all(torch.equal(D[0], d) for d in D[1:])
+
+
+@pytest.mark.parametrize('n,knn', [(7, False), (40, True), (97, True)])
+def test_symmetrised_distances_of_special_values(cuda_ready, n, knn):
+    """Infinite, NaN, negative, tiny and unequal entries, one-sided lists: NaN, non-edges and zeros
+    where numpy has them, values to 1e-14."""
+    torch = cuda_ready
+    rng = np.random.default_rng(n)
+    special = np.array([np.inf, np.nan, -1.0, -0.0, 0.0, 9.99e-7, 1e-6, 1e300, 5e-324, -np.inf])
+    D = _dm_matrix(n, n, False)
+    put = rng.random((n, n)) < 0.5
+    D[put] = rng.choice(special, put.sum())
+    both = np.triu(rng.random((n, n)) < 0.5)          # half of the pairs equal
+    D = np.where(both, D.T, D)
+    near = (rng.random((n, n)) < 0.6) if knn else np.ones((n, n), bool)
+    with np.errstate(all='ignore'):
+        off = ~np.eye(n, dtype=bool)
+        s = np.where(near & off & (D.T >= 1e-6), np.sqrt(D.T), 0.0)
+        Y = s * s + s.T * s.T - s * s.T
+        Y = np.where((Y != 0) | (near & (~off | (D.T < 1e-6))), Y, -1.0)
+    d = torch.from_numpy(D).cuda()
+    nb = torch.from_numpy(near.astype(np.uint8)).cuda() if knn else None
+    y = torch.empty((n, n), dtype=torch.float64, device='cuda')
+    _call(torch, 'mem_dm_symmetrise', d.data_ptr(), n, nb.data_ptr() if knn else None,
+          y.data_ptr())
+    np.testing.assert_allclose(y.cpu().numpy(), Y, rtol=1e-14, atol=0)
