@@ -13,13 +13,13 @@
 // CT columns through a buffer of up to 108 KB, two CTAs per SM.  Between rows and columns the
 // spectra go through the image's own output slot (in L2: 304 slots of 250 KB at 250 px, read back
 // right after they are written).  Keeping the rows of an image in the shared memories of a
-// cluster of two CTAs instead measured 1758 us for the low-pass of 1160 images of 250 px, against
+// cluster of two CTAs instead measured 1758 us for the low-pass of 1198 images of 250 px, against
 // 583 us for this form: the column passes' 8-byte accesses are slow over distributed shared memory.
 //
 // Against cuFFT (a row pass and a column pass over HBM for every transform, the gather and the
 // filter in passes of their own):
 //   1000 images of 192 px:  low-pass 217 us, was 465; spectrum 108, was 150; flip 103, was 153
-//   1160 images of 250 px:  low-pass 583 us, was 1240; spectrum 252, was 434; flip 289, was 451
+//   1198 images of 250 px:  low-pass 583 us, was 1240; spectrum 252, was 434; flip 289, was 451
 #pragma once
 
 #include "fft_mixed.cuh"
@@ -140,7 +140,7 @@ constexpr size_t whole_bytes() {
 // Threads and CTAs per SM: 128 x 5 while five buffers fit, 320 x 2 while two do (the load of one
 // image then overlaps the passes of another), else 384 threads alone; measured against 256 x 2,
 // 256 x 3, 512 x 1, 768 x 1 (low-pass of 1000 images: 120 px 97 us, 256 x 2 the same; 150 px 137,
-// 512 x 1 190; 192 px 217, 512 x 1 235; 800 of 100 px 53, 256 x 2 60)
+// 512 x 1 190; 192 px 217, 512 x 1 235; 846 of 100 px 53, 256 x 2 60)
 template <class Sh>
 constexpr int whole_blocks() {
     return whole_bytes<Sh>() <= 44 * 1024 ? 5 : whole_bytes<Sh>() <= 108 * 1024 ? 2 : 1;
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(NT, MINB) whole_inverse_kernel(InverseArgs a) 
 // on consecutive columns), pass 2 the buffer.  The columns 0 and N/2 of the row spectra are real;
 // between rows and columns a slot [N][H] keeps their real parts in one element.
 // Up to 42 pair-rows and columns at a time, fewer where two buffers of that would not fit an SM:
-// wide tiles keep the columns' global accesses long (1160 images of 250 px, low-pass / spectrum /
+// wide tiles keep the columns' global accesses long (1198 images of 250 px, low-pass / spectrum /
 // flip: 583 / 252 / 289 us; 25 at a time with 128 threads, three CTAs per SM: 707 / 289 / 360;
 // 16 with five CTAs: 578 / 291 / 346; 63 with one: 755 / 287 / 317).
 template <class Sh>

@@ -652,7 +652,7 @@ __device__ __forceinline__ float ctf_eval(int m, uint64_t qf, const CtfConst& cc
 // chain over the item's images in order, whichever kernel runs it (the results are the same bits).
 //
 // pd_sums_kernel: a thread owns the frequencies (ka, kb) and (N - ka, kb), which share |k|^2 and so
-// the CTF: its evaluation (half of a thread's instructions) serves both.  Issue-bound: 10.6 K
+// the CTF: its evaluation (half of a thread's instructions) serves both.  Issue-bound: 10.4 K
 // images of 128 px take 176 us, 219 us with one frequency per thread.
 template <int WHICH>
 __global__ void __launch_bounds__(128) pd_sums_kernel(
@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(256) pd_finalize_kernel(
 //     V_j(R) = C_j(m_R)^2 - mt(R): one column per ring, rings by decreasing |k|^2.  Phase 1
 //     keeps sw u' of every frequency in shared memory at its position in ring order, phase 2
 //     sums each ring's contiguous range.  C is evaluated once per ring, into shared memory, and
-//     a frequency's ring, weight and position come from one table word: 10.6 K images of 128 px
+//     a frequency's ring, weight and position come from one table word: 10.4 K images of 128 px
 //     took 748 us with an evaluation and two divisions per frequency, 488 so.
 template <int MODE, bool RINGS, int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) features_kernel(
@@ -1114,7 +1114,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) features_kernel(
 
 // 6b. the CTF of every image over the full plane (the reference's CTF array).  One evaluation
 // serves the four mirrored elements (+-fa, +-fb): with one per element the evaluations took
-// twice as long as the writes (in the features kernel, 268 of its 860 us for 10.6 K images of
+// twice as long as the writes (in the features kernel, 268 of its 860 us for 10.4 K images of
 // 128 px); a quarter of them leaves this kernel to the HBM writes (139 us, 5.0 TB/s).
 __global__ void __launch_bounds__(256) ctf_kernel(const uint64_t* __restrict__ qfix, int N,
                                                   CtfConst cc, float* __restrict__ ctf) {

@@ -20,7 +20,7 @@
 // axis 1 last, its results written to global memory (lanes on consecutive rows of the transposed
 // output): an image is read and written once, coalesced.  Bound by the latency of the
 // segments at a line's ends (their windows are mirrored or wrapped tap by tap, inner segments slide
-// theirs along the line): 800 images of 100 px take 98 us, 111 with mirrored taps everywhere and
+// theirs along the line): 846 images of 100 px take 98 us, 111 with mirrored taps everywhere and
 // two operations per anticausal step; 209 with a whole line per thread (serial chains of 3 N)
 // and the taps of every output in FP64.  512 threads: 98, a branch per output: 125.  Smaller boxes keep that form, whose start values are exact for
 // any length (relion_small_kernel).

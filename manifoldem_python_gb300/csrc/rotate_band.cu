@@ -22,7 +22,7 @@
 // Bound by issue slots, then shared-memory wavefronts (16 tap loads per sample, about two-way
 // conflicts; one 5x5 window for two samples, rot::sample_pair, has fewer loads but more
 // instructions and took 1016 us).  Three bands of 84 rows at 250 px, two CTAs of 512 threads per
-// SM.  1160 images of 250 px: 956 us; 1032 with the paired rows 16 apart (coordinates, column
+// SM.  1198 images of 250 px: 956 us; 1032 with the paired rows 16 apart (coordinates, column
 // counters and bounds of their own); 1453 with one CTA per image working through the bands of
 // both rotations, which was bound by its barriers (one CTA per SM, the column coefficients
 // through global scratch) and by the sampling loops' idle lanes.

@@ -178,7 +178,7 @@ __device__ __forceinline__ float2 shifted_w(const float2 w[4], int i, bool sa, b
 // row and column, wrapped by the caller's `at`) holds both 4x4 windows: 25 shared-memory loads for
 // two samples instead of 32.  A window's fifth row and column have weight 0, which leaves every
 // partial sum as it is, so the bits are those of two separate samples.  Shared-memory wavefronts
-// bound the rotations; both of 10,000 images of 128 px: 1344 us with two separate windows, 1127 with
+// bound the rotations; both of 10.4 K images of 128 px: 1344 us with two separate windows, 1127 with
 // 25 loads, 1102 with the fifth row and column loaded only where the windows differ.
 template <class At>
 __device__ __forceinline__ float2 sample_pair(int64_t XA, int64_t YA, int64_t XB, int64_t YB, int P,

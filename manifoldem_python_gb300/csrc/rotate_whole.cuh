@@ -12,7 +12,7 @@
 // Bound by shared-memory wavefronts, 25 tap loads per two samples with about two-way bank conflicts.
 //   1000 images of 192 px: 342 us (385 with 32 loads per two samples), 513 with the runtime-size
 //   kernel (serial 18-tap segment starts, one sample at a time, integer division in its loops);
-//   800 of 100 px: 74 us (88), was 135; 300 of 70 px: 18 us (20), was 31.
+//   846 of 100 px: 74 us (88), was 135; 300 of 70 px: 18 us (20), was 31.
 #pragma once
 
 #include "rotate_fixed.cuh"
