@@ -296,10 +296,11 @@ mem_contraction_config default_contraction() {
 // The default tile width of a plan's split-BF16 contraction.  A 128 x 128 tile is bound by the
 // shared-memory bytes of its operands (213 a clock wanted, 128 there), a 128 x 256 tile reads and
 // stages a quarter fewer of them per MMA, but pads small PDs more and takes 1.37 to 1.47 times as
-// long as a 128 x 128 tile; one tile runs per SM at a time, so that a launch takes whole waves of
-// tiles.  So the wide tile is taken where its waves, counted 1.5 fold, are fewer.  PDs of 1909 and
-// 3274 images of 128 px: 4 waves of narrow tiles 1096 us, 2 of wide ones 796; 24 PDs of 400: 2 and 2,
-// 551 and 759; 6 PDs of 1500 at 64 px: 4 and 3, 370 and 408.  The same bits in every schedule.
+// long as a 128 x 128 tile; one tile runs per SM at a time, so that a launch takes waves of tiles,
+// the last one cut (tc_waves).  So the wide tile is taken where its waves, counted 1.45 fold, are
+// fewer.  PDs of 1909 and 3274 images of 128 px: 3.5 waves of narrow tiles, 1.67 of wide ones,
+// 658 us (792 with two whole waves, 1096 with four of narrow tiles); 24 PDs of 400: 1.67 and 1.5,
+// narrow, 469 us (551 with two whole waves; wide 759).  The same bits in every schedule.
 static int32_t default_tile_width(const mem_plan& P, const mem_contraction_config& dc) {
     if (dc.accumulators != 2 || P.tc_kahan) return dc.tile_n;
     int64_t narrow = 0, wide = 0;
@@ -309,8 +310,7 @@ static int32_t default_tile_width(const mem_plan& P, const mem_contraction_confi
         for (int64_t I = 0; I < nb; ++I) wide += nj - I / 2;
     }
     const int64_t sms = std::max(P.num_sms, 1);
-    const int64_t wn = (narrow + sms - 1) / sms, ww = (wide + sms - 1) / sms;
-    return 3 * ww < 2 * wn ? 256 : 128;
+    return 1.45 * tc_waves(wide, sms) < tc_waves(narrow, sms) ? 256 : 128;
 }
 
 int apply_contraction(mem_plan* P, int n_classes, const mem_contraction_config* classes) {
@@ -552,9 +552,13 @@ int mem_plan_create(const mem_params* params, int32_t n_pd, const int32_t* pd_co
     P->tc_part_units = (p.precision == MEM_PREC_FP32 || p.avg_only)
                            ? 0
                            : tc_split_units((int64_t)P->tiles.size(), P->n_chunks, 1024);
+    // or the running sums of up to one 128 x 256 tile per SM (20 MB) for those of a partial wave
+    if (p.precision != MEM_PREC_FP32 && !p.avg_only && (int64_t)P->tiles.size() > P->num_sms)
+        P->tc_carry = P->num_sms;
     L.tc_part = take(P->tc_part_units
                          ? (size_t)(P->tc_part_units + (int64_t)P->tiles.size()) * kTcUnitBytes
-                         : 0);
+                     : P->tc_carry ? kTcFlagBytes + (size_t)P->tc_carry * 2 * kTcUnitBytes
+                                   : 0);
     L.total = off;
     *out_plan = P;
     return MEM_OK;

@@ -72,19 +72,53 @@ struct TcShared {
     int abort_flag;
 };
 
+// Where tile x of the `rest` tiles of the last wave of S CTAs is cut (chunks of its head).  Tile x's
+// head goes to CTA x and its tail to CTA x + d, d = S - rest.  So the CTAs x, x + d, x + 2d, ..
+// form a chain, m tiles on m + 1 CTAs: the k-th tile's head takes (m - k) / (m + 1) of its chunks, and
+// every CTA of the chain gets m / (m + 1) of a tile beside its whole ones.
+__host__ __device__ inline int tc_cut_of(int x, int rest, int S, int nchunks) {
+    const int d = S - rest, k = x / d, m = (rest - x % d + d - 1) / d;
+    return (int)((int64_t)nchunks * (m - k) / (m + 1));
+}
+
+// bounded wait for a flag that another CTA sets; as mbar_wait
+__device__ __forceinline__ bool flag_wait(const unsigned* flag, volatile int* abort_flag,
+                                          uint32_t* status, long long limit) {
+    const long long t0 = clock64();
+    for (;;) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+        if (v) return true;
+        if (*abort_flag) return false;
+        if (clock64() - t0 > limit) {
+            *abort_flag = 1;
+            atomicOr(status, kStatusTimeout);
+            return false;
+        }
+    }
+}
+
 // The contraction over the tiles [tile_begin, tile_begin + tile_count) of the plan's tile list:
 // CTA b takes tiles tile_begin + b + k gridDim.x (a persistent CTA when the grid is smaller
 // than the tile count; one tile per CTA when it is as large).  The producer, the MMA issuer and
 // the epilogue each walk the CTA's tiles in the same order; the stage ring and the NBUF TMEM
 // accumulators (NBUF x 128 columns) continue from one tile to the next, so a tile's first
 // groups are loaded and multiplied while the epilogue still adds and stores the previous tile.
-template <bool KAHAN, bool LOLO, int NBUF, int BN>
+//
+// SPLIT: as many CTAs as SMs (T tiles on S of them, S < T, launched together): each CTA computes
+// T / S whole tiles, and every tile of the last, partial wave is cut in two at a chunk: one CTA
+// computes its first chunks before its whole tiles and leaves the running sums in `carry`, another
+// continues from them after its own, so that the sums are the same, chunk by chunk.  See
+// tc_cut_of for the cuts.  A continuing warp waits (bounded) for the flag of the warp it follows,
+// which was set about a tile's time before.
+template <bool KAHAN, bool LOLO, int NBUF, int BN, bool SPLIT>
 __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
         const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
         const double* __restrict__ pair_norm, const uint32_t* __restrict__ scale_bits,
         const Tile* __restrict__ tiles, const PdDev* __restrict__ pds, double* __restrict__ D,
         uint32_t* __restrict__ status, const int4* __restrict__ chunks, int nchunks,
-        int group_chunks, long long wait_limit, int withhold, int tile_begin, int tile_count) {
+        int group_chunks, long long wait_limit, int withhold, int tile_begin, int tile_count,
+        float* __restrict__ carry, unsigned* __restrict__ carry_flags) {
     static_assert(NBUF == 2 || NBUF == 4, "two or four TMEM accumulators");
     static_assert(BN == 128 || BN == 256, "tile widths");
     static_assert(NBUF * BN <= 512, "TMEM holds 512 columns");
@@ -99,10 +133,31 @@ __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
     TcShared* sh = (TcShared*)(smem + TC_STAGES * TC_STAGE_BYTES);
     volatile int* abort_flag = &sh->abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int my_tiles = (int)blockIdx.x < tile_count
-                             ? (tile_count - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x
-                             : 0;
-    auto tile_of = [&](int lt) { return tiles[tile_begin + (int)blockIdx.x + lt * (int)gridDim.x]; };
+    // SPLIT: this CTA's parts are [head of tile blockIdx.x], whole tiles, [tail of tile tail]
+    const int rest = SPLIT ? tile_count % (int)gridDim.x : 0;
+    const int tail = SPLIT ? (int)blockIdx.x - ((int)gridDim.x - rest) : -1;
+    const int heads = SPLIT && (int)blockIdx.x < rest ? 1 : 0;
+    const int whole = SPLIT ? tile_count / (int)gridDim.x
+                      : (int)blockIdx.x < tile_count
+                          ? (tile_count - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x
+                          : 0;
+    const int my_tiles = heads + whole + (tail >= 0 ? 1 : 0);
+    struct Part {
+        Tile t;
+        int c0, c1;                                // its chunks
+    };
+    auto part_of = [&](int lt) {
+        Part p;
+        const int k = lt - heads;
+        const int i = !SPLIT           ? (int)blockIdx.x + lt * (int)gridDim.x
+                      : k < 0          ? (int)blockIdx.x
+                      : k < whole      ? rest + (int)blockIdx.x + k * (int)gridDim.x
+                                       : tail;
+        p.t = tiles[tile_begin + i];
+        p.c0 = SPLIT && k == whole ? tc_cut_of(tail, rest, (int)gridDim.x, nchunks) : 0;
+        p.c1 = SPLIT && k < 0 ? tc_cut_of(i, rest, (int)gridDim.x, nchunks) : nchunks;
+        return p;
+    };
     const int gsize = (group_chunks > 0 && group_chunks < nchunks) ? group_chunks : nchunks;
     const int ngroups = (nchunks + gsize - 1) / gsize;
 
@@ -139,11 +194,12 @@ __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
             long long gc = 0, withheld = -1;     // chunks issued by this CTA (all its tiles)
             bool stop = false;
             for (int lt = 0; lt < my_tiles && !stop; ++lt) {
-                const Tile t = tile_of(lt);
+                const Part part = part_of(lt);
+                const Tile t = part.t;
                 const PdDev pd = pds[t.pd];
                 const int rowA = (int)(pd.row_off + (int64_t)t.I * TC_M);
                 const int rowB = (int)(pd.row_off + (int64_t)t.J * BN);
-                for (int c = 0; c < nchunks; ++c, ++gc) {
+                for (int c = part.c0; c < part.c1; ++c, ++gc) {
                     const int st = (int)(gc % TC_STAGES);
                     const uint32_t ph = (uint32_t)(gc / TC_STAGES) & 1u;
                     if (gc >= TC_STAGES &&
@@ -186,8 +242,9 @@ __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
             bool issued_any = false, stop = false;
             long long gc = 0, gg = 0;            // chunks and accumulation groups of this CTA
             for (int lt = 0; lt < my_tiles && !stop; ++lt) {
-                int4 ch_next = chunks[0];        // schedule entry, read one chunk ahead
-                for (int c = 0; c < nchunks; ++c, ++gc) {
+                const Part part = part_of(lt);
+                int4 ch_next = chunks[part.c0];  // schedule entry, read one chunk ahead
+                for (int c = part.c0; c < part.c1; ++c, ++gc) {
                     const int4 ch = ch_next;
                     if (c + 1 < nchunks) ch_next = chunks[c + 1];
                     const int st = (int)(gc % TC_STAGES);
@@ -251,13 +308,25 @@ __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
         bool ok = true;
         long long gg = 0;
         for (int lt = 0; lt < my_tiles && ok; ++lt) {
-            const Tile t = tile_of(lt);
+            const Part part = part_of(lt);
+            const Tile t = part.t;
             float acc[EC], cmp[KAHAN ? EC : 1];
+            const int groups = SPLIT ? part.c1 - part.c0 : ngroups;      // SPLIT: gsize is 1
+            if (SPLIT && part.c0 > 0) {            // from the sums that the tile's head left
+                const int64_t at = (int64_t)tail * EPI + warp;
+                ok = flag_wait(carry_flags + at, abort_flag, status, wait_limit);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                const float* from = carry + at * (EC * 32) + lane;
 #pragma unroll
-            for (int j = 0; j < EC; ++j) acc[j] = 0.f;
+                for (int j = 0; j < EC; ++j) acc[j] = __ldcg(from + 32 * j);
+            } else {
+#pragma unroll
+                for (int j = 0; j < EC; ++j) acc[j] = 0.f;
+            }
 #pragma unroll
             for (int j = 0; j < (KAHAN ? EC : 1); ++j) cmp[j] = 0.f;
-            for (int g = 0; g < ngroups; ++g, ++gg) {
+            for (int g = 0; g < groups; ++g, ++gg) {
                 const int b = (int)(gg % NBUF);
                 const long long use = gg / NBUF;
                 ok = mbar_wait(&sh->acc_full[b], (uint32_t)(use & 1), abort_flag, status,
@@ -299,6 +368,19 @@ __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
                 if (lane == 0) mbar_arrive(&sh->acc_empty[b]);
             }
             if (!ok || *abort_flag) break;
+            if (SPLIT && part.c1 < nchunks) {      // a head: leave the sums, then the flag
+                const int64_t at = (int64_t)blockIdx.x * EPI + warp;
+                float* to = carry + at * (EC * 32) + lane;
+#pragma unroll
+                for (int j = 0; j < EC; ++j) __stcg(to + 32 * j, acc[j]);
+                __threadfence();
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(carry_flags + at),
+                                 "r"(1u)
+                                 : "memory");
+                continue;
+            }
             const PdDev pd = pds[t.pd];
             const double sc = (double)feature_scale_from_bits(scale_bits[t.pd]);
             const double inv_sc2 = 1.0 / (sc * sc);
@@ -778,6 +860,21 @@ int64_t tc_split_units(int64_t tiles, int64_t chunks, int64_t most) {
     return per_round * tiles;
 }
 
+// Whether the last wave's tiles of a launch of `tiles` on `sms` SMs are cut in two (gemm_tc_kernel,
+// SPLIT): one to four whole waves before them, beyond which the wave is a small part (and
+// without one a tail would wait for its head).  24 PDs of 400 images of 128 px (250 tiles): 551 us
+// whole, 469 cut; of 64 px 179 and 155; 6 PDs of 1500 at 64 px (347 wide tiles): 408 and 330.
+bool tc_cut_pays(int64_t tiles, int64_t sms) {
+    return tiles > sms && tiles < 5 * sms && tiles % sms != 0 && sms <= kTcFlagBytes / 64;
+}
+
+// waves of `tiles` tiles on `sms` SMs, a cut wave as the longest of its chains (tc_cut_of)
+double tc_waves(int64_t tiles, int64_t sms) {
+    if (!tc_cut_pays(tiles, sms)) return (double)((tiles + sms - 1) / sms);
+    const int64_t rest = tiles % sms, d = sms - rest, m = (rest + d - 1) / d;
+    return (double)(tiles / sms) + (double)m / (double)(m + 1);
+}
+
 namespace kern {
 int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
                     const double* pair_norm, const uint32_t* scale_bits, const Tile* tiles,
@@ -816,6 +913,39 @@ int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
         return MEM_OK;
     }
     const int sms = P.num_sms > 0 ? P.num_sms : 1;
+    // the default schedule where the last wave is partial: its tiles cut in two
+    if (P.tc_carry >= sms && P.tc_ranges.size() == 1 && !c0.persistent && c0.accumulators == 2 &&
+        c0.tile_m == 128 && P.tc_group_chunks == 1 && !P.tc_kahan && P.test_withhold_chunk < 0 &&
+        tc_cut_pays(T, sms)) {
+        const int rest = T % sms;
+        auto kfn = c0.tile_n == 256
+                       ? (P.tc_lolo ? gemm_tc_kernel<false, true, 2, 256, true>
+                                    : gemm_tc_kernel<false, false, 2, 256, true>)
+                       : (P.tc_lolo ? gemm_tc_kernel<false, true, 2, 128, true>
+                                    : gemm_tc_kernel<false, false, 2, 128, true>);
+        const size_t smem = c0.tile_n == 256 ? TcShape<256>::SMEM : TcShape<128>::SMEM;
+        const int threads = c0.tile_n == 256 ? TcShape<256>::THREADS : TcShape<128>::THREADS;
+        unsigned* flags = reinterpret_cast<unsigned*>(part);
+        float* carry = part + kTcFlagBytes / sizeof(float);
+        MEM_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem));
+        MEM_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(unsigned) * 16 * rest, s));
+        cudaLaunchAttribute coop{};
+        coop.id = cudaLaunchAttributeCooperative;      // CTAs wait on one another
+        coop.val.cooperative = 1;
+        cudaLaunchConfig_t lc{};
+        lc.gridDim = dim3((unsigned)sms);
+        lc.blockDim = dim3((unsigned)threads);
+        lc.dynamicSmemBytes = smem;
+        lc.stream = s;
+        lc.attrs = &coop;
+        lc.numAttrs = 1;
+        MEM_CUDA_TRY(cudaLaunchKernelEx(&lc, kfn, mhi, mlo, pair_norm, scale_bits, tiles, pds, D,
+                                        status, chunks, P.n_chunks, P.tc_group_chunks,
+                                        P.wait_cycles, P.test_withhold_chunk, 0, T, carry, flags));
+        MEM_LAUNCH_CHECK();
+        return MEM_OK;
+    }
     CUtensorMap bhi, blo;                // 64-row boxes: the CTA pairs' halves of B
     bool have_b64 = false;
     // one launch per size class of the plan's contraction configuration (tiles sorted by class)
@@ -855,13 +985,14 @@ int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
         const unsigned grid = cfg.persistent ? (unsigned)std::min(count, sms) : (unsigned)count;
 #define MEM_TC_LAUNCH(KAHAN, LOLO, NB, BN)                                                     \
     do {                                                                                       \
-        MEM_CUDA_TRY(cudaFuncSetAttribute(gemm_tc_kernel<KAHAN, LOLO, NB, BN>,                 \
+        MEM_CUDA_TRY(cudaFuncSetAttribute(gemm_tc_kernel<KAHAN, LOLO, NB, BN, false>,          \
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,         \
                                           (int)TcShape<BN>::SMEM));                            \
-        gemm_tc_kernel<KAHAN, LOLO, NB, BN><<<grid, TcShape<BN>::THREADS, TcShape<BN>::SMEM,   \
-                                              s>>>(                                            \
-            mhi, mlo, pair_norm, scale_bits, tiles, pds, D, status, chunks, P.n_chunks,        \
-            P.tc_group_chunks, P.wait_cycles, P.test_withhold_chunk, begin, count);            \
+        gemm_tc_kernel<KAHAN, LOLO, NB, BN, false>                                             \
+            <<<grid, TcShape<BN>::THREADS, TcShape<BN>::SMEM, s>>>(                            \
+                mhi, mlo, pair_norm, scale_bits, tiles, pds, D, status, chunks, P.n_chunks,    \
+                P.tc_group_chunks, P.wait_cycles, P.test_withhold_chunk, begin, count,         \
+                nullptr, nullptr);                                                             \
     } while (0)
 #define MEM_TC_SHAPE(KAHAN, LOLO)                                                              \
     do {                                                                                       \

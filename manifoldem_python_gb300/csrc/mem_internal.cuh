@@ -125,6 +125,7 @@ struct mem_plan {
     std::vector<mem::Tile> tc_tiles;   // the split-BF16 contraction's tiles (J in tile_n units)
     bool uploaded = false;
     int64_t tc_part_units = 0;      // scratch of the chunk-split contraction
+    int tc_carry = 0;               // SMs that scratch for cut tiles was laid out for, else 0
     int tc_group_chunks = 1;        // 64-wide K chunks per TMEM accumulation group (0 = all)
     bool tc_kahan = false;          // compensated register sums across groups
     bool tc_lolo = false;           // add the lo.lo product (4-term split)
@@ -276,6 +277,11 @@ std::vector<int32_t> radius_descending_columns(int N, int64_t Kc, int64_t Kc_pad
 // default contraction schedule: one class, one CTA per 128 x 128 tile, two TMEM accumulators
 // (MEM_TC_PERSISTENT / MEM_TC_BUFS / MEM_TC_TILE_N override it, for tuning)
 mem_contraction_config default_contraction();
+
+// the cut tiles of a partial last wave (gemm_tc.cu): flags of their warps, then running sums
+constexpr size_t kTcFlagBytes = 16384;
+bool tc_cut_pays(int64_t tiles, int64_t sms);
+double tc_waves(int64_t tiles, int64_t sms);
 
 // orders the plan's tiles by size class and sets tc_classes / tc_ranges
 int apply_contraction(mem_plan* P, int n_classes, const mem_contraction_config* classes);

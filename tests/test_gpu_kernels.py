@@ -397,8 +397,13 @@ def test_default_tile_width(cuda_ready, counts, width):
     def tiles(cols):
         return sum(sum(-(-n // cols) - 128 * i // cols for i in range(-(-n // 128)))
                    for n in counts)
-    waves = [-(-tiles(c) // 152) for c in (128, 256)]
-    assert (256 if 3 * waves[1] < 2 * waves[0] else 128) == width
+    def waves(t):                                  # a partial wave's tiles are cut in two
+        full, rest = divmod(t, 152)
+        if not rest or not 1 <= full < 5:
+            return -(-t // 152)
+        m = -(-rest // (152 - rest))
+        return full + m / (m + 1)
+    assert (256 if 1.45 * waves(tiles(256)) < waves(tiles(128)) else 128) == width
     N, n = 32, sum(counts)
     rng = np.random.default_rng(n)
     stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
@@ -417,6 +422,49 @@ def test_default_tile_width(cuda_ready, counts, width):
         torch.cuda.synchronize()
         D.append(out['D'].clone())
     assert torch.equal(D[0], D[1]) and bool(torch.isfinite(D[0]).all())
+
+
+@pytest.mark.parametrize('tile_n', [128, 256])
+@pytest.mark.parametrize('rest', [1, 76, 98, 120, 151])
+def test_cut_tiles_of_a_partial_wave(cuda_ready, tile_n, rest):
+    """T tiles on S SMs, S < T < 2 S: the rest of T is cut in two (chains of 1, 2, .. tiles) and gives
+    the same D, bit for bit, as persistent CTAs with whole tiles, execute after execute."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    N, big = 32, 2000
+    big_tiles = {128: 136, 256: 72}[tile_n]
+    counts = [big] + [3] * (sms + rest - big_tiles)
+    n = sum(counts)
+    rng = np.random.default_rng(rest)
+    stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
+    idx = torch.arange(n, device='cuda')
+    flip = torch.zeros(n, dtype=torch.uint8, device='cuda')
+    psi = torch.from_numpy(rng.uniform(-3, 3, n)).cuda()
+    df = torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda()
+    params = StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1,
+                         precision='bf16x3')
+    D = []
+    for persistent in (1, 0):
+        plan = Plan(params, counts, [0.3] * len(counts),
+                    contraction=[dict(max_n=2 ** 31 - 1, persistent=persistent, accumulators=2,
+                                      tile_n=tile_n)])
+        out = plan.allocate_outputs(('D',))
+        for _ in range(2):
+            out['D'].fill_(float('nan'))
+            plan.execute(stack, idx, flip, psi, df, out)
+            torch.cuda.synchronize()
+            plan.device_status()
+            D.append(out['D'].clone())
+    graph = plan.capture(stack, idx, flip, psi, df, out)
+    for _ in range(2):
+        out['D'].fill_(float('nan'))
+        graph.replay()
+        torch.cuda.synchronize()
+        plan.device_status()
+        D.append(out['D'].clone())
+    assert bool(torch.isfinite(D[0]).all())
+    assert all(torch.equal(D[0], d) for d in D[1:])
 
 
 @pytest.mark.parametrize('N,relion', [(32, False), (36, True)])
