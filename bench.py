@@ -438,7 +438,8 @@ def shared_memory_roofline(r, args, phase):
     (the rotation): wavefronts per image from the committed ncu summary of the kernel x the
     images / the phase's live time, against one wavefront per SM per clock at the SM clock
     sampled during the timed region."""
-    per_img = profile_number(phase, args.config, 'shared_wavefronts_per_image')
+    # the current kernels' figure; 'shared_wavefronts_per_image' is that of the builds before them
+    per_img = profile_number(phase, args.config, 'rotation_wavefronts_per_image')
     mhz = (r.get('clocks') or {}).get('sm_mhz')
     if not per_img or not mhz:
         return None

@@ -15,7 +15,7 @@ adjacent classes that chose the same schedule are merged into one launch.
 
 Results are cached in a JSON file keyed by GPU name, box size and contraction form
 (``MEM_AUTOTUNE_CACHE`` names the file; default ``autotune_cache.json`` beside this module);
-``pipeline.Plan`` applies a cached table when it creates a plan.  The reference has no
+``pipeline.Plan`` applies a cached table when it creates a plan of at least five waves of tiles.  The reference has no
 counterpart: its D is one float64 GEMM per PD on the CPU
 (modules/getDistanceCTF_local_Conj9combinedS2.py:391-397).
 """
@@ -77,6 +77,16 @@ def lookup(gpu_name: str, N: int, precision: str) -> Optional[List[dict]]:
     with _lock:
         ent = _read_cache().get(cache_key(gpu_name, N, precision))
     return None if ent is None else ent['classes']
+
+
+def applies(counts: Sequence[int], sms: int) -> bool:
+    """Whether a plan of PDs of ``counts`` images takes a measured table: from five waves of 128 x 128
+    tiles on.  The tables are measured on about eight waves; with fewer the library's own rules
+    (chunks spread over the SMs, cut tiles, the width by waves) are the faster: at 128 px one PD of
+    2000, 136 tiles, 287 us by them and 399 with the table's wide tiles; one of 300 images of 70 px
+    23 us and 145."""
+    nb = -(-np.asarray(counts, dtype=np.int64) // 128)
+    return int((nb * (nb + 1) // 2).sum()) >= 5 * sms
 
 
 def to_c(classes: Sequence[dict]):

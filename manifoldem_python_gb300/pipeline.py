@@ -69,7 +69,8 @@ class Plan:
                  device=None, contraction=None):
         """``contraction``: the split-BF16 contraction's schedule per size class (a list of
         dicts max_n / persistent / accumulators, see ``autotune``); default: the autotuner's
-        cached table for this GPU and box size if there is one, else the library's default."""
+        cached table for this GPU and box size if there is one and the plan has the tiles that
+        it was measured for (``autotune.applies``), else the library's default."""
         import torch
         self.lib = _lib.load()
         self.params = params
@@ -86,8 +87,9 @@ class Plan:
         self.handle = h
         if contraction is None and params.precision == 'bf16x3':
             from . import autotune
-            contraction = autotune.lookup(torch.cuda.get_device_name(self.device), params.N,
-                                          params.precision)
+            props = torch.cuda.get_device_properties(self.device)
+            if autotune.applies(self.counts, props.multi_processor_count):
+                contraction = autotune.lookup(props.name, params.N, params.precision)
         self.contraction = contraction
         if contraction:
             from . import autotune

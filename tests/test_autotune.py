@@ -26,3 +26,10 @@ def test_adjacent_equal_classes_merge_into_one_launch():
     arr = A.to_c(out)
     assert [arr[i].max_n for i in range(3)] == [192, 1536, big]
     assert arr[1].tile_n == 256 and arr[2].persistent == 1 and arr[0].tile_m == 128
+
+
+def test_table_applies_from_five_waves():
+    from manifoldem_python_gb300 import autotune
+    assert not autotune.applies([300], 152) and not autotune.applies([2000], 152)
+    assert not autotune.applies([128] * 759, 152) and autotune.applies([128] * 760, 152)
+    assert autotune.applies([4900], 152) and not autotune.applies([], 152)
