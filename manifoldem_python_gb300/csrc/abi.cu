@@ -887,7 +887,8 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
         else
             MEM_STEP(kern::gemm_split_bf16(P, feat_a, feat_b, pair_norm, scale_bits,
                                            at<Tile>(ws, L.tc_tiles), pds, ft.chunks, out->D,
-                                           status, at<float>(ws, L.tc_part), P.tc_part_units, s));
+                                           status, at<float>(ws, L.tc_part), P.tc_part_units, !split,
+                                           s));
     }
     MEM_STEP(mark(9));
 #undef MEM_STEP

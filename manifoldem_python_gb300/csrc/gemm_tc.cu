@@ -879,7 +879,7 @@ namespace kern {
 int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
                     const double* pair_norm, const uint32_t* scale_bits, const Tile* tiles,
                     const PdDev* pds, const int4* chunks, double* D, uint32_t* status,
-                    float* part, int64_t part_units, cudaStream_t s) {
+                    float* part, int64_t part_units, bool cut, cudaStream_t s) {
     if (P.tiles.empty() || !D) return MEM_OK;
     // every chunk starts on a 64-column boundary: TMA x offsets are multiples of 8 bf16
     if (P.Kf % TC_BK != 0 || P.n_rows % TC_M != 0 || (int64_t)P.n_chunks * TC_BK != P.Kf)
@@ -913,8 +913,9 @@ int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
         return MEM_OK;
     }
     const int sms = P.num_sms > 0 ? P.num_sms : 1;
-    // the default schedule where the last wave is partial: its tiles cut in two
-    if (P.tc_carry >= sms && P.tc_ranges.size() == 1 && !c0.persistent && c0.accumulators == 2 &&
+    // the default schedule where the last wave is partial: its tiles cut in two (a cooperative launch
+    // waits for all SMs, so not beside the load stream of a split execute)
+    if (cut && P.tc_carry >= sms && P.tc_ranges.size() == 1 && !c0.persistent && c0.accumulators == 2 &&
         c0.tile_m == 128 && P.tc_group_chunks == 1 && !P.tc_kahan && P.test_withhold_chunk < 0 &&
         tc_cut_pays(T, sms)) {
         const int rest = T % sms;

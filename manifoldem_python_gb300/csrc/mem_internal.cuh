@@ -264,7 +264,7 @@ int gemm_fp32(const mem_plan& P, const float* feat, const double* pair_norm,
 int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
                     const double* pair_norm, const uint32_t* scale_bits, const Tile* tiles,
                     const PdDev* pds, const int4* chunks, double* D, uint32_t* status,
-                    float* part, int64_t part_units, cudaStream_t s);
+                    float* part, int64_t part_units, bool cut, cudaStream_t s);
 }  // namespace kern
 
 // scratch of the split-BF16 contraction of few tiles (gemm_tc.cu): units of 64 KB to use, of at most

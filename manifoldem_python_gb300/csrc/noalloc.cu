@@ -296,7 +296,7 @@ extern "C" int mem_pd_distances_noalloc(const mem_params* params, int32_t n, con
         NA_STEP(kern::gemm_split_bf16(P, at<char>(ws, L.feat_a), at<char>(ws, L.feat_b),
                                       pair_norm, scale_bits, at<Tile>(ws, L.tiles), pds,
                                       ft.chunks, D, at<uint32_t>(ws, L.status),
-                                      at<float>(ws, used), units, s));
+                                      at<float>(ws, used), units, false, s));
     }
 #undef NA_STEP
     return MEM_OK;
