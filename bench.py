@@ -386,16 +386,16 @@ def workload_string(config_name, cfg, counts):
 
 def kernels_per_execute(outputs, avg_only, N, counts=None, classes=None):
     """Kernels of this library one mem_plan_execute launches (cuFFT kernels excluded).
-    N = 32, 64, 128 (shared-memory FFTs): lowpass_fft, rot_const, rotate, spectrum_fft, qfix,
-    pd_sums, pd_finalize, features, [ctf], [inverse_fft + avg_store], [inverse_fft + intensity],
+    N = 32, 64, 128 (shared-memory FFTs): lowpass_fft, rot_const, rotate, spectrum_fft, pd_sums,
+    pd_finalize, features, [ctf], [inverse_fft + avg_store], [inverse_fft + intensity],
     [contraction: one launch per size class that has PDs].  Other N, at least (cuFFT transforms;
     the mixed-radix sizes launch two inverse transforms more): gather_normalize, lowpass_apply,
-    rot_const, rotate, qfix, pd_sums, pd_finalize, features, [ctf], [avg_store], [intensity],
+    rot_const, rotate, pd_sums, pd_finalize, features, [ctf], [avg_store], [intensity],
     [contraction]."""
     smem = N in (32, 64, 128) and os.environ.get('MEM_SMEM_FFT', '1') != '0'
     # N = 64, 128: lowpass_fft, rotate and spectrum_fft are one image_stage kernel
     fused = smem and N in (64, 128) and os.environ.get('MEM_FUSED_IMAGE', '0') == '1'
-    k = 6 if fused else 8
+    k = 6 if fused else 7                  # the fused path launches qfix by itself
     if 'ctf' in outputs:
         k += 1
     if 'img_avg' in outputs or 'img_avg_flip' in outputs:

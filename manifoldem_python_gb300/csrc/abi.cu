@@ -767,7 +767,7 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
         // F = fft2(imgAll) in one kernel per image; the lowpass phase holds all of it, the
         // rotate and spectrum phases are empty
         MEM_STEP(mark(1));
-        MEM_STEP(kern::rot_consts(P, *in, pds, img_pd, at<char>(ws, L.rotc), cs));
+        MEM_STEP(kern::rot_consts(P, *in, pds, img_pd, at<char>(ws, L.rotc), nullptr, cs));
         MEM_STEP(kern::image_stage(P, lin, at<float>(ws, L.gtab), at<float2>(ws, L.twid), xbuf,
                                    img_all, at<char>(ws, L.rotc), fspec, status, cs));
     } else if (P.smem_fft) {
@@ -790,7 +790,8 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     MEM_STEP(mark(2));
     // (a4, a6) mask and the two rotations -> imgAll
     if (!fused)
-        MEM_STEP(kern::rotate(P, *in, xbuf, img_all, pds, img_pd, spec, at<char>(ws, L.rotc), s));
+        MEM_STEP(kern::rotate(P, *in, xbuf, img_all, pds, img_pd, spec, at<char>(ws, L.rotc), qf,
+                              s));
     MEM_STEP(mark(3));
     // (a8) F = fft2(imgAll); (a7, a9) CTF and per-PD sums.  With a volume mask the spectra of
     // D, of the phase flips and of imgAvgFlip are those of imgAll * msk2 (:344), while the Wiener
@@ -806,7 +807,7 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     // (a volume mask's first spectra, those of imgAll itself, serve the Wiener average only)
     if (!fused && (!in->pd_mask || out->img_avg)) MEM_STEP(spectrum(img_all, nullptr));
     MEM_STEP(mark(4));
-    MEM_STEP(kern::qfix(P, *in, qf, s));
+    if (fused) MEM_STEP(kern::qfix(P, *in, qf, s));     // else with the rotation constants
     float* partial = at<float>(ws, L.partial);
     float* means = at<float>(ws, L.means);
     float2* avg_spec = at<float2>(ws, L.avg_spec);

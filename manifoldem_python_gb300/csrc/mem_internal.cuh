@@ -216,19 +216,20 @@ int spectrum_fft(const mem_plan& P, int64_t count, const float* images, const ui
 // signed = the phase-flip inverse: element k of image i multiplied by sign(C_i(k)) / N^2 on load
 int inverse_fft(const mem_plan& P, int64_t count, const float2* spec, const float2* twid,
                 float* images, const uint64_t* qf, bool signed_flip, cudaStream_t s);
-// the two rotations' fixed-point constants of every image into rot_scratch (64 bytes each)
+// the two rotations' fixed-point constants of every image into rot_scratch (64 bytes each); with qf
+// also the defocus phases (as qfix does)
 int rot_consts(const mem_plan& P, const mem_inputs& in, const PdDev* pd_table,
-               const int32_t* img_pd, void* rot_scratch, cudaStream_t s);
+               const int32_t* img_pd, void* rot_scratch, uint64_t* qf, cudaStream_t s);
 // N = 64, 128: gather + flip + normalisation + low-pass, mask + both rotations and the spectrum
 // of imgAll in one kernel (rot_consts first); img_out receives imgAll, spec the spectra
 bool image_stage_supported(const mem_plan& P);
 int image_stage(const mem_plan& P, const mem_inputs& in, const float* gtab, const float2* twid,
                 float* xbuf, float* img_out, const void* rotc, float2* spec, uint32_t* status,
                 cudaStream_t s);
-// rot_scratch: 64 bytes per image (the two rotations' fixed-point constants)
+// rot_scratch: 64 bytes per image (the two rotations' fixed-point constants); qf: see rot_consts
 int rotate(const mem_plan& P, const mem_inputs& in, float* xbuf, float* img_out,
            const PdDev* pd_table, const int32_t* img_pd, float2* spec, void* rot_scratch,
-           cudaStream_t s);
+           uint64_t* qf, cudaStream_t s);
 // the two rotations with the coefficient image in bands of rows (64 <= N <= 512); spec holds the
 // first one's results
 bool rotate_band_supported(int N);

@@ -323,9 +323,19 @@ __global__ void lowpass_apply_kernel(float2* __restrict__ spec, const float* __r
 // then by the PD's -psi_p (its cosine and sine are in the PD table).  Computed once per image so
 // that the rotation kernels read them instead of one thread per CTA evaluating FP64
 // trigonometry while the CTA waits (FP64 is slow on this part).
+// With qfix, also the image's defocus phase (one launch for what depends on an image alone).  One
+// warp per CTA: FP64 (2 FMA per clock and SM) bounds it, so that 300 images are spread over ten SMs
+// rather than two: 4.7 us, 6.2 with 256 threads and 1.8 for the phases in a launch of their own.
+__device__ __forceinline__ uint64_t phase_fix(double df, double q_scale) {
+    const double q = q_scale * df;
+    const double v = ldexp(q - floor(q), 64);
+    return (v >= 18446744073709551615.0) ? 0ull : __double2ull_rn(v);
+}
+
 __global__ void rot_const_kernel(const double* __restrict__ psi_rad, const PdDev* __restrict__ pds,
                                  const int32_t* __restrict__ img_pd, RotConst* __restrict__ out,
-                                 int64_t n, int N) {
+                                 int64_t n, int N, const double* __restrict__ df,
+                                 uint64_t* __restrict__ qfix, double q_scale) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double ang = -(180.0 / 3.141592653589793) * psi_rad[i];
@@ -333,6 +343,7 @@ __global__ void rot_const_kernel(const double* __restrict__ psi_rad, const PdDev
     out[2 * i] = make_rot(cos(t), sin(t), N);
     const PdDev& pd = pds[img_pd[i]];
     out[2 * i + 1] = make_rot(pd.rot2_cos, pd.rot2_sin, N);
+    if (qfix) qfix[i] = phase_fix(df[i], q_scale);
 }
 
 // one axis of the periodic prefilter over an N x N image in smem (row stride P).
@@ -602,11 +613,7 @@ __global__ void __launch_bounds__(NT) rotate_global_kernel(
 __global__ void qfix_kernel(const double* __restrict__ df, uint64_t* __restrict__ qfix,
                             int64_t n, double q_scale) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double q = q_scale * df[i];
-    double fr = q - floor(q);
-    double v = ldexp(fr, 64);
-    qfix[i] = (v >= 18446744073709551615.0) ? 0ull : __double2ull_rn(v);
+    if (i < n) qfix[i] = phase_fix(df[i], q_scale);
 }
 
 // sin(2 pi u / 2^64) of a phase u in 64-bit fixed-point cycles.  The top three bits give the
@@ -1279,21 +1286,22 @@ int lowpass_table(const mem_plan& P, float* gtab, cudaStream_t s) {
 }
 
 int rot_consts(const mem_plan& P, const mem_inputs& in, const PdDev* pd_table,
-               const int32_t* img_pd, void* rot_scratch, cudaStream_t s) {
+               const int32_t* img_pd, void* rot_scratch, uint64_t* qf, cudaStream_t s) {
     if (P.n_images == 0) return MEM_OK;
-    rot_const_kernel<<<(unsigned)((P.n_images + 255) / 256), 256, 0, s>>>(
-        in.psi_rad, pd_table, img_pd, static_cast<RotConst*>(rot_scratch), P.n_images, P.N);
+    rot_const_kernel<<<(unsigned)((P.n_images + 31) / 32), 32, 0, s>>>(
+        in.psi_rad, pd_table, img_pd, static_cast<RotConst*>(rot_scratch), P.n_images, P.N, in.df,
+        qf, P.ctf.q_scale);
     MEM_LAUNCH_CHECK();
     return MEM_OK;
 }
 
 int rotate(const mem_plan& P, const mem_inputs& in, float* xbuf, float* img_out,
            const PdDev* pd_table, const int32_t* img_pd, float2* spec, void* rot_scratch,
-           cudaStream_t s) {
+           uint64_t* qf, cudaStream_t s) {
     if (P.n_images == 0) return MEM_OK;
     const int N = P.N;
     RotConst* rotc = static_cast<RotConst*>(rot_scratch);
-    const int st = rot_consts(P, in, pd_table, img_pd, rot_scratch, s);
+    const int st = rot_consts(P, in, pd_table, img_pd, rot_scratch, qf, s);
     if (st != MEM_OK) return st;
     // the banded kernel where no whole image fits, and for large boxes without a compile-time
     // kernel (800 images of 190 px: 432 us, 456 with the runtime-size kernel; 1000 of 142 px: 327
