@@ -523,6 +523,7 @@ int mem_plan_create(const mem_params* params, int32_t n_pd, const int32_t* pd_co
         return o;
     };
     L.status = take(sizeof(uint32_t) * 4);
+    L.pd_max = take(sizeof(uint32_t) * n_pd);           // beside status: cleared together
     L.pd_table = take(sizeof(PdDev) * n_pd);
     L.sum_items = take(sizeof(SumItem) * P->items.size());
     L.item_off = take(sizeof(int32_t) * (n_pd + 1));
@@ -537,7 +538,6 @@ int mem_plan_create(const mem_params* params, int32_t n_pd, const int32_t* pd_co
     L.qfix = take(sizeof(uint64_t) * P->n_images);
     L.rotc = take(64 * (size_t)P->n_images);            // two fixed-point rotations per image
     L.gtab = take(sizeof(float) * P->N * P->Nh);
-    L.pd_max = take(sizeof(uint32_t) * n_pd);
     L.xbuf = take(sizeof(float) * NN * P->n_images);
     L.spec = take(sizeof(float) * 2 * P->Kc * P->n_images);
     L.feat_a = take(feat_elem * P->Kf * P->n_rows);
@@ -723,7 +723,11 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     } while (0)
 
     // the stack is read by exactly one kernel (the first), issued on the load stream
-    MEM_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(uint32_t) * 4, ls));
+    // the status words, and the PDs' maxima in the same memset (of a split execute later, on the
+    // stream that uses them)
+    MEM_CUDA_TRY(cudaMemsetAsync(status, 0,
+                                 split ? sizeof(uint32_t) * 4
+                                       : L.pd_max + sizeof(uint32_t) * P.n_pd - L.status, ls));
     MEM_STEP(mark(0));
     mem_inputs lin = *in;
     const int64_t* ident = at<int64_t>(ws, L.ident);
@@ -826,7 +830,7 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
         if (out->img_avg) {
             MEM_STEP(kern::pd_sums(P, fspec, qf, items, partial, 1, s));
             MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
-                                       avg_spec, pd_max, 1, s));
+                                       avg_spec, pd_max, 1, false, s));
         }
         if (P.smem_fft && kern::spectrum_masks_supported(P)) {
             MEM_STEP(spectrum(img_all, in->pd_mask));
@@ -837,12 +841,12 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
         if (want_feat || out->img_avg_flip) {
             MEM_STEP(kern::pd_sums(P, fspec, qf, items, partial, 3, s));
             MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
-                                       avg_spec, pd_max, 2, s));
+                                       avg_spec, pd_max, 2, split, s));
         }
     } else if (want_sums) {
         MEM_STEP(kern::pd_sums(P, fspec, qf, items, partial, 3, s));
         MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
-                                   avg_spec, pd_max, 3, s));
+                                   avg_spec, pd_max, 3, split, s));
     }
     MEM_STEP(mark(5));
     // features of D, a_i, sign(C) F, CTF output

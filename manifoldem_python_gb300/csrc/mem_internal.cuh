@@ -242,7 +242,7 @@ int pd_sums(const mem_plan& P, const float2* spec, const uint64_t* qf, const Sum
 // mode bit 1: Wiener average spectrum; bit 2: centring vectors, scale, phase-flip average
 int pd_finalize(const mem_plan& P, const float* partial, const SumItem* items,
                 const int32_t* item_off, const PdDev* pds, const int32_t* ring_of, float* means,
-                float2* avg_spec, uint32_t* pd_max, int mode, cudaStream_t s);
+                float2* avg_spec, uint32_t* pd_max, int mode, bool clear_max, cudaStream_t s);
 int features(const mem_plan& P, float2* spec, const uint64_t* qf, const PdDev* pds,
              const int32_t* img_pd, const int32_t* img_row, const FeatTables& ft,
              const float* means, const uint32_t* scale_bits, void* feat_a, void* feat_b,

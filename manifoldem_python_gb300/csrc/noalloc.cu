@@ -107,14 +107,16 @@ long long ftab_hash(const std::vector<int32_t>& t) {
 // the per-call tables of a one-PD plan of n images, written on the device (no host copy):
 // the PD, the partial-sum items of kSumChunk images, image -> (PD, feature row), and the
 // upper-triangle tiles (I, J), I <= J < nb, in the host plan's order (I outer); and zeros in the
-// status words and the padding rows of the feature matrices (the scratch keeps old contents).
+// status words, the PD's maximum and the padding rows of the feature matrices (the scratch keeps old
+// contents).
 // One launch for all of it: three memsets and a copy of the spectra besides took 300 images of
-// 70 px 100 us, 76 so.
+// 70 px 100 us, 76 without, 73 with the maximum cleared here too.
 __global__ void noalloc_tables_kernel(PdDev* __restrict__ pd, SumItem* __restrict__ items,
                                       int32_t* __restrict__ item_off, int32_t* __restrict__ img_pd,
                                       int32_t* __restrict__ img_row, Tile* __restrict__ tiles,
                                       int n, int n_items, int nb, int n_tiles,
-                                      uint32_t* __restrict__ status, uint4* __restrict__ pad_a,
+                                      uint32_t* __restrict__ status, uint32_t* __restrict__ pd_max,
+                                      uint4* __restrict__ pad_a,
                                       uint4* __restrict__ pad_b, int64_t pad16) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint4 zero = make_uint4(0, 0, 0, 0);
@@ -123,6 +125,7 @@ __global__ void noalloc_tables_kernel(PdDev* __restrict__ pd, SumItem* __restric
         pad_b[i] = zero;
     }
     if (t < 4) status[t] = 0;
+    if (t == 0) *pd_max = 0;
     if (t == 0) {
         *pd = PdDev{0, 0, 0, n, 0, 1.0, 0.0};
         item_off[0] = 0;
@@ -248,7 +251,8 @@ extern "C" int mem_pd_distances_noalloc(const mem_params* params, int32_t n, con
     noalloc_tables_kernel<<<(unsigned)blocks, 256, 0, s>>>(
         at<PdDev>(ws, L.pd_table), at<SumItem>(ws, L.items), at<int32_t>(ws, L.item_off),
         at<int32_t>(ws, L.img_pd), at<int32_t>(ws, L.img_row), at<Tile>(ws, L.tiles), n, n_items,
-        nb, n_tiles, at<uint32_t>(ws, L.status), at<uint4>(ws, L.feat_a + n * row_bytes),
+        nb, n_tiles, at<uint32_t>(ws, L.status), at<uint32_t>(ws, L.pd_max),
+        at<uint4>(ws, L.feat_a + n * row_bytes),
         at<uint4>(ws, L.feat_b + n * row_bytes), pad16);
     MEM_LAUNCH_CHECK();
     // the kernels only read the spectra here, 16 bytes at a time: from the caller's array, or from
@@ -280,7 +284,7 @@ extern "C" int mem_pd_distances_noalloc(const mem_params* params, int32_t n, con
     const FeatTables ft = feat_tables(P, at<char>(ws, L.colmap));
     NA_STEP(kern::pd_finalize(P, at<float>(ws, L.partial), at<SumItem>(ws, L.items),
                               at<int32_t>(ws, L.item_off), pds, ft.ring_of, means,
-                              at<float2>(ws, L.avg_spec), pd_max, 3, s));
+                              at<float2>(ws, L.avg_spec), pd_max, 3, false, s));
     NA_STEP(kern::features(P, spec, qf, pds, at<int32_t>(ws, L.img_pd), at<int32_t>(ws, L.img_row),
                            ft, means, scale_bits, at<char>(ws, L.feat_a),
                            at<char>(ws, L.feat_b), pair_norm, nullptr, false, s));

@@ -1399,8 +1399,8 @@ int pd_sums(const mem_plan& P, const float2* spec, const uint64_t* qf, const Sum
 
 int pd_finalize(const mem_plan& P, const float* partial, const SumItem* items,
                 const int32_t* item_off, const PdDev* pds, const int32_t* ring_of, float* means,
-                float2* avg_spec, uint32_t* pd_max, int mode, cudaStream_t s) {
-    if (mode & 2) MEM_CUDA_TRY(cudaMemsetAsync(pd_max, 0, sizeof(uint32_t) * P.n_pd, s));
+                float2* avg_spec, uint32_t* pd_max, int mode, bool clear_max, cudaStream_t s) {
+    if (clear_max) MEM_CUDA_TRY(cudaMemsetAsync(pd_max, 0, sizeof(uint32_t) * P.n_pd, s));
     dim3 grid((unsigned)P.n_pd, (unsigned)((P.Kc_pad + 255) / 256));
     pd_finalize_kernel<<<grid, 256, 0, s>>>(partial, items, item_off, pds,
                                             P.ring_features ? ring_of : nullptr, means, avg_spec,
