@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "float_sums.cuh"
 #include "mem_internal.cuh"
 
 namespace mem {
@@ -37,6 +38,8 @@ constexpr int kMuRows = 256;       // mu_psi rows staged in shared memory at a t
 constexpr int kAhead = 4;          // steps of a correlation thread whose loads travel together
 static_assert(kMuRows % kAhead == 0, "whole groups of steps");
 constexpr int kWienerChunk = 64;   // Wiener denominators per thread (sliding window)
+constexpr int kMaxParts = 64;      // chunks S of the correlation at most
+static_assert(kWienerChunk <= 64 && kMaxParts <= 64, "wiener_kernel's flags, PartSum's terms");
 constexpr int64_t kTargetThreads = 152 * 4096;   // correlation threads aimed for (chunks S)
 
 inline size_t align_up(size_t x) { return (x + 255) / 256 * 256; }
@@ -63,7 +66,7 @@ NlsaLayout nlsa_layout(int N, int num, int c, int T, bool wiener) {
     L.groups = (T + kModes - 1) / kModes;
     const int64_t lag_blocks = (c + kLags - 1) / kLags;
     int64_t S = (kTargetThreads + L.K * lag_blocks - 1) / (L.K * lag_blocks);
-    S = std::max<int64_t>(1, std::min<int64_t>({S, 64, (int64_t)m}));
+    S = std::max<int64_t>(1, std::min<int64_t>({S, kMaxParts, (int64_t)m}));
     L.chunk = (int)((m + S - 1) / S);
     L.S = (m + L.chunk - 1) / L.chunk;
     L.smem_fft = wiener && (N == 32 || N == 64 || N == 128);
@@ -113,46 +116,14 @@ __global__ void twiddle_kernel(int N, float2* __restrict__ tw) {
     tw[k] = make_float2((float)cs, (float)sn);
 }
 
-// A sum kept as an unevaluated pair of floats (hi + lo, 48 bits): the two-sum of Knuth and, with
-// the FMA, exact products.  FP64 runs at 1/64 of the FP32 rate on this part, and both users round
-// the sum to float: the pair gives the float that FP64 gives, but for sums within 2^-46 of the
-// middle between two floats.
-struct Pair {
-    float hi = 0.f, lo = 0.f;
-    __device__ __forceinline__ void add(float x) {               // Knuth's two-sum of hi and x
-        const float s = __fadd_rn(hi, x);
-        const float t = __fsub_rn(s, hi);
-        lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(x, t)));
-        hi = s;
-    }
-    __device__ __forceinline__ void add_square(float x) {        // + x^2, exactly
-        const float p = __fmul_rn(x, x);
-        add(p);
-        lo = __fadd_rn(lo, __fmaf_rn(x, x, -p));
-    }
-    __device__ __forceinline__ void sub_square(float x) {
-        const float p = __fmul_rn(x, x);
-        add(-p);
-        lo = __fsub_rn(lo, __fmaf_rn(x, x, -p));
-    }
-    __device__ __forceinline__ void settle() {                   // lo back below half an ulp of hi
-        const float s = __fadd_rn(hi, lo);
-        if (s == s) {
-            lo = __fsub_rn(lo, __fsub_rn(s, hi));
-            hi = s;
-        }
-    }
-    __device__ __forceinline__ float value() const {             // an infinite hi has a NaN lo
-        const float s = __fadd_rn(hi, lo);
-        return s == s ? s : hi;
-    }
-};
-
 // rw[i][k] = 1 / wd_i(k), wd_i = sum_{t = i+1 .. i+c} C_t(k)^2 + 1/5 (get_wiener.py:14-19), C_t(k)
 // = ctf[t][ky][kx] for half-plane frequency k = ky Nh + kx.  Each thread starts its chunk of i
-// with the direct sum (t = i+c first, as the reference adds) and slides it as a Pair, the next
-// steps' loads issued ahead; the reciprocal is taken in float32 (the correlation's precision).
-// 1000 images of 128 px, c = 20: 29 us, 134 in FP64 (five FP64 operations per step bound it).
+// with the direct sum (t = i+c first, as the reference adds) and slides it in FP64 precision, the
+// next steps' loads issued ahead; the reciprocal is taken in float32 (the correlation's precision).
+// The float that is inverted is that of the FP64 sum: from the pair sum, or where that leaves it
+// open from the FP64 sum over the chunk (one denominator in 20 thousand for ordinary CTFs).
+// 1000 images of 128 px, c = 20: 48 us, 134 with FP64 sums alone (five FP64 operations per step
+// bound them).
 __global__ void __launch_bounds__(128) wiener_kernel(const float* __restrict__ ctf, int N, int Nh,
                                                      int64_t K, int c, int m,
                                                      float* __restrict__ rw) {
@@ -164,12 +135,10 @@ __global__ void __launch_bounds__(128) wiener_kernel(const float* __restrict__ c
     const float* C = ctf + (int64_t)ky * N + kx;
     const int i0 = blockIdx.y * kWienerChunk;
     const int i1 = min(m, i0 + kWienerChunk);
-    Pair w;
+    SlidingSquares w;
 #pragma unroll 4
-    for (int t = i0 + c; t > i0; --t) {
-        w.add_square(C[t * NN]);
-        w.settle();
-    }
+    for (int t = i0 + c; t > i0; --t) w.start(C[t * NN]);
+    w.started();
     constexpr int B = 8;                           // steps whose samples travel together
     float a[B], b[B];
     auto load = [&](int i) {
@@ -180,6 +149,7 @@ __global__ void __launch_bounds__(128) wiener_kernel(const float* __restrict__ c
             b[u] = C[q * NN];
         }
     };
+    uint64_t open = 0;                             // values that the pair leaves open
     load(i0);
     for (int i = i0; i < i1; i += B) {
         float x[B], y[B];
@@ -192,14 +162,18 @@ __global__ void __launch_bounds__(128) wiener_kernel(const float* __restrict__ c
 #pragma unroll
         for (int u = 0; u < B; ++u) {
             if (i + u >= i1) break;
-            Pair d = w;
-            d.add(0.2f);
-            d.lo = __fadd_rn(d.lo, (float)(0.2 - (double)0.2f));
-            rw[(int64_t)(i + u) * K + k] = __frcp_rn(d.value());
-            w.add_square(x[u]);
-            w.sub_square(y[u]);
-            w.settle();
+            float v;
+            if (!w.plus_fifth(c, i + u - i0, &v)) open |= 1ull << (i + u - i0);
+            rw[(int64_t)(i + u) * K + k] = __frcp_rn(v);
+            w.step(x[u], y[u]);
         }
+    }
+    if (open == 0) return;
+    SlidingSquares64 e;
+    for (int t = i0 + c; t > i0; --t) e.start(C[t * NN]);
+    for (int i = i0; open != 0; ++i, open >>= 1) {
+        if (open & 1) rw[(int64_t)i * K + k] = __frcp_rn(e.plus_fifth());
+        if (open > 1) e.step(C[(int64_t)(i + 1 + c) * NN], C[(int64_t)(i + 1) * NN]);
     }
 }
 
@@ -319,20 +293,30 @@ __global__ void __launch_bounds__(kCorrThreads, 4) correlate_kernel(
     }
 }
 
-// G[q][k] = sum_s part[s][q][k] in a fixed order (q = ii kModes + l), as Pairs: bound by reading the
-// parts (160 MB for 1000 images of 128 px, c = 20: 43 us, 156 with FP64 sums)
+// G[q][k] = sum_s part[s][q][k] in a fixed order (q = ii kModes + l), the floats of FP64 sums: bound by
+// reading the parts (160 MB for 1000 images of 128 px, c = 20: 44 us, 156 with FP64 sums alone)
 __global__ void reduce_parts_kernel(const float2* __restrict__ part, int S, int64_t total,
                                     float2* __restrict__ G) {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= total) return;
-    Pair re, im;
+    PartSum re, im;
 #pragma unroll 8
     for (int s = 0; s < S; ++s) {
         const float2 v = part[(int64_t)s * total + e];
         re.add(v.x);
         im.add(v.y);
     }
-    G[e] = make_float2(re.value(), im.value());
+    float2 g;
+    if (!re.value(S, &g.x) || !im.value(S, &g.y)) {
+        double x = 0.0, y = 0.0;
+        for (int s = 0; s < S; ++s) {
+            const float2 v = part[(int64_t)s * total + e];
+            x += v.x;
+            y += v.y;
+        }
+        g = make_float2((float)x, (float)y);
+    }
+    G[e] = g;
 }
 
 // A[(ii NN + x N + y) T + l0 + l] = msk[y][x] * scale * img[ii kModes + l][y][x], l < nl: the

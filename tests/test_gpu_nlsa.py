@@ -146,3 +146,91 @@ def test_odd_ctf_is_rejected(cuda_ready):
     args[6] = ctf
     with pytest.raises(ValueError):
         NLSA.op(*args)
+
+
+def _delta_snapshots(torch, C, mu_psi, c, N):
+    """A N^2 [c, T] of images that are 1 at one pixel and CTFs that are C_j at frequency 0 alone:
+    every transform is exact there, so each entry is the float sum of the correlation itself."""
+    from manifoldem_python_gb300 import NLSA
+    num = len(C)
+    imgs = torch.zeros((num, N, N), dtype=torch.float32, device='cuda')
+    imgs[:, 0, 0] = 1
+    ctf = torch.zeros((num, N, N), dtype=torch.float32, device='cuda')
+    ctf[:, 0, 0] = torch.from_numpy(C)
+    A = NLSA.snapshots(NLSA._Gpu(None), imgs, ctf, mu_psi, np.array(1), c).cpu().numpy()
+    A = A.reshape(c, N * N, -1) * (N * N)
+    assert np.array_equal(A, np.broadcast_to(A[:, :1], A.shape))
+    return A[:, 0]
+
+
+def _denominators(C, c, m):
+    """1 / wd_i in float from FP64 sums: a direct sum, then a sliding one over 64 denominators."""
+    C = C.astype(np.float64)
+    r = np.empty(m, np.float32)
+    for i in range(m):
+        if i % 64 == 0:
+            w = 0.0
+            for t in range(i + c, i, -1):
+                w += C[t] * C[t]
+        else:
+            w += C[i + c] * C[i + c] - C[i] * C[i]
+        r[i] = np.float32(1) / np.float32(w + 0.2)
+    return r
+
+
+@pytest.mark.parametrize('kind', ['normal', 'large', 'decades', 'zeros'])
+@pytest.mark.parametrize('N,c', [(32, 1), (32, 5), (64, 20)])
+def test_wiener_denominators_are_those_of_fp64_sums(cuda_ready, N, c, kind):
+    """The float Wiener denominators bit for bit, also where a term 10^8 times the sum has left the
+    window: with one mode per denominator (mu_psi one-hot) an entry of A is C_j / wd_i, one float
+    product."""
+    m = 192
+    rng = np.random.default_rng(N + c)
+    C = rng.standard_normal(m + c)
+    if kind == 'large':
+        C[rng.random(m + c) < 0.05] *= 1e4
+    elif kind == 'decades':
+        C *= 10.0 ** rng.uniform(-4, 2, m + c)
+    elif kind == 'zeros':
+        C[rng.random(m + c) < 0.9] = 0
+    C = C.astype(np.float32)
+    r = _denominators(C, c, m)
+    for i0 in range(0, m, 64):
+        got = _delta_snapshots(cuda_ready, C, np.eye(m)[:, i0:i0 + 64], c, N)
+        i = i0 + np.arange(64)
+        for ii in range(c):
+            assert np.array_equal(got[ii], (C[i + c - 1 - ii] * r[i]).astype(np.float64))
+
+
+@pytest.mark.parametrize('kind', ['normal', 'decades', 'short', 'cancel'])
+@pytest.mark.parametrize('N,c,m', [(32, 2, 640), (128, 4, 300)])
+def test_sums_over_parts_are_those_of_fp64(cuda_ready, N, c, m, kind):
+    """The sums over the correlation's parts bit for bit, ties and cancellation among them: mu_psi is
+    not 0 at one step per chunk of i, so every part is a float product."""
+    rng = np.random.default_rng(N + m)
+    T = 64
+    # the chunks of mem_nlsa_snapshots
+    lags = N * (N // 2 + 1) * -(-c // 4)
+    S = max(1, min(-(-152 * 4096 // lags), 64, m))
+    chunk = -(-m // S)
+    first = np.arange(0, m, chunk)
+    v = rng.standard_normal((len(first), T))
+    if kind == 'decades':
+        v *= 10.0 ** rng.uniform(-6, 6, v.shape)
+    elif kind == 'short':
+        v = np.ldexp(rng.integers(-2048, 2048, v.shape).astype(np.float64),
+                     rng.integers(0, 26, v.shape))
+    elif kind == 'cancel':
+        v[1::2] = -v[:len(v) - len(v) % 2:2] * (1 + 1e-6 * rng.integers(0, 2, (len(v) // 2, T)))
+        v[::2] *= 10.0 ** rng.uniform(-3, 3, v[::2].shape)
+    mu = np.zeros((m, T))
+    mu[first] = v
+    # C^2 = 2/15, so that c C^2 + 1/5 is a power of two or near it; the products round as usual
+    C = np.full(m + c, np.float32(np.sqrt(2 / 15)), np.float32)
+    r = _denominators(C, c, m)
+    got = _delta_snapshots(cuda_ready, C, mu, c, N)
+    parts = C[0] * (r[first][:, None] * v.astype(np.float32))
+    want = np.zeros(T)
+    for p in parts.astype(np.float64):
+        want = want + p
+    assert np.array_equal(got, np.broadcast_to(want.astype(np.float32), got.shape))
