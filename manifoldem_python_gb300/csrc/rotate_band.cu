@@ -22,7 +22,7 @@
 // Bound by issue slots, then shared-memory wavefronts (16 tap loads per sample, about two-way
 // conflicts; one 5x5 window for two samples, rot::sample_pair, has fewer loads but more
 // instructions and took 1016 us).  Three bands of 84 rows at 250 px, two CTAs of 512 threads per
-// SM.  1198 images of 250 px: 956 us; 1032 with the paired rows 16 apart (coordinates, column
+// SM.  1198 images of 250 px: 961 us; 1032 with the paired rows 16 apart (coordinates, column
 // counters and bounds of their own); 1453 with one CTA per image working through the bands of
 // both rotations, which was bound by its barriers (one CTA per SM, the column coefficients
 // through global scratch) and by the sampling loops' idle lanes.
@@ -256,16 +256,19 @@ __global__ void __launch_bounds__(kBandThreads, 2) rotate_band_kernel(
     {
         const int r = 2 * warp + 2 * kBandWarps * (lane >> 1) + (lane & 1);
         const int64_t Ur = U00 + (int64_t)r * dUr;
-        const float u0 = (float)Ur * 2.3283064365386963e-10f;
-        const float inv = 4294967296.0f / (float)dUc;
+        const float inv = 1.0f / (float)dUc;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const int base = b0 + (k - 1) * N;
             lo[k] = 0;
             hi[k] = N;
             if (dUc != 0) {
-                // in layout rows; widened by a column each way (every sample checks its row)
-                const float ea = ((float)base - u0) * inv, eb = ((float)(base + h) - u0) * inv;
+                // The distances to the band are formed in fixed point, so that the bounds are good to
+                // 2^-22 of themselves at any slope (from coordinates rounded to float they were
+                // many columns off where a row is almost level, near multiples of 90 degrees).
+                // Widened by a column each way; every sample checks its row
+                const float ea = (float)((int64_t)base * kOne - Ur) * inv;
+                const float eb = (float)((int64_t)(base + h) * kOne - Ur) * inv;
                 const float a = fminf(fmaxf(fminf(ea, eb), -2.f), (float)N + 2.f);
                 const float b = fminf(fmaxf(fmaxf(ea, eb), -2.f), (float)N + 2.f);
                 lo[k] = max(0, (int)floorf(a) - 1);

@@ -230,3 +230,38 @@ def test_band_rotation_matches_whole_image_kernels(cuda_ready, N):
             e = rel(np.asarray(outs[2, variant][k]), np.asarray(outs[0, 0][k]))
             print('N=%d variant %d %s: banded vs whole-image rotation %.3g' % (N, variant, k, e))
             assert e < 2e-6, (variant, k, e)
+
+
+@pytest.mark.parametrize('N,bands', [(65, 0), (97, 9), (187, 0), (190, 5), (237, 0), (250, 0),
+                                     (250, 7), (257, 9), (300, 0), (400, 0), (511, 0), (512, 9)])
+def test_band_rotation_near_right_angles(cuda_ready, monkeypatch, N, bands):
+    """The banded rotation where a row of samples is almost level in the other image (angles within
+    1e-9 to 1e-3 of multiples of 90 degrees, exact ones and multiples rounded to float32 among
+    them), with more bands than the default, odd sizes and short last segments, against the
+    whole-image kernels.  Outputs and the workspace's image slots hold NaN before, so that a sample
+    that no band computes fails.  Tolerance: float rounding of both, 1e-5 of the largest value as
+    for every image output."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    near = [k * np.pi / 2 + s * d for k in (-1, 0, 1, 2) for d in (0, 1e-9, 1e-7, 1e-6, 1e-5, 1e-4, 1e-3)
+            for s in (1, -1)] + [float(np.float32(k * np.pi / 2)) for k in (1, 2, 3)] + [0.6, 2.9]
+    psi_p = np.degrees(near[::5] + near[-5:])
+    rng = np.random.default_rng(N)
+    psi = rng.permutation(np.resize(near, 4 * len(psi_p)))
+    n = len(psi)
+    stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
+    args = (torch.arange(n, device='cuda'), torch.zeros(n, dtype=torch.uint8, device='cuda'),
+            torch.from_numpy(psi).cuda(), torch.full((n,), 2e4, dtype=torch.float64, device='cuda'))
+    got = []
+    for band in ('0', '2'):
+        monkeypatch.setenv('MEM_ROT_BAND', band)
+        monkeypatch.setenv('MEM_ROT_BANDS', str(bands))
+        plan = Plan(StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1,
+                                avg_only=True), [4] * len(psi_p), psi_p)
+        out = plan.allocate_outputs(('img_all',))
+        plan.execute(torch.full_like(stack, float('nan')), *args, out)     # NaN in every slot
+        out['img_all'].fill_(float('nan'))
+        plan.execute(stack, *args, out)
+        got.append(out['img_all'].cpu().numpy())
+    assert np.isfinite(got[1]).all()
+    assert np.abs(got[1] - got[0]).max() <= 1e-5 * np.abs(got[0]).max()
