@@ -875,11 +875,19 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     MEM_STEP(mark(7));
     // phase-flipped images and their mean intensity
     if (want_flip) {
-        float* flip_imgs = out->img_all_flip ? out->img_all_flip : xbuf;
+        // a caller's array may start on any float; the transforms that keep pairs in it go through
+        // xbuf then
+        const bool copied = out->img_all_flip && P.smem_fft &&
+                            reinterpret_cast<uintptr_t>(out->img_all_flip) %
+                                    mixed::inverse_alignment(P.N) != 0;
+        float* flip_imgs = out->img_all_flip && !copied ? out->img_all_flip : xbuf;
         if (P.smem_fft)
             MEM_STEP(kern::inverse_fft(P, P.n_images, fspec, twid, flip_imgs, qf, true, s));
         else
             MEM_STEP(exec_fft(P, CUFFT_C2R, P.n_images, specN, NN, spec, flip_imgs, work, s));
+        if (copied)
+            MEM_CUDA_TRY(cudaMemcpyAsync(out->img_all_flip, xbuf, sizeof(float) * NN * P.n_images,
+                                         cudaMemcpyDeviceToDevice, s));
         MEM_STEP(kern::intensity(P, flip_imgs, pds, out->img_all_intensity, s));
     }
     MEM_STEP(mark(8));

@@ -57,6 +57,7 @@ struct InverseArgs {
 // the kernels of one box size
 struct Kernels {
     int N, threads;
+    bool tiled;                  // the inverse keeps pairs of floats in its output
     size_t smem;
     void (*lowpass)(LowpassArgs);
     void (*spectrum)(SpectrumArgs);
@@ -670,11 +671,11 @@ constexpr Kernels make_kernels() {
     using Sh = fft::MixShape<N, R1, N / R1>;
     if constexpr (whole_bytes<Sh>() + sizeof(float2) * N + 1024 <= 227 * 1024) {
         constexpr int NT = whole_threads<Sh>(), MB = whole_blocks<Sh>();
-        return Kernels{N, NT, whole_bytes<Sh>(), whole_lowpass_kernel<Sh, NT, MB>,
+        return Kernels{N, NT, false, whole_bytes<Sh>(), whole_lowpass_kernel<Sh, NT, MB>,
                        whole_spectrum_kernel<Sh, NT, MB>, whole_inverse_kernel<Sh, NT, MB, false>,
                        whole_inverse_kernel<Sh, NT, MB, true>, nullptr, 0, 0};
     } else {
-        return Kernels{N, Tile<Sh>::NT, Tile<Sh>::bytes, tiled_lowpass_kernel<Sh>,
+        return Kernels{N, Tile<Sh>::NT, true, Tile<Sh>::bytes, tiled_lowpass_kernel<Sh>,
                        tiled_spectrum_kernel<Sh>, tiled_inverse_kernel<Sh, false>,
                        tiled_inverse_kernel<Sh, true>, nullptr, 0, 0};
     }

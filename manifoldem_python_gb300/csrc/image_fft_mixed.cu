@@ -47,6 +47,11 @@ int launch(const Kernels& k, void (*fn)(Args), const Args& args, int64_t images,
 
 bool supported(int N) { return find(N) != nullptr; }
 
+size_t inverse_alignment(int N) {
+    const Kernels* k = find(N);
+    return k && k->tiled ? sizeof(float2) : sizeof(float);
+}
+
 int lowpass(int N, const mem_inputs& in, int64_t images, const float* gtab, const float2* twid,
             float* xbuf, uint32_t* status, cudaStream_t s) {
     const Kernels* k = find(N);

@@ -176,6 +176,7 @@ int spectrum(int N, int64_t images, const float* src, const uint8_t* masks, cons
              const float2* twid, float2* spec, cudaStream_t s);
 int inverse(int N, int64_t images, const float2* spec, const float2* twid, float* dst,
             const uint64_t* qf, const CtfConst& cc, cudaStream_t s);
+size_t inverse_alignment(int N);     // bytes that dst starts on a multiple of
 // the two rotations of whole images in shared memory (sizes up to 224 of the table); rotc: the
 // constants that rot_consts writes
 bool rotate_supported(int N);

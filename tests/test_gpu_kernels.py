@@ -546,3 +546,31 @@ def test_symmetrised_distances_of_special_values(cuda_ready, n, knn):
     _call(torch, 'mem_dm_symmetrise', d.data_ptr(), n, nb.data_ptr() if knn else None,
           y.data_ptr())
     np.testing.assert_allclose(y.cpu().numpy(), Y, rtol=1e-14, atol=0)
+
+
+@pytest.mark.parametrize('N', [32, 100, 230, 250, 300])
+def test_image_outputs_at_any_float_address(cuda_ready, N):
+    """Image outputs that start one float past an aligned address: the same bits as aligned ones.
+    For images beyond one SM's shared memory the inverse transform keeps pairs of floats in its output
+    meanwhile."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    rng = np.random.default_rng(N)
+    n = 5
+    stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
+    plan = Plan(StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1, avg_only=True),
+                [3, 2], [10.0, -50.0])
+    args = (stack, torch.arange(n, device='cuda'), torch.zeros(n, dtype=torch.uint8, device='cuda'),
+            torch.from_numpy(rng.uniform(-3, 3, n)).cuda(),
+            torch.full((n,), 2e4, dtype=torch.float64, device='cuda'))
+    names = ('img_all', 'img_all_flip', 'img_all_intensity', 'ctf')
+    got = []
+    for shift in (0, 1):
+        out = plan.allocate_outputs(names)
+        for k in ('img_all', 'img_all_flip', 'ctf'):
+            buf = torch.full((n * N * N + 4,), float('nan'), dtype=torch.float32, device='cuda')
+            out[k] = buf[shift:shift + n * N * N].view(n, N, N)
+        plan.execute(*args, out)
+        got.append({k: out[k].cpu().numpy() for k in names})
+    for k in names:
+        assert np.isfinite(got[0][k]).all() and np.array_equal(got[0][k], got[1][k]), k
