@@ -195,9 +195,10 @@ __device__ __forceinline__ void shift_axis(float* s, float* carry, const float* 
     const int k0 = g * L, len = min(L, N - k0);
     // output k samples at k - shift = k + i0 + t
     const double fl = floor(-shift);
-    // far outside, where every sample wraps, the whole part is first reduced by whole periods
+    // far outside, where every sample wraps, the whole part is first reduced by whole periods, to the
+    // same side (a sample a whole number of periods away lands on the line's other end)
     const double per = (double)(N - 1);
-    const double fr = fabs(fl) > 1.0e6 ? fl - per * floor(fl / per) - 16.0 * per : fl;
+    const double fr = fabs(fl) > 1.0e6 ? fl - per * floor(fl / per) + copysign(16.0 * per, fl) : fl;
     const int i0 = (int)fmin(fmax(fr, -1.0e9), 1.0e9);       // in range for a NaN or inf shift too
     const float t = (float)(-shift - fl);
     float w[4];

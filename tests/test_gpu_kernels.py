@@ -574,3 +574,34 @@ def test_image_outputs_at_any_float_address(cuda_ready, N):
         got.append({k: out[k].cpu().numpy() for k in names})
     for k in names:
         assert np.isfinite(got[0][k]).all() and np.array_equal(got[0][k], got[1][k]), k
+
+
+@pytest.mark.parametrize('N', [8, 39, 40, 97, 128, 236])
+def test_relion_shift_by_far_whole_numbers(cuda_ready, N):
+    """Whole-number shifts of both signs beyond a million pixels, whole periods (N - 1) among them,
+    whose wrapped sample is an end of the line: as scipy's shift, tolerance as test_relion_shift."""
+    torch = cuda_ready
+    from scipy.ndimage import shift
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    rng = np.random.default_rng(N)
+    far = [s * v for v in (999999, 1000001, 1000005, 3 * 10 ** 9 + 1, (N - 1) * 20011, (N - 1) * 300007,
+                           (N - 1) * 300007 + 3, 2 ** 33) for s in (1, -1)]
+    sh = np.array([[a, b] for a, b in zip(far, far[3:] + far[:3])], dtype=np.float64)
+    n = len(sh)
+    stack = rng.standard_normal((n, N, N)).astype(np.float32)
+    plan = Plan(StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1,
+                            filter_Qc=1e9, avg_only=True), [n], [0.0])
+    out = plan.allocate_outputs(('img_all',))
+    plan.execute(torch.from_numpy(stack).cuda(), torch.arange(n, device='cuda'),
+                 torch.zeros(n, dtype=torch.uint8, device='cuda'),
+                 torch.zeros(n, dtype=torch.float64, device='cuda'),
+                 torch.full((n,), 2e4, dtype=torch.float64, device='cuda'), out,
+                 shift_yx=torch.from_numpy(sh).cuda())
+    got = out['img_all'].cpu().numpy()
+    r, c = np.mgrid[0:N, 0:N]
+    msk = ((r - N / 2 + 1) ** 2 + (c - N / 2) ** 2 < (N / 2) ** 2)
+    for i in range(n):
+        x = shift(stack[i].astype(np.float64), sh[i], order=3, mode='wrap')
+        b = x * (1 - msk)
+        ref = (x - b.mean()) / b.std() * msk
+        assert np.abs(got[i] - ref).max() <= 1e-5 * np.abs(ref).max(), (i, sh[i])
