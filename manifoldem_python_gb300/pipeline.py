@@ -134,6 +134,7 @@ class Plan:
         """(outputs, block): outputs of up to ONE_BLOCK_BYTES in all as spans of one allocation,
         which is read back in one copy; larger ones as ``allocate_outputs``, block None."""
         import torch
+        names = tuple(names)
         spans, o = {}, 0
         for k, (shape, dt) in self._output_shapes(names).items():
             dt = np.float64 if dt == torch.float64 else np.float32

@@ -5,6 +5,7 @@ import pickle
 import tempfile
 
 import numpy as np
+import pytest
 
 from manifoldem_python_gb300 import GetDistancesS2 as G
 from manifoldem_python_gb300 import myio
@@ -175,3 +176,18 @@ def test_bench_reads_profile_figures():
     assert bench.profile_number('rotate', 'config5', 'shared_wavefronts_per_image') == 149825
     assert bench.traffic_from_profiles('contraction_bf16x3', 'config4') == 3.11e10
     assert bench.profile_number('rotate', 'config3', 'shared_wavefronts_per_image') is None
+
+
+@pytest.mark.parametrize('limit', [0, 1 << 20])
+def test_output_names_from_an_iterator(monkeypatch, limit):
+    """The outputs of a call may be named by an iterator, in one block and as arrays of their own."""
+    torch = pytest.importorskip('torch')
+    from manifoldem_python_gb300 import pipeline
+    monkeypatch.setattr(pipeline, 'ONE_BLOCK_BYTES', limit)
+    plan = pipeline.Plan.__new__(pipeline.Plan)
+    plan.params = pipeline.StageParams(N=8, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1)
+    plan.counts, plan.n_images, plan.d_elems = np.array([3]), 3, 9
+    plan.device = torch.device('cpu')
+    outs, block = plan._allocate_block(iter(('D', 'img_all')))
+    assert list(outs) == ['D', 'img_all'] and (block is None) == (limit == 0)
+    assert tuple(outs['img_all'].shape) == (3, 8, 8)
