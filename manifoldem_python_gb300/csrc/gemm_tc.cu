@@ -70,6 +70,7 @@ struct TcShared {
     uint64_t mma_done;
     uint32_t tmem_base;
     int abort_flag;
+    int ticket;
 };
 
 // Where tile x of the `rest` tiles of the last wave of S CTAs is cut (chunks of its head).  Tile x's
@@ -105,12 +106,14 @@ __device__ __forceinline__ bool flag_wait(const unsigned* flag, volatile int* ab
 // accumulators (NBUF x 128 columns) continue from one tile to the next, so a tile's first
 // groups are loaded and multiplied while the epilogue still adds and stores the previous tile.
 //
-// SPLIT: as many CTAs as SMs (T tiles on S of them, S < T, launched together): each CTA computes
-// T / S whole tiles, and every tile of the last, partial wave is cut in two at a chunk: one CTA
-// computes its first chunks before its whole tiles and leaves the running sums in `carry`, another
-// continues from them after its own, so that the sums are the same, chunk by chunk.  See
-// tc_cut_of for the cuts.  A continuing warp waits (bounded) for the flag of the warp it follows,
-// which was set about a tile's time before.
+// SPLIT: as many CTAs as SMs (T tiles on S of them, S < T): each CTA computes T / S whole tiles, and
+// every tile of the last, partial wave is cut in two at a chunk: one CTA computes its first chunks
+// before its whole tiles and leaves the running sums in `carry`, another continues from them after
+// its own, so that the sums are the same, chunk by chunk.  See tc_cut_of for the cuts.  A continuing
+// warp waits (bounded) for the flag of the warp it follows, which was set about a tile's time
+// before.  CTA b is the b-th to start (a ticket): it only waits for CTAs that started before it, and
+// only for what they do first and without waiting, so that the waits end also where the CTAs do not
+// all fit at once (SMs held by other work, a context with fewer of them).
 template <bool KAHAN, bool LOLO, int NBUF, int BN, bool SPLIT>
 __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
         const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
@@ -118,7 +121,8 @@ __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
         const Tile* __restrict__ tiles, const PdDev* __restrict__ pds, double* __restrict__ D,
         uint32_t* __restrict__ status, const int4* __restrict__ chunks, int nchunks,
         int group_chunks, long long wait_limit, int withhold, int tile_begin, int tile_count,
-        float* __restrict__ carry, unsigned* __restrict__ carry_flags) {
+        float* __restrict__ carry, unsigned* __restrict__ carry_flags,
+        unsigned* __restrict__ tickets) {
     static_assert(NBUF == 2 || NBUF == 4, "two or four TMEM accumulators");
     static_assert(BN == 128 || BN == 256, "tile widths");
     static_assert(NBUF * BN <= 512, "TMEM holds 512 columns");
@@ -133,31 +137,6 @@ __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
     TcShared* sh = (TcShared*)(smem + TC_STAGES * TC_STAGE_BYTES);
     volatile int* abort_flag = &sh->abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // SPLIT: this CTA's parts are [head of tile blockIdx.x], whole tiles, [tail of tile tail]
-    const int rest = SPLIT ? tile_count % (int)gridDim.x : 0;
-    const int tail = SPLIT ? (int)blockIdx.x - ((int)gridDim.x - rest) : -1;
-    const int heads = SPLIT && (int)blockIdx.x < rest ? 1 : 0;
-    const int whole = SPLIT ? tile_count / (int)gridDim.x
-                      : (int)blockIdx.x < tile_count
-                          ? (tile_count - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x
-                          : 0;
-    const int my_tiles = heads + whole + (tail >= 0 ? 1 : 0);
-    struct Part {
-        Tile t;
-        int c0, c1;                                // its chunks
-    };
-    auto part_of = [&](int lt) {
-        Part p;
-        const int k = lt - heads;
-        const int i = !SPLIT           ? (int)blockIdx.x + lt * (int)gridDim.x
-                      : k < 0          ? (int)blockIdx.x
-                      : k < whole      ? rest + (int)blockIdx.x + k * (int)gridDim.x
-                                       : tail;
-        p.t = tiles[tile_begin + i];
-        p.c0 = SPLIT && k == whole ? tc_cut_of(tail, rest, (int)gridDim.x, nchunks) : 0;
-        p.c1 = SPLIT && k < 0 ? tc_cut_of(i, rest, (int)gridDim.x, nchunks) : nchunks;
-        return p;
-    };
     const int gsize = (group_chunks > 0 && group_chunks < nchunks) ? group_chunks : nchunks;
     const int ngroups = (nchunks + gsize - 1) / gsize;
 
@@ -172,6 +151,7 @@ __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
         }
         mbar_init(&sh->mma_done, 1);
         sh->abort_flag = 0;
+        if (SPLIT) sh->ticket = (int)atomicAdd(tickets, 1u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == EPI + 1) {
@@ -185,6 +165,32 @@ __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = sh->tmem_base;
+    const int cta = SPLIT ? sh->ticket : (int)blockIdx.x;
+    // SPLIT: this CTA's parts are [head of tile cta], whole tiles, [tail of tile tail]
+    const int rest = SPLIT ? tile_count % (int)gridDim.x : 0;
+    const int tail = SPLIT ? cta - ((int)gridDim.x - rest) : -1;
+    const int heads = SPLIT && cta < rest ? 1 : 0;
+    const int whole = SPLIT ? tile_count / (int)gridDim.x
+                      : cta < tile_count
+                          ? (tile_count - cta + (int)gridDim.x - 1) / (int)gridDim.x
+                          : 0;
+    const int my_tiles = heads + whole + (tail >= 0 ? 1 : 0);
+    struct Part {
+        Tile t;
+        int c0, c1;                                // its chunks
+    };
+    auto part_of = [&](int lt) {
+        Part p;
+        const int k = lt - heads;
+        const int i = !SPLIT           ? cta + lt * (int)gridDim.x
+                      : k < 0          ? cta
+                      : k < whole      ? rest + cta + k * (int)gridDim.x
+                                       : tail;
+        p.t = tiles[tile_begin + i];
+        p.c0 = SPLIT && k == whole ? tc_cut_of(tail, rest, (int)gridDim.x, nchunks) : 0;
+        p.c1 = SPLIT && k < 0 ? tc_cut_of(i, rest, (int)gridDim.x, nchunks) : nchunks;
+        return p;
+    };
 
     if (warp == EPI) {
         // ---------------------------------------------------------------- TMA producer
@@ -369,7 +375,7 @@ __global__ void __launch_bounds__(TcShape<BN>::THREADS, 1) gemm_tc_kernel(
             }
             if (!ok || *abort_flag) break;
             if (SPLIT && part.c1 < nchunks) {      // a head: leave the sums, then the flag
-                const int64_t at = (int64_t)blockIdx.x * EPI + warp;
+                const int64_t at = (int64_t)cta * EPI + warp;
                 float* to = carry + at * (EC * 32) + lane;
 #pragma unroll
                 for (int j = 0; j < EC; ++j) __stcg(to + 32 * j, acc[j]);
@@ -913,8 +919,8 @@ int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
         return MEM_OK;
     }
     const int sms = P.num_sms > 0 ? P.num_sms : 1;
-    // the default schedule where the last wave is partial: its tiles cut in two (a cooperative launch
-    // waits for all SMs, so not beside the load stream of a split execute)
+    // the default schedule where the last wave is partial: its tiles cut in two (no gain beside the load
+    // stream of a split execute, whose CTAs hold some SMs)
     if (cut && P.tc_carry >= sms && P.tc_ranges.size() == 1 && !c0.persistent && c0.accumulators == 2 &&
         c0.tile_m == 128 && P.tc_group_chunks == 1 && !P.tc_kahan && P.test_withhold_chunk < 0 &&
         tc_cut_pays(T, sms)) {
@@ -926,24 +932,16 @@ int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
                                     : gemm_tc_kernel<false, false, 2, 128, true>);
         const size_t smem = c0.tile_n == 256 ? TcShape<256>::SMEM : TcShape<128>::SMEM;
         const int threads = c0.tile_n == 256 ? TcShape<256>::THREADS : TcShape<128>::THREADS;
-        unsigned* flags = reinterpret_cast<unsigned*>(part);
+        unsigned* tickets = reinterpret_cast<unsigned*>(part);    // one, then the flags
+        unsigned* flags = tickets + 16;
         float* carry = part + kTcFlagBytes / sizeof(float);
         MEM_CUDA_TRY(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
-        MEM_CUDA_TRY(cudaMemsetAsync(flags, 0, sizeof(unsigned) * 16 * rest, s));
-        cudaLaunchAttribute coop{};
-        coop.id = cudaLaunchAttributeCooperative;      // CTAs wait on one another
-        coop.val.cooperative = 1;
-        cudaLaunchConfig_t lc{};
-        lc.gridDim = dim3((unsigned)sms);
-        lc.blockDim = dim3((unsigned)threads);
-        lc.dynamicSmemBytes = smem;
-        lc.stream = s;
-        lc.attrs = &coop;
-        lc.numAttrs = 1;
-        MEM_CUDA_TRY(cudaLaunchKernelEx(&lc, kfn, mhi, mlo, pair_norm, scale_bits, tiles, pds, D,
-                                        status, chunks, P.n_chunks, P.tc_group_chunks,
-                                        P.wait_cycles, P.test_withhold_chunk, 0, T, carry, flags));
+        MEM_CUDA_TRY(cudaMemsetAsync(tickets, 0, sizeof(unsigned) * (16 + 16 * rest), s));
+        kfn<<<(unsigned)sms, threads, smem, s>>>(mhi, mlo, pair_norm, scale_bits, tiles, pds, D,
+                                                 status, chunks, P.n_chunks, P.tc_group_chunks,
+                                                 P.wait_cycles, P.test_withhold_chunk, 0, T, carry,
+                                                 flags, tickets);
         MEM_LAUNCH_CHECK();
         return MEM_OK;
     }
@@ -993,7 +991,7 @@ int gemm_split_bf16(const mem_plan& P, const void* feat_hi, const void* feat_lo,
             <<<grid, TcShape<BN>::THREADS, TcShape<BN>::SMEM, s>>>(                            \
                 mhi, mlo, pair_norm, scale_bits, tiles, pds, D, status, chunks, P.n_chunks,    \
                 P.tc_group_chunks, P.wait_cycles, P.test_withhold_chunk, begin, count,         \
-                nullptr, nullptr);                                                             \
+                nullptr, nullptr, nullptr);                                                    \
     } while (0)
 #define MEM_TC_SHAPE(KAHAN, LOLO)                                                              \
     do {                                                                                       \

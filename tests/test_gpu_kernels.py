@@ -605,3 +605,98 @@ def test_relion_shift_by_far_whole_numbers(cuda_ready, N):
         b = x * (1 - msk)
         ref = (x - b.mean()) / b.std() * msk
         assert np.abs(got[i] - ref).max() <= 1e-5 * np.abs(ref).max(), (i, sh[i])
+
+
+@pytest.mark.parametrize('tile_n', [128, 256])
+def test_cut_tiles_beside_other_streams(cuda_ready, tile_n):
+    """Contractions with cut tiles on three streams at once, so that the CTAs of none of them have the
+    SMs to themselves: the same D, bit for bit, as one after the other."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    N, big_tiles = 64, {128: 136, 256: 72}[tile_n]
+    params = StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1,
+                         precision='bf16x3')
+    runs = []
+    for rest in (30, 98, sms - 1):
+        counts = [2000] + [3] * (sms + rest - big_tiles)
+        n = sum(counts)
+        rng = np.random.default_rng(rest)
+        plan = Plan(params, counts, [0.3] * len(counts),
+                    contraction=[dict(max_n=2 ** 31 - 1, persistent=0, accumulators=2,
+                                      tile_n=tile_n)])
+        out = plan.allocate_outputs(('D',))
+        args = (torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda(),
+                torch.arange(n, device='cuda'), torch.zeros(n, dtype=torch.uint8, device='cuda'),
+                torch.from_numpy(rng.uniform(-3, 3, n)).cuda(),
+                torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda(), out)
+        plan.execute(*args)
+        torch.cuda.synchronize()
+        plan.device_status()
+        runs.append((plan, args, out['D'].clone(), torch.cuda.Stream()))
+        out['D'].fill_(float('nan'))
+    torch.cuda.synchronize()
+    for _ in range(4):
+        for plan, args, _, stream in runs:
+            plan.execute(*args, stream)
+    torch.cuda.synchronize()
+    for plan, args, D, _ in runs:
+        plan.device_status()
+        assert bool(torch.isfinite(D).all()) and torch.equal(D, args[-1]['D'])
+
+
+@pytest.fixture
+def few_sms(cuda_ready):
+    """A stream that may use at least 64 but not all of the SMs (a green context's)."""
+    torch = cuda_ready
+    cu = ctypes.CDLL('libcuda.so.1')
+    if torch.cuda.get_device_properties(0).multi_processor_count < 96:
+        pytest.skip('too few SMs to leave some out')
+    torch.zeros(1, device='cuda')
+    every, some, rest = ((ctypes.c_byte * 144)() for _ in range(3))        # CUdevResource
+    n, desc, ctx, stream = (ctypes.c_uint(1), ctypes.c_void_p(), ctypes.c_void_p(),
+                            ctypes.c_void_p())
+
+    def call(name, *args):
+        if getattr(cu, name)(*args) != 0:
+            pytest.skip(name + ' is not available')
+
+    call('cuDeviceGetDevResource', 0, every, 1)                            # 1: SMs
+    call('cuDevSmResourceSplitByCount', some, ctypes.byref(n), every, rest, 0, 64)
+    call('cuDevResourceGenerateDesc', ctypes.byref(desc), some, 1)
+    call('cuGreenCtxCreate', ctypes.byref(ctx), desc, 0, 1)                # 1: default stream
+    call('cuGreenCtxStreamCreate', ctypes.byref(stream), ctx, 1, 0)        # 1: non-blocking
+    yield torch.cuda.ExternalStream(stream.value)
+    torch.cuda.synchronize()
+    cu.cuStreamDestroy_v2(stream)
+    cu.cuGreenCtxDestroy(ctx)
+
+
+@pytest.mark.parametrize('tile_n', [128, 256])
+def test_cut_tiles_on_some_of_the_sms(cuda_ready, few_sms, tile_n):
+    """A plan with cut tiles, laid out for all SMs of the device, on a stream that may use fewer: the
+    CTAs do not fit at once.  The same D, bit for bit."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    N, rest, big_tiles = 32, 98, {128: 136, 256: 72}[tile_n]
+    counts = [2000] + [3] * (sms + rest - big_tiles)
+    n = sum(counts)
+    rng = np.random.default_rng(1)
+    plan = Plan(StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1,
+                            precision='bf16x3'), counts, [0.3] * len(counts),
+                contraction=[dict(max_n=2 ** 31 - 1, persistent=0, accumulators=2, tile_n=tile_n)])
+    out = plan.allocate_outputs(('D',))
+    args = (torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda(),
+            torch.arange(n, device='cuda'), torch.zeros(n, dtype=torch.uint8, device='cuda'),
+            torch.from_numpy(rng.uniform(-3, 3, n)).cuda(),
+            torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda(), out)
+    D = []
+    for stream in (None, few_sms):
+        out['D'].fill_(float('nan'))
+        torch.cuda.synchronize()
+        plan.execute(*args, stream)
+        torch.cuda.synchronize()
+        plan.device_status()
+        D.append(out['D'].clone())
+    assert bool(torch.isfinite(D[0]).all()) and torch.equal(D[0], D[1])
