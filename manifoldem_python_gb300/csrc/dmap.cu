@@ -38,9 +38,10 @@ constexpr int kTile = 32;
 constexpr long long kInfBits = 0x7ff0000000000000ll;
 // kZeroDist <= d <= inf
 __device__ __forceinline__ bool dm_far(double d) {
-    const long long zero = __double_as_longlong(kZeroDist);
-    return (unsigned long long)(__double_as_longlong(d) - zero) <=
-           (unsigned long long)(kInfBits - zero);
+    // unsigned: a negative d's pattern lies above all positive ones
+    const unsigned long long zero = (unsigned long long)__double_as_longlong(kZeroDist);
+    return (unsigned long long)__double_as_longlong(d) - zero <=
+           (unsigned long long)kInfBits - zero;
 }
 __device__ __forceinline__ bool dm_nan(double d) {
     return (__double_as_longlong(d) & 0x7fffffffffffffffll) > kInfBits;
