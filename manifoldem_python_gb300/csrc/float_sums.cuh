@@ -84,9 +84,10 @@ struct Pair {
         add(-p);
         lo = MEM_SUB(lo, MEM_FMA(x, x, -p));
     }
-    MEM_SUM_HD void settle() {                                   // exact where |hi| >= |lo|
+    MEM_SUM_HD void settle() {                                   // the two-sum of hi and lo
         const float s = MEM_ADD(hi, lo);
-        lo = MEM_SUB(lo, MEM_SUB(s, hi));
+        const float t = MEM_SUB(s, hi);
+        lo = MEM_ADD(MEM_SUB(hi, MEM_SUB(s, t)), MEM_SUB(lo, t));
         hi = s;
     }
     // the float that every value within err of hi + lo rounds to; false where there are several (or
@@ -104,7 +105,7 @@ struct Pair {
 // 6 for 1/5; FP64: 2^-53 b per operation.  err() holds them with room for (1 + eps) factors.
 struct SlidingSquares {
     Pair w;
-    float most = 0.f, least = 3.4e38f;             // of hi; least: after a step
+    float most = 0.f;                              // of hi
     MEM_SUM_HD void start(float x) {
         w.add_square(x);
         w.settle();
@@ -115,21 +116,21 @@ struct SlidingSquares {
         most = fmaxf(most, w.hi);
         w.sub_square(y);
         w.settle();
-        least = fminf(least, w.hi);
     }
-    // c starting terms, k steps so far; settle() is exact while hi >= 5 eps most
+    // c starting terms, k steps so far
     MEM_SUM_HD bool plus_fifth(int c, int k, float* v) const {
         Pair d = w;
         d.add(0.2f);
         d.lo = MEM_ADD(d.lo, (float)(0.2 - (double)0.2f));
         const float err = (most + 0.2f) * kEps2 * (5.25f * (float)c + 14.5f * (float)k + 8.f);
-        return d.rounds(err, v) && least * 2097152.f >= most;
+        return d.rounds(err, v);
     }
 };
 // the FP64 sum itself
 struct SlidingSquares64 {
     double w = 0.0;
     MEM_SUM_HD void start(float x) { w += (double)x * (double)x; }
+    MEM_SUM_HD void started() {}
     MEM_SUM_HD void step(float x, float y) {
         w += (double)x * (double)x - (double)y * (double)y;
     }
@@ -138,9 +139,10 @@ struct SlidingSquares64 {
 
 // The sum of n <= 64 floats in order.  Multiples of g, the last bit of the smallest term but 0, that
 // add up to less than 2^42 g (total <= 2^18 smallest) are exact in FP64 and, with lo below 2^24 g, in
-// the pair; that takes in the ties, which such sums hit often.  Else lo is at most s eps total
-// after s terms, so that the pair is within n (n + 1) / 2 eps^2 total.
+// the pair; that takes in the ties, which such sums hit often.  Else, settled after every kRun terms,
+// lo is below (kRun + 1) eps total and the pair within (2 + .. + 9) / 8 eps^2 total per term.
 struct PartSum {
+    static constexpr int kRun = 8;
     Pair s;
     float total = 0.f, smallest = 3.4e38f;         // of the magnitudes
     MEM_SUM_HD void add(float x) {
@@ -151,7 +153,7 @@ struct PartSum {
     }
     MEM_SUM_HD bool value(int n, float* v) const {
         if (!(total < 1e38f)) return false;
-        const bool one = s.rounds(total * kEps2 * (float)(n * n), v);
+        const bool one = s.rounds(total * kEps2 * (6.f * (float)n + 16.f), v);
         if (one) return true;
         *v = MEM_ADD(s.hi, s.lo);
         return total <= 131072.f * smallest;

@@ -135,46 +135,49 @@ __global__ void __launch_bounds__(128) wiener_kernel(const float* __restrict__ c
     const float* C = ctf + (int64_t)ky * N + kx;
     const int i0 = blockIdx.y * kWienerChunk;
     const int i1 = min(m, i0 + kWienerChunk);
-    SlidingSquares w;
-#pragma unroll 4
-    for (int t = i0 + c; t > i0; --t) w.start(C[t * NN]);
-    w.started();
     constexpr int B = 8;                           // steps whose samples travel together
-    float a[B], b[B];
-    auto load = [&](int i) {
+    auto walk = [&](auto& w, int end, auto visit) {            // denominators i0 .. end - 1
+#pragma unroll 4
+        for (int t = i0 + c; t > i0; --t) w.start(C[t * NN]);
+        w.started();
+        float a[B], b[B];
+        auto load = [&](int i) {
 #pragma unroll
-        for (int u = 0; u < B; ++u) {
-            const int64_t q = min(i + u + 1, i1 - 1);              // the step from q - 1 to q
-            a[u] = C[(q + c) * NN];
-            b[u] = C[q * NN];
+            for (int u = 0; u < B; ++u) {
+                const int64_t q = min(i + u + 1, end - 1);         // the step from q - 1 to q
+                a[u] = C[(q + c) * NN];
+                b[u] = C[q * NN];
+            }
+        };
+        load(i0);
+        for (int i = i0; i < end; i += B) {
+            float x[B], y[B];
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                x[u] = a[u];
+                y[u] = b[u];
+            }
+            load(i + B);
+#pragma unroll
+            for (int u = 0; u < B; ++u) {
+                if (i + u >= end) break;
+                visit(i + u);
+                w.step(x[u], y[u]);
+            }
         }
     };
+    SlidingSquares w;
     uint64_t open = 0;                             // values that the pair leaves open
-    load(i0);
-    for (int i = i0; i < i1; i += B) {
-        float x[B], y[B];
-#pragma unroll
-        for (int u = 0; u < B; ++u) {
-            x[u] = a[u];
-            y[u] = b[u];
-        }
-        load(i + B);
-#pragma unroll
-        for (int u = 0; u < B; ++u) {
-            if (i + u >= i1) break;
-            float v;
-            if (!w.plus_fifth(c, i + u - i0, &v)) open |= 1ull << (i + u - i0);
-            rw[(int64_t)(i + u) * K + k] = __frcp_rn(v);
-            w.step(x[u], y[u]);
-        }
-    }
+    walk(w, i1, [&](int i) {
+        float v;
+        if (!w.plus_fifth(c, i - i0, &v)) open |= 1ull << (i - i0);
+        rw[(int64_t)i * K + k] = __frcp_rn(v);
+    });
     if (open == 0) return;
     SlidingSquares64 e;
-    for (int t = i0 + c; t > i0; --t) e.start(C[t * NN]);
-    for (int i = i0; open != 0; ++i, open >>= 1) {
-        if (open & 1) rw[(int64_t)i * K + k] = __frcp_rn(e.plus_fifth());
-        if (open > 1) e.step(C[(int64_t)(i + 1 + c) * NN], C[(int64_t)(i + 1) * NN]);
-    }
+    walk(e, i0 + 64 - __clzll(open), [&](int i) {
+        if (open >> (i - i0) & 1) rw[(int64_t)i * K + k] = __frcp_rn(e.plus_fifth());
+    });
 }
 
 // mu[g][i][l] = mu_psi[i][kModes g + l] in float32, zero past the last mode
@@ -294,21 +297,38 @@ __global__ void __launch_bounds__(kCorrThreads, 4) correlate_kernel(
 }
 
 // G[q][k] = sum_s part[s][q][k] in a fixed order (q = ii kModes + l), the floats of FP64 sums: bound by
-// reading the parts (160 MB for 1000 images of 128 px, c = 20: 44 us, 156 with FP64 sums alone)
+// reading the parts, the next ones loaded ahead (160 MB for 1000 images of 128 px, c = 20: 34 us, 156
+// with FP64 sums alone)
 __global__ void reduce_parts_kernel(const float2* __restrict__ part, int S, int64_t total,
                                     float2* __restrict__ G) {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= total) return;
     PartSum re, im;
-#pragma unroll 8
-    for (int s = 0; s < S; ++s) {
-        const float2 v = part[(int64_t)s * total + e];
-        re.add(v.x);
-        im.add(v.y);
+    constexpr int B = PartSum::kRun;
+    float2 next[B];                                // the next terms, loaded ahead
+    auto load = [&](int s0) {
+#pragma unroll
+        for (int u = 0; u < B; ++u) next[u] = part[(int64_t)min(s0 + u, S - 1) * total + e];
+    };
+    load(0);
+    for (int s0 = 0; s0 < S; s0 += B) {
+        float2 v[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) v[u] = next[u];
+        if (s0 + B < S) load(s0 + B);
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            if (s0 + u >= S) break;
+            re.add(v[u].x);
+            im.add(v[u].y);
+        }
+        re.s.settle();
+        im.s.settle();
     }
     float2 g;
     if (!re.value(S, &g.x) || !im.value(S, &g.y)) {
         double x = 0.0, y = 0.0;
+#pragma unroll 8
         for (int s = 0; s < S; ++s) {
             const float2 v = part[(int64_t)s * total + e];
             x += v.x;

@@ -68,6 +68,7 @@ static void parts(const char* name, int sums, int terms, Draw draw) {
         for (int s = 0; s < terms; ++s) {
             const float x = draw(s);
             p.add(x);
+            if (s % PartSum::kRun == PartSum::kRun - 1) p.s.settle();
             r += x;
         }
         float v;
