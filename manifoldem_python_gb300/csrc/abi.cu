@@ -808,8 +808,12 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
         return exec_fft(P, CUFFT_R2C, P.n_images, NN, specN, const_cast<float*>(images), fspec,
                         work, s);
     };
+    // the averages to make: the two of a PD go through one batched inverse transform, and the library's
+    // may work on two entries of a batch at once, so that neither is left unwritten there
+    const bool want_avg = out->img_avg || (out->img_avg_flip && !P.smem_fft);
+    const bool want_avg_flip = out->img_avg_flip || (out->img_avg && !P.smem_fft);
     // (a volume mask's first spectra, those of imgAll itself, serve the Wiener average only)
-    if (!fused && (!in->pd_mask || out->img_avg)) MEM_STEP(spectrum(img_all, nullptr));
+    if (!fused && (!in->pd_mask || want_avg)) MEM_STEP(spectrum(img_all, nullptr));
     MEM_STEP(mark(4));
     if (fused) MEM_STEP(kern::qfix(P, *in, qf, s));     // else with the rotation constants
     float* partial = at<float>(ws, L.partial);
@@ -827,7 +831,7 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
     if (in->pd_mask) {
         // the Wiener average from the unmasked spectra, then everything else (centring vectors
         // included, so that they centre the features D is computed from) from the masked ones
-        if (out->img_avg) {
+        if (want_avg) {
             MEM_STEP(kern::pd_sums(P, fspec, qf, items, partial, 1, s));
             MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
                                        avg_spec, pd_max, 1, false, s));
@@ -838,7 +842,7 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
             MEM_STEP(kern::apply_pd_mask(P, img_all, xbuf, in->pd_mask, img_pd, s));
             MEM_STEP(spectrum(xbuf, nullptr));
         }
-        if (want_feat || out->img_avg_flip) {
+        if (want_feat || want_avg_flip) {
             MEM_STEP(kern::pd_sums(P, fspec, qf, items, partial, 3, s));
             MEM_STEP(kern::pd_finalize(P, partial, items, item_off, pds, ft.ring_of, means,
                                        avg_spec, pd_max, 2, split, s));

@@ -700,3 +700,35 @@ def test_cut_tiles_on_some_of_the_sms(cuda_ready, few_sms, tile_n):
         plan.device_status()
         D.append(out['D'].clone())
     assert bool(torch.isfinite(D[0]).all()) and torch.equal(D[0], D[1])
+
+
+@pytest.mark.parametrize('masked', [False, True])
+@pytest.mark.parametrize('N', [33, 64, 100, 250, 257])
+def test_each_output_alone(cuda_ready, N, masked):
+    """An execute that is asked for one output gives the bits that it has among all of them, also where
+    the workspace held NaN before (what the output does not need is not computed)."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import OUTPUT_NAMES, Plan, StageParams
+    rng = np.random.default_rng(N)
+    counts = [5, 1, 9]
+    n = sum(counts)
+    plan = Plan(StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1,
+                            precision='bf16x3'), counts, [10.0, 180.0, -77.0])
+    stack = torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda()
+    args = dict(stack_index=torch.arange(n, device='cuda'),
+                flip=torch.from_numpy(rng.integers(0, 2, n).astype(np.uint8)).cuda(),
+                psi_rad=torch.from_numpy(rng.uniform(-3, 3, n)).cuda(),
+                df=torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda())
+    if masked:
+        args['pd_mask'] = torch.from_numpy((rng.random((3, N, N)) < 0.7).astype(np.uint8)).cuda()
+
+    def run(names, images):
+        out = plan.allocate_outputs(names)
+        plan.execute(images, outputs=out, **args)
+        return out
+
+    every = run(OUTPUT_NAMES, stack)
+    for names in [(k,) for k in OUTPUT_NAMES] + [('img_avg', 'img_all_flip')]:
+        run(OUTPUT_NAMES, torch.full_like(stack, float('nan')))
+        for k, v in run(names, stack).items():
+            assert bool(torch.isfinite(v).all()) and torch.equal(v, every[k]), k
