@@ -158,8 +158,9 @@ typedef struct mem_contraction_config {
 int mem_plan_set_contraction(mem_plan* plan, int32_t n_classes,
                              const mem_contraction_config* classes);
 
-/* Copy the plan's tables into the workspace (stream-ordered).  Call once per workspace
- * before mem_plan_execute (and before capturing it).                                      */
+/* Copy the plan's tables into the workspace and make its low-pass table there, which every
+ * execute reads (stream-ordered; an execute on another stream waits for it).  Call once per
+ * workspace before mem_plan_execute (and before capturing it).                            */
 int mem_plan_upload(mem_plan* plan, void* workspace, size_t workspace_bytes, void* stream);
 
 /* The distance stage for every PD of the plan: replaces

@@ -732,3 +732,40 @@ def test_each_output_alone(cuda_ready, N, masked):
         run(OUTPUT_NAMES, torch.full_like(stack, float('nan')))
         for k, v in run(names, stack).items():
             assert bool(torch.isfinite(v).all()) and torch.equal(v, every[k]), k
+
+
+@pytest.mark.parametrize('N', [100, 128, 250])
+def test_execute_on_another_stream_than_the_upload(cuda_ready, N):
+    """A plan made while the device is busy, executed at once on a stream of higher priority: the
+    execute waits for the tables that the plan's upload leaves to its own stream."""
+    torch = cuda_ready
+    from manifoldem_python_gb300.pipeline import Plan, StageParams
+    n = 400
+    rng = np.random.default_rng(N)
+    params = StageParams(N=N, pix_size=2.0, Cs=2.7, EkV=300.0, AmpContrast=0.1, avg_only=True)
+    args = (torch.from_numpy(rng.standard_normal((n, N, N)).astype(np.float32)).cuda(),
+            torch.arange(n, device='cuda'), torch.zeros(n, dtype=torch.uint8, device='cuda'),
+            torch.from_numpy(rng.uniform(-3, 3, n)).cuda(),
+            torch.from_numpy(rng.uniform(1e4, 3e4, n)).cuda())
+    plan = Plan(params, [n], [10.0])
+    want = plan.allocate_outputs(('img_all',))
+    plan.execute(*args, want)
+    got = plan.allocate_outputs(('img_all',))
+    busy, urgent = torch.cuda.Stream(), torch.cuda.Stream(priority=-5)
+    a = torch.randn((8192, 8192), device='cuda')
+    b = torch.empty_like(a)
+    torch.mm(a, a, out=b)
+    torch.cuda.synchronize()
+    ws = plan.workspace
+    ws.view(torch.float32)[:] = float('nan')           # the next plan's workspace: the same block
+    where = ws.data_ptr()
+    del plan, ws
+    with torch.cuda.stream(busy):
+        for _ in range(4):
+            torch.mm(a, a, out=b)
+    plan = Plan(params, [n], [10.0])
+    assert plan.workspace.data_ptr() == where
+    plan.execute(*args, got, urgent)
+    torch.cuda.synchronize()
+    plan.device_status()
+    assert torch.equal(got['img_all'], want['img_all'])
