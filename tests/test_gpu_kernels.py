@@ -736,8 +736,8 @@ def test_each_output_alone(cuda_ready, N, masked):
 
 @pytest.mark.parametrize('N', [100, 128, 250])
 def test_execute_on_another_stream_than_the_upload(cuda_ready, N):
-    """A plan made while the device is busy, executed at once on a stream of higher priority: the
-    execute waits for the tables that the plan's upload leaves to its own stream."""
+    """A plan uploaded while the device is busy and executed at once on a stream of higher priority:
+    the execute waits for the tables that the upload leaves to its own stream."""
     torch = cuda_ready
     from manifoldem_python_gb300.pipeline import Plan, StageParams
     n = 400
@@ -756,15 +756,11 @@ def test_execute_on_another_stream_than_the_upload(cuda_ready, N):
     b = torch.empty_like(a)
     torch.mm(a, a, out=b)
     torch.cuda.synchronize()
-    ws = plan.workspace
-    ws.view(torch.float32)[:] = float('nan')           # the next plan's workspace: the same block
-    where = ws.data_ptr()
-    del plan, ws
+    plan.workspace.view(torch.float32)[:] = float('nan')
     with torch.cuda.stream(busy):
         for _ in range(4):
             torch.mm(a, a, out=b)
-    plan = Plan(params, [n], [10.0])
-    assert plan.workspace.data_ptr() == where
+    _call(torch, 'mem_plan_upload', plan.handle, plan.workspace.data_ptr(), plan.ws_bytes)
     plan.execute(*args, got, urgent)
     torch.cuda.synchronize()
     plan.device_status()
