@@ -153,8 +153,10 @@ typedef struct mem_contraction_config {
 
 /* Sets the plan's contraction schedule (HOST array of n_classes >= 1 entries, max_n
  * strictly increasing); call before mem_plan_upload.  Default: one class, one CTA per tile,
- * two accumulators, 128-wide tiles.  MEM_ERR_INVALID on a malformed table or after the
- * upload.                                                                                  */
+ * two accumulators, 128- or 256-wide tiles, whichever take fewer waves of tiles.  A class of
+ * one CTA per 128-row tile and two accumulators, alone, has the tiles of a partial last wave cut
+ * in two, and those of few 128 x 128 tiles split by K chunks.  D has the same bits in all
+ * of them.  MEM_ERR_INVALID on a malformed table or after the upload.                       */
 int mem_plan_set_contraction(mem_plan* plan, int32_t n_classes,
                              const mem_contraction_config* classes);
 

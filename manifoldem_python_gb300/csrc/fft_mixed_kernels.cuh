@@ -5,7 +5,7 @@
 //   inverse    half-plane spectrum (times sign(C) / N^2) -> image (:375-389).
 // Layout and scaling are those of a cuFFT R2C / C2R pair.  Two forms, by where an image fits:
 //
-// Whole (N <= 224): one image per CTA, the N x N / 2 complex buffer in shared memory; an image is
+// Whole (N <= 228): one image per CTA, the N x N / 2 complex buffer in shared memory; an image is
 // read and written once.  Bound by the latency of its 8 (low-pass 12) shared-memory passes at the
 // 12 to 20 warps that the buffer and about 100 registers per thread leave on an SM.
 //

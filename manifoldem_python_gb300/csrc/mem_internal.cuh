@@ -279,8 +279,9 @@ int64_t tc_split_units(int64_t tiles, int64_t chunks, int64_t most);
 
 std::vector<int32_t> radius_descending_columns(int N, int64_t Kc, int64_t Kc_pad);
 
-// default contraction schedule: one class, one CTA per 128 x 128 tile, two TMEM accumulators
-// (MEM_TC_PERSISTENT / MEM_TC_BUFS / MEM_TC_TILE_N override it, for tuning)
+// default contraction schedule: one class, one CTA per tile, two TMEM accumulators, 128 x 128 tiles
+// (MEM_TC_PERSISTENT / MEM_TC_BUFS / MEM_TC_TILE_N override it, for tuning); the plan widens
+// the tiles by its own count of waves
 mem_contraction_config default_contraction();
 
 // the cut tiles of a partial last wave (gemm_tc.cu): flags of their warps, then running sums

@@ -1304,8 +1304,8 @@ int rotate(const mem_plan& P, const mem_inputs& in, float* xbuf, float* img_out,
     const int st = rot_consts(P, in, pd_table, img_pd, rot_scratch, qf, s);
     if (st != MEM_OK) return st;
     // the banded kernel where no whole image fits, and for large boxes without a compile-time
-    // kernel (800 images of 190 px: 432 us, 456 with the runtime-size kernel; 1000 of 142 px: 327
-    // against 277)
+    // kernel (800 images of 186 px: 386 us, 435 with the runtime-size kernel; 900 of 174 px: 410
+    // against 405, 1000 of 142 px: 299 against 277)
     const bool fixed_n = N == 64 || N == 128;
     const bool whole = P.rot_whole && mixed::rotate_supported(N);
     if (kern::rotate_band_supported(N) &&

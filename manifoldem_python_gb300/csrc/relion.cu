@@ -15,7 +15,9 @@
 // unchanged.  One CTA per image, the image in shared memory, N <= 236.
 //
 // relion_shift_kernel (N >= 40): a line is split into nseg segments of L <= 32 samples, one thread
-// per segment holding it in registers; the states between segments go through shared memory.
+// per segment holding it in registers; the states between segments go through shared memory (z^20 =
+// 4e-12 of a state is left out at a line's start, where the float transforms that follow round at
+// 1e-7 of the image's largest value).
 // Axis 0 comes first, its lines read from global memory (lanes on consecutive columns), and
 // axis 1 last, its results written to global memory (lanes on consecutive rows of the transposed
 // output): an image is read and written once, coalesced.  Bound by the latency of the

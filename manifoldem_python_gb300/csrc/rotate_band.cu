@@ -5,7 +5,8 @@
 // One launch per rotation, one CTA per image and band of h consecutive layout rows:
 //   1. the prefilter along layout columns for the band's rows and the 3 below them (the 4x4
 //      window), straight from the input image in global memory: the recursions start kWarm rows
-//      outside (periodic; z1^20 = 4e-12 of a state is left out), so a band needs no other
+//      outside (periodic; z1^20 = 4e-12 of a state is left out, where the float transforms that
+//      the image comes from round at 1e-7 of its largest value), so a band needs no other
 //      band's coefficients and no scratch; lanes on consecutive columns, segments of up to 32
 //      rows in registers;
 //   2. the prefilter along each of the band's rows in shared memory, and the 3-column halo;
