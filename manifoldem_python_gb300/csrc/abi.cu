@@ -646,8 +646,9 @@ int mem_plan_upload(mem_plan* plan, void* workspace, size_t workspace_bytes, voi
     // the pageable source above is consumed before cudaMemcpyAsync returns
     if (!plan->upload_done)
         MEM_CUDA_TRY(cudaEventCreateWithFlags(&plan->upload_done, cudaEventDisableTiming));
+    else                               // another workspace's, on another stream: after both
+        MEM_CUDA_TRY(cudaStreamWaitEvent(s, plan->upload_done, 0));
     MEM_CUDA_TRY(cudaEventRecord(plan->upload_done, s));
-    plan->upload_over = false;
     return MEM_OK;
 }
 
@@ -683,19 +684,13 @@ int mem_plan_execute_split(mem_plan* plan, const mem_inputs* in, const mem_outpu
 namespace {
 // Orders an execute after the upload where that ran on another stream and is still under way (its
 // kernel and its memsets, unlike the copy of the tables, wait for SMs).  A graph runs what was
-// captured after the upload later.
-int wait_for_upload(mem_plan& P, cudaStream_t ls, cudaStream_t s) {
-    if (P.upload_over) return MEM_OK;
+// captured after the upload later.  (No query of the event: one invalidates captures of other
+// threads.)
+int wait_for_upload(const mem_plan& P, cudaStream_t ls, cudaStream_t s) {
+    if (!P.upload_done) return MEM_OK;     // uploaded with a plan like this one
     cudaStreamCaptureStatus capture;
     MEM_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
     if (capture != cudaStreamCaptureStatusNone) return MEM_OK;
-    const cudaError_t e = cudaEventQuery(P.upload_done);
-    if (e == cudaSuccess) {
-        P.upload_over = true;
-        return MEM_OK;
-    }
-    if (e != cudaErrorNotReady) return MEM_ERR_CUDA;
-    cudaGetLastError();
     MEM_CUDA_TRY(cudaStreamWaitEvent(ls, P.upload_done, 0));
     if (s != ls) MEM_CUDA_TRY(cudaStreamWaitEvent(s, P.upload_done, 0));
     return MEM_OK;
@@ -746,7 +741,7 @@ int execute_impl(mem_plan* plan, const mem_inputs* in, const mem_outputs* out, v
         if (st != MEM_OK) return st; \
     } while (0)
 
-    MEM_STEP(wait_for_upload(PM, ls, s));
+    MEM_STEP(wait_for_upload(P, ls, s));
     // the stack is read by exactly one kernel (the first), issued on the load stream
     // the status words, and the PDs' maxima in the same memset (of a split execute later, on the
     // stream that uses them)

@@ -157,8 +157,7 @@ struct mem_plan {
     cudaEvent_t ev[MEM_NUM_PHASES + 1] = {};
     bool phase_ran[MEM_NUM_PHASES] = {};
     cudaEvent_t load_done = nullptr; // end of the stack-reading phase (mem_plan_execute_split)
-    cudaEvent_t upload_done = nullptr;  // end of the upload, until upload_over
-    bool upload_over = false;
+    cudaEvent_t upload_done = nullptr;  // end of the upload
     ~mem_plan() {
         for (auto& e : ev)
             if (e) cudaEventDestroy(e);

@@ -734,8 +734,8 @@ def test_each_output_alone(cuda_ready, N, masked):
             assert bool(torch.isfinite(v).all()) and torch.equal(v, every[k]), k
 
 
-@pytest.mark.parametrize('N', [100, 128, 250])
-def test_execute_on_another_stream_than_the_upload(cuda_ready, N):
+@pytest.mark.parametrize('N,second', [(100, False), (128, False), (250, False), (128, True)])
+def test_execute_on_another_stream_than_the_upload(cuda_ready, N, second):
     """A plan uploaded while the device is busy and executed at once on a stream of higher priority:
     the execute waits for the tables that the upload leaves to its own stream."""
     torch = cuda_ready
@@ -761,6 +761,10 @@ def test_execute_on_another_stream_than_the_upload(cuda_ready, N):
         for _ in range(4):
             torch.mm(a, a, out=b)
     _call(torch, 'mem_plan_upload', plan.handle, plan.workspace.data_ptr(), plan.ws_bytes)
+    if second:                                         # the last upload is another workspace's
+        other = torch.empty_like(plan.workspace)
+        with torch.cuda.stream(torch.cuda.Stream(priority=-5)):
+            _call(torch, 'mem_plan_upload', plan.handle, other.data_ptr(), plan.ws_bytes)
     plan.execute(*args, got, urgent)
     torch.cuda.synchronize()
     plan.device_status()
